@@ -12,7 +12,10 @@ std::unique_ptr<Runner> make_runner3d(const claw_config& cfg) {
     // src/3d/claw3ez.f:136: any splitting request runs dimsp3's Godunov splitting
     if (cfg.dimensional_split > 0)
         return std::unique_ptr<Runner>(new SplitRunner3D<VCAcoustics3D<double>, 0>());
-    return runner3d_for<double, 0>(cfg);
+    using S = VCAcoustics3D<double>;
+    if (cfg.order == 2 && cfg.transverse_waves == 22 && cfg.limiter[0] == 4 && cfg.limiter[1] == 4)
+        return std::unique_ptr<Runner>(new Runner3D<S, MethodMC3D>());
+    return std::unique_ptr<Runner>(new Runner3D<S, MethodGeneric3D>());
 }
 
 }  // namespace clawb200

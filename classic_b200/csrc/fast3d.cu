@@ -1,9 +1,59 @@
 // The 3D step with fused multiply-adds (CLAW_FP64_FMA) and in FP32
-// (CLAW_FP32; Courant number, dt and time stay FP64): the same kernels as
-// claw3d.cu compiled with --fmad=true.
+// (CLAW_FP32; Courant number, dt and time stay FP64), compiled with
+// --fmad=true: step3f_kernel (step3d_fast.cuh) for the unsplit step, the
+// split sweeps of step3ds.cuh for Godunov splitting.
 #include "runner3d.cuh"
+#include "step3d_fast.cuh"
 
 namespace clawb200 {
+
+template <typename real, int LIM, bool TRANS>
+struct Step3fRunner : Runner {
+    using Sh = Step3fShape<real>;
+    Step3fArgs<real> args;
+    int grid = 1;
+
+    int prepare(const claw_config& cfg, const Geometry& g) override {
+        auto k = &step3f_kernel<real, LIM, TRANS>;
+        std::memset(&args, 0, sizeof(args));
+        fill_sweep3(args.g, cfg, g);
+        args.tilesx = (g.mx + Sh::outx - 1) / Sh::outx;
+        args.tilesy = (g.my + Sh::outy - 1) / Sh::outy;
+        CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::smem));
+        int dev = 0, nsm = 0, per_sm = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * Sh::rows, Sh::smem));
+        if (per_sm < 1) return fail(CLAW_E_CUDA, "step3f kernel cannot be resident on an SM");
+        // Segments of planes: the count with the least work in the longest
+        // column of CTAs (waves of CTAs times planes each marches, with 4
+        // planes' worth of start-up: two halo planes and the first copies).
+        const long long tiles = (long long)args.tilesx * args.tilesy, slots = (long long)nsm * per_sm;
+        long long best = -1;
+        for (int n = 1; n <= g.mz; ++n) {
+            const int len = (g.mz + n - 1) / n;
+            const int segs = (g.mz + len - 1) / len;
+            const long long cost = (tiles * segs + slots - 1) / slots * (len + 4);
+            if (best < 0 || cost < best) {
+                best = cost;
+                args.seglen = len;
+                if (tiles * segs > 0x7fffffffLL) return fail(CLAW_E_UNSUPPORTED, "3D grid too large");
+                grid = (int)(tiles * segs);
+            }
+        }
+        return 0;
+    }
+    cudaError_t launch(cudaStream_t s) override {
+        return launch_step(&step3f_kernel<real, LIM, TRANS>, dim3(grid), dim3(32 * Sh::rows), Sh::smem, s, args);
+    }
+};
+
+template <typename real>
+static std::unique_ptr<Runner> step3f_runner(const claw_config& cfg) {
+    if (cfg.transverse_waves < 10) return std::unique_ptr<Runner>(new Step3fRunner<real, -1, false>());
+    if (cfg.limiter[0] == 4 && cfg.limiter[1] == 4) return std::unique_ptr<Runner>(new Step3fRunner<real, 4, true>());
+    return std::unique_ptr<Runner>(new Step3fRunner<real, -1, true>());
+}
 
 std::unique_ptr<Runner> make_fast_runner3d(const claw_config& cfg) {
     if (cfg.solver_id != CLAW_SOLVER_VC_ACOUSTICS_3D) return nullptr;
@@ -14,8 +64,8 @@ std::unique_ptr<Runner> make_fast_runner3d(const claw_config& cfg) {
             return std::unique_ptr<Runner>(new SplitRunner3D<VCAcoustics3D<double>, 1>());
         return nullptr;
     }
-    if (cfg.precision == CLAW_FP32) return runner3d_for<float, 1>(cfg);
-    if (cfg.precision == CLAW_FP64_FMA) return runner3d_for<double, 1>(cfg);
+    if (cfg.precision == CLAW_FP32) return step3f_runner<float>(cfg);
+    if (cfg.precision == CLAW_FP64_FMA) return step3f_runner<double>(cfg);
     return nullptr;
 }
 

@@ -133,10 +133,7 @@ using MethodMC3D = Method3D<2, 2, 4>;  // transverse_waves 22, MC on both waves
 // bit-identical to the serial reference order in FP64 without contraction.
 constexpr int NT3P = 2 * NT3;
 
-// BUILD tells apart the instantiations of the reference-order unit (0,
-// --fmad=false) and the contracted unit (1, --fmad=true): the same template
-// arguments in both would be one symbol with two different bodies.
-template <class S, int DIR, class M, bool LAST, int BUILD>
+template <class S, int DIR, class M, bool LAST>
 __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const Sweep3Args<typename S::real> a) {
     using real = typename S::real;
     using Split = typename S::Split;
@@ -288,7 +285,7 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
         real s[2];
         S::rpn(pL, uL, pR, uR, Zo(i - 1, 0, 0), Co(i - 1, 0, 0), Zo(i, 0, 0), Co(i, 0, 0), w, s, am, ap);
         if (i >= 1 && i <= mN + 1) {
-            for (int k = 0; k < 2; ++k) {  // Courant number in FP64 (FP32 builds too)
+            for (int k = 0; k < 2; ++k) {
                 const double c = tn_d * (double)s[k];
                 cfl = fmax(fmax(cfl, c), -c);
             }

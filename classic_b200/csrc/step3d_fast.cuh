@@ -1,528 +1,498 @@
 // 3D unsplit step, contracted FP64 and FP32 builds (src/3d/step3.f90 with
-// src/3d/flux3.f90, transverse codes of flux3.f90:189-197), for sm_100a.
+// src/3d/flux3.f90, transverse codes of flux3.f90:189-197), for sm_100a: one
+// launch per step, q and aux read once and q written once.
 //
-// The tiling, the march and the per-value arithmetic are those of the
-// reference-order kernel in step3d.cuh, with three changes that the exact
-// build cannot take:
-//   * the pair of threads that shares a slice is the same lane of two
-//     neighbouring warps, so each warp's role h is a compile-time constant and
-//     every shared-memory index folds to an immediate offset; the four
-//     combinations each role needs from the other's splits
-//     (flux3.f90:363-376 and :488-495) cross through shared memory under a
-//     64-thread named barrier of the warp pair, the centre terms with the
-//     CTA barrier of the position;
-//   * the aux ring holds the face reciprocals 1 / (Z + Z_next) along the
-//     tile's two axes, so the 16 transverse splits of a slice position
-//     multiply instead of dividing (rounding differs from the divisions);
-//   * Z, c and the next position's q values are copied by cp.async issued at
-//     the top of a position and awaited just before its CTA barrier, so their
-//     latency overlaps the position's arithmetic, and the reciprocals of a
-//     ring position are formed from the landed Z one position later;
-//   * a cell adds its nine neighbour terms in a fixed order instead of
-//     step3's 2x2-block colour order.
-// The Courant number is the same FP64 product as the exact build's, so the
-// dt sequence is identical.
+// flux3 splits, at both cells of every interface and in both directions
+// across, the fluctuation and the correction flux (rpt3), and splits the
+// parts again (rptt3): 24 splits per interface and sweep.  The splits of
+// variable-coefficient acoustics act on the pressure part alone, with
+// coefficients of the receiving cells, and every later use is linear.  With
+// s = A+dq (left face) + A-dq (right face) and d = cqxx(right) - cqxx(left),
+// pressure parts, a cell's share of all of them depends on two numbers per
+// sweep along n:
+//   X = -dt/(2 dn) s - dt/dn d          (what rpt3 splits)
+//   Y = s + 3 d                         (what rptt3 splits twice)
+// and the sums collapse to fluxes (K = c Z, r = 1/(Z + Z') at a face):
+//   * across a face between cells a | b:  velocity r (c_b X_a + c_a X_b),
+//     pressure r (K_b X_a - K_a X_b).  The y- and z-sweeps' X act on the same
+//     x faces with the same factor dt/dx, so a face takes the sum of the two.
+//   * at an edge with cells A B / C D around it, the double splits in both
+//     orders: with f = dt^3/(6 dx dy dz), q changes by the mixed second
+//     difference of f times
+//       p   (m1 + m2)(Z_D yA + Z_A yD) - (m3 + m4)(Z_C yB + Z_B yC)
+//       u   m1 yA + m3 yB - m4 yC - m2 yD     (along A-B)
+//       v   m2 yA - m4 yB + m3 yC - m1 yD     (along A-C)
+//     yA = c_D Y_A, yB = c_C Y_B, yC = c_B Y_C, yD = c_A Y_D and, with a the
+//     A-C, b the B-D, g the A-B and e the C-D face's r, m1 = a e K_C,
+//     m2 = b g K_B, m3 = b e K_D, m4 = a g K_A.
+// About 330 FP64 instructions per cell and step where the splits written out
+// one by one took 1815.  The limiter works on wave strengths: the ratio of
+// two waves' products is a'/a (1 + Z Z')/(1 + Z^2) with per-cell 1/(1 + Z^2).
+//
+// The march.  A warp holds 32 cells of a row (lane = x), a CTA ROWS rows; the
+// CTA marches up z, one plane per iteration, through a segment of planes.
+// x neighbours come by shuffle or from the shared planes, y neighbours
+// through shared memory, z neighbours are the thread's own registers.  The
+// outer two lanes and the outer row each side are halo: 28 x (ROWS-2) cells
+// per plane are written.  Planes arrive by cp.async three ahead of their
+// in-plane use (p, Z, c and w serve the z interfaces first).  Per plane:
+//   A  strengths at the x, y and z interfaces
+//   -- barrier
+//   B  limited waves, correction fluxes, the x and z sums of the cell
+//   -- barrier
+//   C  the y sums; face fluxes of plane t, edge fluxes at plane t and
+//      between planes t-1 and t
+//   -- barrier
+//   D  plane t-1 complete: differences of the fluxes, store
+// The Courant number is the largest |c| times dt/dn in FP64, the value the
+// interface-by-interface maximum takes, so the dt sequence is the
+// reference-order build's.
+//
+// Measured against three sweep launches that formed every split (1815 FP64
+// instructions and 245 B of DRAM traffic per cell): 256^3 FP64 7.45 -> 1.32
+// ms per step, 161x130x147 FP32 1.02 -> 0.167.  What bounds it: FP64 at
+// 192^3 runs the FP64 pipe at 30 % and issue at 46 % with 12 warps per SM
+// (fixed-latency chains and the three barriers); FP32 is issue bound (71 %).
+// DRAM traffic is 77 B per cell (80 algorithmic).
 #pragma once
+#include "char2d.cuh"
 #include "step3d.cuh"
 
 namespace clawb200 {
 
-constexpr int XCH3 = 10;  // exchange planes of NT3 values: L [h][2], R [h][2], centre [h]
-constexpr int NPL3F = 4;  // aux planes: Z, c, 1/(Z+Z_e1), 1/(Z+Z_e2)
+// Rows (warps) of a CTA and resident CTAs.  FP64: 12 rows leave 168 registers
+// a thread and nothing spills; the shared planes leave so little L1 that any
+// spill goes to L2 (256^3, ms per step: 12 rows 1.32, 13 rows at 144
+// registers 2.41, 16 rows at 128 2.1, 8 rows x 2 CTAs 1.9).  FP32: two CTAs of
+// 9 rows hide each other's barriers (161x130x147, us per step: 9 x 2 167,
+// 8 x 2 172, 10 x 2 181, 16 x 1 177, 18 x 1 188, 7 x 3 193).
+#ifndef CLAW_STEP3F_ROWS
+#define CLAW_STEP3F_ROWS 12
+#endif
+#ifndef CLAW_STEP3F_MINB
+#define CLAW_STEP3F_MINB 1
+#endif
+#ifndef CLAW_STEP3F_ROWS32
+#define CLAW_STEP3F_ROWS32 9
+#endif
+#ifndef CLAW_STEP3F_MINB32
+#define CLAW_STEP3F_MINB32 2
+#endif
 
-// Shared memory is sized to the carveout steps (100, 132, 164, 196, 228 KB):
-// what the carveout leaves is L1, which serves the x-sweep's strided loads.
-// buffers of neighbour terms: two (by position parity) in FP32 (106 KB, the
-// 132 KB step); one in FP64, with a second CTA barrier per position (149 KB,
-// the 164 KB step, instead of the 228 KB step)
+#ifndef CLAW_STEP3F_UNROLL
+#define CLAW_STEP3F_UNROLL 1  // 2 spills in FP64 (256^3: 30.1 against 24.9 ms a frame)
+#endif
+
 template <typename real>
-__host__ __device__ constexpr int term3_bufs() {
-    return sizeof(real) == 4 ? 2 : 1;
-}
-
-constexpr int VST3 = 8;  // staged values of the cells each role updates: [position & 1][role][2]
+struct Step3fShape {
+    static constexpr int rows = sizeof(real) == 8 ? CLAW_STEP3F_ROWS : CLAW_STEP3F_ROWS32;
+    static constexpr int minb = sizeof(real) == 8 ? CLAW_STEP3F_MINB : CLAW_STEP3F_MINB32;
+    static constexpr int outx = 28, outy = rows - 2;  // cells written per plane
+    static constexpr int nr = rows + 2;               // rows of a shared plane
+    static constexpr int pl = nr * 32;                // values of a shared plane
+    // rings: p, Z, c of 5 planes; u, v, w of 2; 20 planes that threads
+    // exchange and 9 for values held from plane to plane
+    static constexpr int ring = 15, uvw = 6, exch = 29;
+    static constexpr int smem = (ring + uvw + exch) * pl * (int)sizeof(real);
+};
 
 template <typename real>
-__host__ __device__ constexpr int sweep3f_smem_bytes() {
-    return (RING3 * NPL3F * NS3 + term3_bufs<real>() * NTERM3 * NT3 +
-            (XCH3 + QST3 + VST3) * NT3) *
-               (int)sizeof(real) +
-           16 * (int)sizeof(double);
-}
+struct Step3fArgs {
+    Sweep3Args<real> g;  // q, aux, strides, sizes, boundary conditions, method
+    int tilesx, tilesy, seglen;
+};
 
-__device__ __forceinline__ void pair_sync(int id) {
-    asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
-}
-
-// The march of one tile of slices for the threads of role H; returns the
-// thread's Courant number.
-template <class S, int DIR, class M, int H>
-__device__ __forceinline__ double sweep3f_march(const Sweep3Args<typename S::real>& a,
-                                               unsigned char* smem_raw) {
-    using real = typename S::real;
-    using Split = typename S::Split;
-    constexpr int AXN = DIR, AXA = DIR == 0 ? 1 : 0, AXB = DIR == 2 ? 1 : 2;
-    constexpr bool E1A = DIR != 1;
-    constexpr int CN = 1 + AXN, CE1 = 1 + (E1A ? AXA : AXB), CE2 = 1 + (E1A ? AXB : AXA);
-    constexpr int NPL = NPL3F;
-    constexpr int NTB = term3_bufs<real>();
-    // shared-memory steps of this role's own split direction and the other
-    constexpr int E1S = E1A ? 1 : S3A, E2S = E1A ? S3A : 1;
-    constexpr int OWNS = H ? E2S : E1S, OTHS = H ? E1S : E2S;
-    constexpr int CA = H ? CE1 : 0, CB = H ? CE2 : CN;  // components this role updates
-
-    real* saux = reinterpret_cast<real*>(smem_raw);  // [RING3][NPL][NS3]
-    real* sterm = saux + RING3 * NPL * NS3;          // [NTB][NTERM3][NT3]
-    real* sxch = sterm + NTB * NTERM3 * NT3;         // [XCH3][NT3]
-    real* sq = sxch + XCH3 * NT3;                    // [QST3][NT3]
-    real* sv = sq + QST3 * NT3;                      // [VST3][NT3]
-
+template <typename real, int LIM, bool TRANS>
+__global__ void __launch_bounds__(32 * Step3fShape<real>::rows, Step3fShape<real>::minb)
+step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
+    using Sh = Step3fShape<real>;
+    constexpr int ROWS = Sh::rows, PL = Sh::pl;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int kUnroll = CLAW_STEP3F_UNROLL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double red[ROWS];
+    const Sweep3Args<real>& a = A.g;
     ClawCtl* ctl = a.ctl;
-    const int cur = ctl->cur;
+    grid_dependency_sync();
+    if (*(volatile int*)&ctl->done) return;
+    const int cur = *(volatile int*)&ctl->cur;
+    const double dt = *(volatile double*)&ctl->dt;
+    const double tbc = *(volatile double*)&ctl->told;
     const real* __restrict__ qold = a.q[cur];
     real* __restrict__ qnew = a.q[cur ^ 1];
     const real* __restrict__ aux = a.aux;
-    const double dt = ctl->dt;
-    const double tbc = ctl->told;
-    const double tn_d = dt / a.d[AXN];
-    const real tn = (real)tn_d;
-    const real te1 = (real)(dt / a.d[E1A ? AXA : AXB]);
-    const real te2 = (real)(dt / a.d[E1A ? AXB : AXA]);
-    const real H5 = real(0.5) * tn;
-    const real S6g = (real(1.0) / real(6.0)) * tn * te2;
-    const real S6h = (real(1.0) / real(6.0)) * tn * te1;
-    const real dtdxave = real(0.5) * (tn + tn);
-    const real t_own = H ? te2 : te1;
-    const real S6own = H ? S6h : S6g;
+    const real tx = (real)(dt / a.d[0]), ty = (real)(dt / a.d[1]), tz = (real)(dt / a.d[2]);
+    const real half2 = a.order == 2 ? real(0.5) : real(0);   // order 1: no correction fluxes
+    const real xd = a.m3 == 2 ? real(1) : real(0);           // rpt3 splits the correction flux too
+    const real yd = a.m3 == 2 && a.m4 == 2 ? real(3) : real(0);
+    const real f6 = TRANS && a.m4 > 0 ? (real(1) / real(6)) * tx * ty * tz : real(0);
+    const int lim1 = a.mthlim[0], lim2 = a.mthlim[1];
 
-    const int m3 = M::m3 >= 0 ? M::m3 : a.m3;
-    const int m4 = M::m4 >= 0 ? M::m4 : a.m4;
-    const int order = M::m3 >= 0 ? 2 : a.order;
+    const int mx = a.m[0], my = a.m[1], mz = a.m[2];
+    const int lane = threadIdx.x & 31;
+    // FP32, bound by issue: a warp-uniform value to the compiler (3 % faster);
+    // in FP64 that costs registers it does not have
+    const int r = sizeof(real) == 4 ? __shfl_sync(FULL, (int)(threadIdx.x >> 5), 0) : (int)(threadIdx.x >> 5);
+    int bid = blockIdx.x;
+    const int bx = bid % A.tilesx;
+    bid /= A.tilesx;
+    const int by = bid % A.tilesy, seg = bid / A.tilesy;
+    const int k0 = 1 + seg * A.seglen, k1 = min(k0 + A.seglen, mz + 1);  // planes written: k0 .. k1-1
+    const int i = 1 + bx * Sh::outx - 2 + lane;  // this thread's column
+    const int j0 = 1 + by * Sh::outy;            // first row written
+    const int j = j0 - 1 + r;                    // this warp's row
+    const bool out = lane >= 2 && lane < 30 && i <= mx && r >= 1 && r < ROWS - 1 && j <= my;
 
-    const int mN = a.m[AXN], mA = a.m[AXA], mB = a.m[AXB];
-    const int bid = blockIdx.x;
-    const int seg = bid % a.nseg, tile = bid / a.nseg;
-    const int A0 = 1 + (tile % a.tilesA) * (T3A - 2);
-    const int B0 = 1 + (tile / a.tilesA) * (T3B - 2);
-    const int p0 = 1 + seg * SEG3;
-    const int p1 = min(p0 + SEG3, mN + 1);
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5;
-    const int sl = (warp >> 1) * 32 + (tid & 31);  // slice within the tile
-    const int pair_id = 1 + (warp >> 1);           // named barrier of the warp pair
-    const int ta = sl % T3A, tb = sl / T3A;
-    const int A = A0 - 1 + ta, B = B0 - 1 + tb;
-    const bool active = A <= mA + 1 && B <= mB + 1;
-    const bool apply = active && ta >= 1 && ta <= T3A - 2 && tb >= 1 && tb <= T3B - 2 &&
-                       A <= mA && B <= mB;
+    // source cell of a column and a row under the boundary conditions; cells
+    // past the last ghost layer repeat it (nothing written depends on them)
+    bool negx, negy, negb, negh;
+    const int ic = min(i, mx + 2), jc = min(j, my + 2);
+    const int im = bc3_src(ic, mx, a.bc[0], a.bc[1], negx);
+    const int jm = bc3_src(jc, my, a.bc[2], a.bc[3], negy);
+    (void)bc3_src(min(j - 1, my + 2), my, a.bc[2], a.bc[3], negb);  // the row below
+    // the first and the last warp also copy the row beyond theirs
+    const bool edge = r == 0 || r == ROWS - 1;
+    const int jh = min(r == 0 ? j - 1 : j + 1, my + 2);
+    const int jhm = bc3_src(jh, my, a.bc[2], a.bc[3], negh);
+    const long long qxy = (long long)(im - 1) + (long long)(jm - 1) * a.qs[1];
+    const long long qxh = (long long)(im - 1) + (long long)(jhm - 1) * a.qs[1];
+    const long long axy = (long long)(ic + 1) + (long long)(jc + 1) * a.as[1];
+    const long long axh = (long long)(ic + 1) + (long long)(jh + 1) * a.as[1];
 
-    bool flipA, flipB;
-    const int Am = bc3_src(min(max(A, -1), mA + 2), mA, a.bc[2 * AXA], a.bc[2 * AXA + 1], flipA);
-    const int Bm = bc3_src(min(max(B, -1), mB + 2), mB, a.bc[2 * AXB], a.bc[2 * AXB + 1], flipB);
-    const long long qoffAB = (long long)(Am - 1) * a.qs[AXA] + (long long)(Bm - 1) * a.qs[AXB];
-    const bool pistonB = AXB == 2 && B > mB && a.bc[5] == BC_PISTON;
+    real* ring = reinterpret_cast<real*>(smem_raw);  // [5][p, Z, c][PL]
+    real* uvw = ring + Sh::ring * PL;                // [2][u, v, w][PL]
+    real* ex = uvw + Sh::uvw * PL;
+    const int own = (r + 1) * 32 + lane;
+    const int lm = own - (lane > 0 ? 1 : 0), lp = own + (lane < 31 ? 1 : 0);
+    const int hal = r == 0 ? lane : (ROWS + 1) * 32 + lane;
+    real *SA1 = ex, *SA2 = ex + PL, *SG = ex + 2 * PL, *ST1 = ex + 3 * PL, *SCP = ex + 4 * PL,
+         *SCV = ex + 5 * PL, *SXY = ex + 6 * PL, *SYZ = ex + 7 * PL, *SRZ = ex + 8 * PL;
+    real* SP = ex + 9 * PL;    // [2 by the plane's parity][Yx, rx, ry]
+    real* SE = ex + 15 * PL;   // [5] what a row hands to the row above it
+    // [9] values held from plane to plane (registers would spill): plane t-1's
+    // q plus its own sums, the edge fluxes at t-3/2, plane t-1's Yy
+    real* SB = ex + 20 * PL;
 
-    auto load_pn = [&](int pos, real& qp, real& qn) {
-        bool fN;
-        const int pm = bc3_src(pos, mN, a.bc[2 * AXN], a.bc[2 * AXN + 1], fN);
-        const long long off = qoffAB + (long long)(pm - 1) * a.qs[AXN];
-        qp = qold[off];
-        qn = qold[off + CN * a.fstride];
-        if (fN) qn = -qn;
-        if (CN == 3) {
-            const bool pist = (AXN == 2 && pos > mN && a.bc[5] == BC_PISTON) || pistonB;
-            if (pist) {
-                const int ci = AXN == 0 ? pos : A;
-                const int cj = AXN == 1 ? pos : (AXA == 1 ? A : B);
-                qn = (real)(2.0 * piston_speed(a, ci, cj, tbc)) - qn;
-            }
+    auto zsrc = [&](int pos, bool& neg) {
+        return bc3_src(min(pos, mz + 2), mz, a.bc[4], a.bc[5], neg);
+    };
+    // copies of plane pos: p, Z, c into ring slot `so`, w into its parity's
+    auto issue_pzc = [&](int pos, int so) {
+        bool neg;
+        const int pm = zsrc(pos, neg);
+        const long long qz = (long long)(pm - 1) * a.qs[2];
+        const long long az = (long long)(min(pos, mz + 2) + 1) * a.as[2];
+        real* d = ring + so + own;
+        cp_async_el(d, qold + qxy + qz);
+        cp_async_el(d + PL, aux + axy + az);
+        cp_async_el(d + 2 * PL, aux + axy + az + a.afstride);
+        cp_async_el(uvw + ((pos & 1) * 3 + 2) * PL + own, qold + qxy + qz + 3 * a.fstride);
+        if (edge) {
+            real* h = ring + so + hal;
+            cp_async_el(h, qold + qxh + qz);
+            cp_async_el(h + PL, aux + axh + az);
+            cp_async_el(h + 2 * PL, aux + axh + az + a.afstride);
         }
     };
-    // Z and c of ring position pos, copied asynchronously
-    auto load_aux = [&](int pos) {
-        real* dst = saux + (pos & (RING3 - 1)) * NPL * NS3;
-        const long long pofs = (long long)(pos + 1) * a.as[AXN];
-        for (int e = tid; e < NS3; e += NT3P) {
-            const int sa = e % S3A, sb = e / S3A;
-            const int Ai = min(A0 - 2 + sa, mA + 2), Bi = min(B0 - 2 + sb, mB + 2);
-            const long long o = pofs + (long long)(Ai + 1) * a.as[AXA] + (long long)(Bi + 1) * a.as[AXB];
-            cp_async_el(dst + e, aux + o);
-            cp_async_el(dst + NS3 + e, aux + o + a.afstride);
-        }
+    auto issue_uv = [&](int pos) {
+        bool neg;
+        const int pm = zsrc(pos, neg);
+        const long long qz = (long long)(pm - 1) * a.qs[2];
+        real* d = uvw + (pos & 1) * 3 * PL;
+        cp_async_el(d + own, qold + qxy + qz + a.fstride);
+        cp_async_el(d + PL + own, qold + qxy + qz + 2 * a.fstride);
+        if (edge) cp_async_el(d + PL + hal, qold + qxh + qz + 2 * a.fstride);
     };
-    // 1 / (Z + Z_next) along A and B of ring position pos, from its landed Z.
-    // The next tile element is the next cell, or the same clamped cell past
-    // the grid's last ghost; the tile's last row and column are never read.
-    auto make_rcp = [&](int pos) {
-        real* dst = saux + (pos & (RING3 - 1)) * NPL * NS3;
-        for (int e = tid; e < NS3; e += NT3P) {
-            const int sa = e % S3A, sb = e / S3A;
-            if (sa == S3A - 1 || sb == S3B - 1) continue;
-            const real z = dst[e];
-            const real rA = real(1) / (z + dst[e + 1]);
-            const real rB = real(1) / (z + dst[e + S3A]);
-            dst[(E1A ? 2 : 3) * NS3 + e] = rA;
-            dst[(E1A ? 3 : 2) * NS3 + e] = rB;
-        }
+    // w at plane pos from its stored value (the walls' and the piston's sign)
+    auto wbc = [&](int pos, real w) {
+        bool neg;
+        (void)zsrc(pos, neg);
+        if (neg) w = -w;
+        if (pos > mz && a.bc[5] == BC_PISTON) w = (real)(2.0 * piston_speed(a, i, j, tbc)) - w;
+        return w;
     };
-    // q of this slice at position pos: role 0 stages p, role 1 the normal
-    // velocity; boundary conditions are applied when the pair takes them
-    auto issue_q = [&](int pos) {
-        if (!active) return;
-        bool fN;
-        const int pm = bc3_src(pos, mN, a.bc[2 * AXN], a.bc[2 * AXN + 1], fN);
-        const long long off = qoffAB + (long long)(pm - 1) * a.qs[AXN] + (H ? CN * a.fstride : 0);
-        cp_async_el(sq + ((pos & 1) * 2 + H) * NT3 + sl, qold + off);
-    };
-    auto take_q = [&](int pos, real& qp, real& qn) {
-        qp = sq[((pos & 1) * 2) * NT3 + sl];
-        qn = sq[((pos & 1) * 2 + 1) * NT3 + sl];
-        bool fN;
-        (void)bc3_src(pos, mN, a.bc[2 * AXN], a.bc[2 * AXN + 1], fN);
-        if (fN) qn = -qn;
-        if (CN == 3) {
-            const bool pist = (AXN == 2 && pos > mN && a.bc[5] == BC_PISTON) || pistonB;
-            if (pist) {
-                const int ci = AXN == 0 ? pos : A;
-                const int cj = AXN == 1 ? pos : (AXA == 1 ? A : B);
-                qn = (real)(2.0 * piston_speed(a, ci, cj, tbc)) - qn;
-            }
-        }
-    };
-    const int sown = (tb + 1) * S3A + (ta + 1);
-    auto plane = [&](int pos, int k) -> const real* {
-        return saux + (pos & (RING3 - 1)) * NPL * NS3 + k * NS3 + sown;
-    };
-    // split in the own direction of a fluctuation at the cell `w` across
-    auto split_own = [&](real xp, int pos, int w) -> Split {
-        const real* Zp = plane(pos, 0);
-        const real* Cp = plane(pos, 1);
-        const real* Rp = plane(pos, 2 + H);  // 1 / (Z + Z_next) along the own direction
-        return S::split_r(xp, Rp[-OWNS + w * OTHS], Zp[-OWNS + w * OTHS], Cp[-OWNS + w * OTHS],
-                          Rp[w * OTHS], Zp[OWNS + w * OTHS], Cp[OWNS + w * OTHS]);
+    auto lim_a = [&](real s, real n) { return limited_strength<real, LIM>(s, n, lim1); };
+    auto lim_b = [&](real s, real n) { return limited_strength<real, LIM>(s, n, lim2); };
+    // factor of a limited wave in the correction flux of a direction: |s| (1 - |s| dt/dn) / 2
+    auto coef = [&](real c, real tn) { return half2 * fabs(c) * (real(1) - fabs(c) * tn); };
+    // p, u (along A-B) and v (along A-C) of an edge flux
+    auto edge_flux = [&](real ra, real rb, real rg, real re, real zA, real cA, real zB, real cB, real zC,
+                         real cC, real zD, real cD, real YA, real YB, real YC, real YD, real& ep,
+                         real& eu, real& ev) {
+        const real m1 = (ra * re) * (cC * zC), m2 = (rb * rg) * (cB * zB);
+        const real m3 = (rb * re) * (cD * zD), m4 = (ra * rg) * (cA * zA);
+        const real yA = cD * YA, yB = cC * YB, yC = cB * YC, yD = cA * YD;
+        ep = (m1 + m2) * (zD * yA + zA * yD) - (m3 + m4) * (zC * yB + zB * yC);
+        eu = (m1 * yA - m2 * yD) + (m3 * yB - m4 * yC);
+        ev = (m2 * yA - m1 * yD) + (m3 * yC - m4 * yB);
     };
 
-    double cfl = 0.0;
-    auto solve = [&](int i, real pL, real uL, real pR, real uR, real w[2][2], real am[2], real ap[2]) {
-        real s[2];
-        const real zl = *plane(i - 1, 0), cl = *plane(i - 1, 1);
-        const real zr = *plane(i, 0), cr = *plane(i, 1);
-        S::rpn_r(pL, uL, pR, uR, zl, cl, zr, cr, w, s, am, ap);
-        if (i >= 1 && i <= mN + 1) {
-            for (int k = 0; k < 2; ++k) {  // Courant number in FP64 (FP32 builds too)
-                const double c = tn_d * (double)s[k];
-                cfl = fmax(fmax(cfl, c), -c);
-            }
-        }
-    };
-
-    load_aux(p0 - 2);
-    load_aux(p0 - 1);
-    load_aux(p0);
-    load_aux(p0 + 1);
-    issue_q(p0 + 1);
+    // ---- planes t0-1 .. t0+2 (t0 = k0 - 1): z strengths at t0-1/2 and t0+1/2
+    int sm = 0, s0 = 3 * PL, s1 = 6 * PL, s2 = 9 * PL, s3 = 12 * PL;  // slots of planes t-1 .. t+3
+    const int t0 = k0 - 1;
+    real w0, w1, wm;  // w at planes t, t+1 (t-1)
+    real a1z, a2z, a2zm, rz, rz1, g0;
+    {
+        bool neg;
+        auto w_at = [&](int pos) {
+            return wbc(pos, qold[qxy + (long long)(zsrc(pos, neg) - 1) * a.qs[2] + 3 * a.fstride]);
+        };
+        wm = w_at(t0 - 1);
+        w0 = w_at(t0);
+        w1 = w_at(t0 + 1);
+    }
+    issue_pzc(t0 - 1, sm);
+    issue_pzc(t0, s0);
+    issue_uv(t0);
+    // the w copies of planes t0-1 and t0 must not land after those of t0+1 and t0+2
     cp_async_wait_all();
     __syncthreads();
-    make_rcp(p0 - 1);
-    make_rcp(p0);
+    issue_pzc(t0 + 1, s1);
+    issue_pzc(t0 + 2, s2);
+    cp_async_wait_all();
     __syncthreads();
-
-    real wA[2][2], wB[2][2];
-    real amB[2], apB[2];
-    real qLp = 0, qLn = 0;
-    real F0[2] = {0, 0};
-    real Qs[2] = {0, 0};
-    real O[2][3][2];  // own side's gadd or hadd (side, level, comp) of cell p
-    for (int s_ = 0; s_ < 2; ++s_)
-        for (int l = 0; l < 3; ++l)
-            for (int c = 0; c < 2; ++c) O[s_][l][c] = 0;
-    if (active) {
-        real q0p, q0n, q1p, q1n;
-        load_pn(p0 - 2, q0p, q0n);
-        load_pn(p0 - 1, q1p, q1n);
-        load_pn(p0, qLp, qLn);
-        real am_[2], ap_[2];
-        solve(p0 - 1, q0p, q0n, q1p, q1n, wA, am_, ap_);
-        solve(p0, q1p, q1n, qLp, qLn, wB, amB, apB);
+    {
+        const real pA = ring[sm + own], zA = ring[sm + PL + own];
+        const real pB = ring[s0 + own], zB = ring[s0 + PL + own];
+        const real pC = ring[s1 + own], zC = ring[s1 + PL + own];
+        rz = rcp_newton(zA + zB);
+        rz1 = rcp_newton(zB + zC);
+        a2zm = (zA * (w0 - wm) + (pB - pA)) * rz;
+        a1z = (zC * (w1 - w0) - (pC - pB)) * rz1;
+        a2z = (zB * (w1 - w0) + (pC - pB)) * rz1;
+        g0 = rcp_newton(real(1) + zB * zB);
     }
-    __syncthreads();
+    real t2zm = 0, cpzm = 0, cwzm = 0;          // z interface t-1/2: right-going fluctuation, correction flux
+    real cmax = 0;
+    real fxp = 0, fxu = 0, fyp = 0, fyv = 0;    // plane t-1: face fluxes so far
+    real fzp = 0, fzw = 0;                      // z face t-3/2
+    real XZm = 0;                               // plane t-1
+    const bool inxy = i >= 0 && i <= mx + 1 && j <= my + 1 && lane >= 1;
 
-    const bool xch = m3 > 0 && m4 > 0;  // the pair exchanges split combinations
-    // exchange planes: [side L/R][role][value] of NT3 slices each
-    auto xplane = [&](int side, int role, int v) -> real* {
-        return sxch + ((side * 2 + role) * 2 + v) * NT3 + sl;
-    };
-
-    for (int p = p0 - 1; p < p1; ++p) {
-        const bool emit = p >= p0;
-        // position p+3: its ring slot and staged q were last read before the
-        // previous position's barrier
-        if (p + 3 <= p1 + 1) {
-            load_aux(p + 3);
-            issue_q(p + 3);
+#pragma unroll kUnroll
+    for (int t = t0; t <= k1; ++t) {
+        if (t + 3 <= k1 + 1) issue_pzc(t + 3, s3);
+        if (t + 1 <= k1) issue_uv(t + 1);
+        const int par = t & 1;
+        real* SPt = SP + par * 3 * PL;
+        real* SPm = SP + (par ^ 1) * 3 * PL;
+        // ------------------------------------------------- A: strengths
+        const real* P = ring + s0;
+        const real p = P[own], z = P[PL + own], c = P[2 * PL + own];
+        const real* UV = uvw + par * 3 * PL;
+        real u = UV[own], v = UV[PL + own];
+        if (negx) u = -u;
+        if (negy) v = -v;
+        if (inxy) cmax = fmax(cmax, fabs(c));
+        const real zl = P[PL + lm], cl = P[2 * PL + lm];
+        real rx, a1x, a2x;
+        {
+            const real du = u - __shfl_up_sync(FULL, u, 1), dp = p - P[lm];
+            rx = rcp_newton(zl + z);
+            a1x = (z * du - dp) * rx;
+            a2x = (zl * du + dp) * rx;
         }
-        // the reciprocals of position p+2 (its Z landed before the last barrier)
-        if (p + 2 <= p1 + 1) make_rcp(p + 2);
-        const real* vsrc = DIR == 0 ? qold : qnew;
-        real vA = 0, vB = 0;
-        // the cell values of position p+1, staged for the next position (only
-        // this thread writes that cell, at that position)
-        if (apply && p + 1 >= p0 && p + 1 < p1) {
-            const long long off = qoffAB + (long long)p * a.qs[AXN];
-            real* dv = sv + (((p + 1) & 1) * 2 + H) * 2 * NT3 + sl;
-            cp_async_el(dv, vsrc + off + CA * a.fstride);
-            cp_async_el(dv + NT3, vsrc + off + CB * a.fstride);
+        const real zb = P[PL + own - 32], cb = P[2 * PL + own - 32];
+        real ry, a1y, a2y;
+        {
+            real vb = UV[PL + own - 32];
+            if (negb) vb = -vb;
+            const real dv = v - vb, dp = p - P[own - 32];
+            ry = rcp_newton(zb + z);
+            a1y = (z * dv - dp) * ry;
+            a2y = (zb * dv + dp) * ry;
         }
-        real F1[2] = {0, 0};
-        real Qp[2] = {0, 0};
-        real wC[2][2] = {}, amC[2] = {}, apC[2] = {}, qRp = 0, qRn = 0;
-        real cterm = 0, own_c = 0;  // centre terms: sent to the partner / kept
-        real cq[2] = {0, 0};
-        Split qm = {0, 0, 0, 0};
-        const int L = p, R = p + 1;
-        if (active) {
-            take_q(p + 2, qRp, qRn);
-            solve(p + 2, qLp, qLn, qRp, qRn, wC, amC, apC);
-            real wl[2][2];
-            const real sB[2] = {-*plane(p, 1), *plane(p + 1, 1)};
-            for (int k = 0; k < 2; ++k) {
-                wl[k][0] = wB[k][0];
-                wl[k][1] = wB[k][1];
-                const int lim = M::lim >= 0 ? M::lim : a.mthlim[k];
-                if (order == 2 && lim > 0) {
-                    const real wn2 = wB[k][0] * wB[k][0] + wB[k][1] * wB[k][1];
-                    if (wn2 != real(0)) {
-                        const real dl = wA[k][0] * wB[k][0] + wA[k][1] * wB[k][1];
-                        const real dr = wB[k][0] * wC[k][0] + wB[k][1] * wC[k][1];
-                        const real r = (sB[k] > real(0) ? dl : dr) / wn2;
-                        const real phi = phi_limiter<real>(lim, r);
-                        wl[k][0] = phi * wB[k][0];
-                        wl[k][1] = phi * wB[k][1];
-                    }
-                }
-            }
-            if (order == 2) {
-                for (int k = 0; k < 2; ++k) {
-                    const real as_ = fabs(sB[k]);
-                    const real coef = (real(0.5) * as_) * (real(1) - as_ * dtdxave);
-                    cq[0] = cq[0] + coef * wl[k][0];
-                    cq[1] = cq[1] + coef * wl[k][1];
-                }
-            }
-            F1[0] = cq[0];
-            F1[1] = cq[1];
-            Qp[0] = Qs[0] - tn * amB[0];
-            Qp[1] = Qs[1] - tn * amB[1];
-            Qs[0] = real(0) - tn * apB[0];
-            Qs[1] = real(0) - tn * apB[1];
-
-            // ---- cell p: the amdq side of interface p+1 completes gadd/hadd
-            if (m3 > 0) {
-                const Split ma = split_own(amB[0], L, 0);
-                if (m3 == 2) qm = split_own(cq[0], L, 0);
-                O[0][1][0] = O[0][1][0] - H5 * ma.dp;
-                O[0][1][1] = O[0][1][1] - H5 * ma.dt;
-                O[1][1][0] = O[1][1][0] - H5 * ma.up;
-                O[1][1][1] = O[1][1][1] - H5 * ma.ut;
-                if (m4 > 0) {
-                    // the combinations the partner splits (flux3.f90:363-376, 488-495)
-                    real x1 = ma.up, x3 = ma.dp;
-                    if (m4 == 2) {
-                        x1 = ma.up + real(3) * qm.up;
-                        x3 = ma.dp + real(3) * qm.dp;
-                    }
-                    *xplane(0, H, 0) = x1;
-                    *xplane(0, H, 1) = x3;
-                }
-            }
+        SA1[own] = a1y;
+        SA2[own] = a2y;
+        SG[own] = g0;
+        SRZ[own] = rz;
+        SPt[PL + own] = rx;
+        SPt[2 * PL + own] = ry;
+        if (r == ROWS - 1) {  // the left-going strength one row above, and that face's r
+            real va = UV[PL + own + 32];
+            if (negh) va = -va;
+            const real za = P[PL + own + 32];
+            SA1[own + 32] = (za * (va - v) - (P[own + 32] - p)) * rcp_newton(z + za);
         }
-        if (xch) {
-            pair_sync(pair_id);
-            if (active) {
-                const real y1 = *xplane(0, 1 - H, 0), y3 = *xplane(0, 1 - H, 1);
-                const Split tpm = split_own(y1, L, 1), tmm = split_own(y3, L, -1);
-                O[1][1][0] = O[1][1][0] + S6own * (tpm.up - tmm.up);
-                O[1][1][1] = O[1][1][1] + S6own * (tpm.ut - tmm.ut);
-                O[0][1][0] = O[0][1][0] + S6own * (tpm.dp - tmm.dp);
-                O[0][1][1] = O[0][1][1] + S6own * (tpm.dt - tmm.dt);
-                O[1][2][0] = O[1][2][0] - S6own * tpm.up;
-                O[1][2][1] = O[1][2][1] - S6own * tpm.ut;
-                O[0][2][0] = O[0][2][0] - S6own * tpm.dp;
-                O[0][2][1] = O[0][2][1] - S6own * tpm.dt;
-                O[1][0][0] = O[1][0][0] + S6own * tmm.up;
-                O[1][0][1] = O[1][0][1] + S6own * tmm.ut;
-                O[0][0][0] = O[0][0][0] + S6own * tmm.dp;
-                O[0][0][1] = O[0][0][1] + S6own * tmm.dt;
-            }
+        // z interface t+3/2
+        const real z1 = ring[s1 + PL + own], c1 = ring[s1 + 2 * PL + own];
+        const real z2 = ring[s2 + PL + own];
+        const real w2 = wbc(t + 2, uvw[(par * 3 + 2) * PL + own]);
+        real a1zn, a2zn, rz2;
+        {
+            const real dw = w2 - w1, dp = ring[s2 + own] - ring[s1 + own];
+            rz2 = rcp_newton(z1 + z2);
+            a1zn = (z2 * dw - dp) * rz2;
+            a2zn = (z1 * dw + dp) * rz2;
         }
-        Split qp = {0, 0, 0, 0};
-        if (active) {
-            if (m3 == 2) {
-                O[1][1][0] = O[1][1][0] - tn * qm.up;
-                O[1][1][1] = O[1][1][1] - tn * qm.ut;
-                O[0][1][0] = O[0][1][0] - tn * qm.dp;
-                O[0][1][1] = O[0][1][1] - tn * qm.dt;
-            }
-            if (emit) {
-                // terms for the eight neighbours: own offset o (the side), other w (the level)
-                real* out = sterm + (NTB == 2 ? (p & 1) : 0) * NTERM3 * NT3 + sl;
-#pragma unroll
-                for (int w = -1; w <= 1; ++w)
-#pragma unroll
-                    for (int o = -1; o <= 1; ++o) {
-                        if (o == 0 && w == 0) continue;
-                        const int de1 = H ? w : o, de2 = H ? o : w;
-                        const int idx9 = (de2 + 1) * 3 + (de1 + 1);
-                        const int nb = idx9 < 4 ? idx9 : idx9 - 1;
-#pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            const real tv = o < 0 ? -(t_own * O[0][w + 1][c])
-                                          : o == 0 ? -(t_own * (O[1][w + 1][c] - O[0][w + 1][c]))
-                                                   : t_own * O[1][w + 1][c];
-                            out[(nb * 4 + 2 * H + c) * NT3] = tv;
-                        }
-                    }
-                // centre: h = 0 keeps te1*dG_p and sends te1*dG_e1; h = 1
-                // keeps te2*dH_e2 and sends te2*dH_p
-                const real dp_ = t_own * (O[1][1][0] - O[0][1][0]);
-                const real dv_ = t_own * (O[1][1][1] - O[0][1][1]);
-                cterm = H ? dp_ : dv_;
-                own_c = H ? dv_ : dp_;
-            }
-            // ---- cell p+1: the apdq side of interface p+1 starts gadd/hadd
-            for (int s_ = 0; s_ < 2; ++s_)
-                for (int l = 0; l < 3; ++l)
-                    for (int c = 0; c < 2; ++c) O[s_][l][c] = 0;
-            if (m3 > 0) {
-                const Split mp = split_own(apB[0], R, 0);
-                if (m3 == 2) qp = split_own(cq[0], R, 0);
-                O[0][1][0] = O[0][1][0] - H5 * mp.dp;
-                O[0][1][1] = O[0][1][1] - H5 * mp.dt;
-                O[1][1][0] = O[1][1][0] - H5 * mp.up;
-                O[1][1][1] = O[1][1][1] - H5 * mp.ut;
-                if (m4 > 0) {
-                    real x0 = mp.up, x2 = mp.dp;
-                    if (m4 == 2) {
-                        x0 = mp.up - real(3) * qp.up;
-                        x2 = mp.dp - real(3) * qp.dp;
-                    }
-                    *xplane(1, H, 0) = x0;
-                    *xplane(1, H, 1) = x2;
-                }
-            }
+        const real g1 = rcp_newton(real(1) + z1 * z1);
+        __syncthreads();
+        // ---------------------------- B: limited waves, x and z sums
+        real bp = p, bu = u, bv = v, bw = w0;
+        real Xx, Yx, Xz, Yz;
+        {
+            const real h = real(1) + zl * z;
+            const real n1 = __shfl_down_sync(FULL, a1x, 1) * (h * __shfl_up_sync(FULL, g0, 1));
+            const real n2 = __shfl_up_sync(FULL, a2x, 1) * (h * g0);
+            const real e1 = coef(cl, tx) * lim_a(a1x, n1), e2 = coef(c, tx) * lim_b(a2x, n2);
+            const real cp = z * e2 - zl * e1, cu = e1 + e2;
+            const real ta = cl * a1x, tb = c * a2x;
+            const real tr = __shfl_down_sync(FULL, ta, 1);
+            const real sp = z * (tb + tr), su = tb - tr;
+            const real dp = __shfl_down_sync(FULL, cp, 1) - cp, du = __shfl_down_sync(FULL, cu, 1) - cu;
+            bp -= tx * (sp + dp);
+            bu -= tx * (su + du);
+            Xx = -tx * (real(0.5) * sp + xd * dp);
+            Yx = sp + yd * dp;
         }
-        if (xch) {
-            pair_sync(pair_id);
-            if (active) {
-                const real y0 = *xplane(1, 1 - H, 0), y2 = *xplane(1, 1 - H, 1);
-                const Split tpp = split_own(y0, R, 1), tmp = split_own(y2, R, -1);
-                O[1][1][0] = O[1][1][0] + S6own * (tpp.up - tmp.up);
-                O[1][1][1] = O[1][1][1] + S6own * (tpp.ut - tmp.ut);
-                O[0][1][0] = O[0][1][0] + S6own * (tpp.dp - tmp.dp);
-                O[0][1][1] = O[0][1][1] + S6own * (tpp.dt - tmp.dt);
-                O[1][2][0] = O[1][2][0] - S6own * tpp.up;
-                O[1][2][1] = O[1][2][1] - S6own * tpp.ut;
-                O[0][2][0] = O[0][2][0] - S6own * tpp.dp;
-                O[0][2][1] = O[0][2][1] - S6own * tpp.dt;
-                O[1][0][0] = O[1][0][0] + S6own * tmp.up;
-                O[1][0][1] = O[1][0][1] + S6own * tmp.ut;
-                O[0][0][0] = O[0][0][0] + S6own * tmp.dp;
-                O[0][0][1] = O[0][0][1] + S6own * tmp.dt;
+        {
+            const real h = real(1) + z * z1;
+            const real e1 = coef(c, tz) * lim_a(a1z, a1zn * (h * g0));
+            const real e2 = coef(c1, tz) * lim_b(a2z, a2zm * (h * g1));
+            const real cp = z1 * e2 - z * e1, cw = e1 + e2;
+            const real ta = c * a1z;
+            const real sp = z * (t2zm + ta), sw = t2zm - ta;
+            const real dp = cp - cpzm, dw = cw - cwzm;
+            bp -= tz * (sp + dp);
+            bw -= tz * (sw + dw);
+            Xz = -tz * (real(0.5) * sp + xd * dp);
+            Yz = sp + yd * dp;
+            t2zm = c1 * a2z;
+            cpzm = cp;
+            cwzm = cw;
+        }
+        real cpy = 0, cvy = 0, tby = 0;
+        if (r >= 1) {  // y interface below this row
+            const real h = real(1) + zb * z;
+            const real n1 = SA1[own + 32] * (h * SG[own - 32]);
+            const real n2 = SA2[own - 32] * (h * g0);
+            const real e1 = coef(cb, ty) * lim_a(a1y, n1), e2 = coef(c, ty) * lim_b(a2y, n2);
+            cpy = z * e2 - zb * e1;
+            cvy = e1 + e2;
+            tby = c * a2y;
+            ST1[own] = cb * a1y;
+            SCP[own] = cpy;
+            SCV[own] = cvy;
+        }
+        if (TRANS) {
+            SXY[own] = Xx + Xz;
+            SYZ[own] = Yz;
+            SPt[own] = Yx;
+        }
+        __syncthreads();
+        // ------------- C: y sums, fluxes at plane t and at z face t-1/2
+        real Xy = 0, Yy = 0;
+        if (r >= 1 && r < ROWS - 1) {
+            const real tr = ST1[own + 32];
+            const real sp = z * (tby + tr), sv = tby - tr;
+            const real dp = SCP[own + 32] - cpy, dv = SCV[own + 32] - cvy;
+            bp -= ty * (sp + dp);
+            bv -= ty * (sv + dv);
+            Xy = -ty * (real(0.5) * sp + xd * dp);
+            Yy = sp + yd * dp;
+        }
+        real nfxp = 0, nfxu = 0, nfyp = 0, nfyv = 0, nfzp = 0, nfzw = 0;
+        real nexzp = 0, nexzu = 0, exzw = 0, neyzp = 0, neyzv = 0, eyzw = 0, exyp = 0, exyu = 0, exyv = 0;
+        const real XX = Xy + Xz, XZ = Xx + Xy;
+        if (TRANS && r < ROWS - 1) {
+            const real* M = ring + sm;  // plane t-1
+            const real zR = P[PL + lp], cR = P[2 * PL + lp];
+            const real zU = P[PL + own + 32], cU = P[2 * PL + own + 32];
+            const real rxR = SPt[PL + lp], ryU = SPt[2 * PL + own + 32];
+            const real zm = M[PL + own], cm = M[2 * PL + own];
+            {  // faces i+1/2, j+1/2, t-1/2
+                const real XR = __shfl_down_sync(FULL, XX, 1);
+                const real hi = cR * (rxR * XX), lo = c * (rxR * XR);
+                nfxu = tx * (hi + lo);
+                nfxp = tx * (zR * hi - z * lo);
+                const real hu = cU * (ryU * (Xx + Xz)), lu = c * (ryU * SXY[own + 32]);
+                nfyv = ty * (hu + lu);
+                nfyp = ty * (zU * hu - z * lu);
+                const real hz = c * (rz * XZm), lz = cm * (rz * XZ);
+                nfzw = tz * (hz + lz);
+                nfzp = tz * (z * hz - zm * lz);
             }
+            {  // edge (i+1/2, j+1/2) of plane t
+                const real zD = P[PL + lp + 32], cD = P[2 * PL + lp + 32];
+                edge_flux(ryU, SPt[2 * PL + lp + 32], rxR, SPt[PL + lp + 32], z, c, zR, cR, zU, cU, zD, cD, Yz,
+                          SYZ[lp], SYZ[own + 32], SYZ[lp + 32], exyp, exyu, exyv);
+            }
+            {  // edge (i+1/2, t-1/2)
+                const real YR = __shfl_down_sync(FULL, Yy, 1);
+                edge_flux(rz, SRZ[lp], SPm[PL + lp], rxR, zm, cm, M[PL + lp], M[2 * PL + lp], z, c, zR, cR,
+                          SB[8 * PL + own], SB[8 * PL + lp], Yy, YR, nexzp, nexzu, exzw);
+            }
+            {  // edge (j+1/2, t-1/2)
+                edge_flux(rz, SRZ[own + 32], SPm[2 * PL + own + 32], ryU, zm, cm, M[PL + own + 32],
+                          M[2 * PL + own + 32], z, c, zU, cU, SPm[own], SPm[own + 32], Yx, SPt[own + 32], neyzp,
+                          neyzv, eyzw);
+            }
+            // the y faces of plane t-1 are complete
+            fyp += f6 * (neyzp - SB[6 * PL + own]);
+            fyv += f6 * (neyzv - SB[7 * PL + own]);
+            SB[6 * PL + own] = neyzp;
+            SB[7 * PL + own] = neyzv;
+            SE[own] = fyp;
+            SE[PL + own] = fyv;
+            SE[2 * PL + own] = eyzw;
+            SE[3 * PL + own] = exyp;
+            SE[4 * PL + own] = exyu;
         }
-        if (active && m3 == 2) {
-            O[1][1][0] = O[1][1][0] + tn * qp.up;
-            O[1][1][1] = O[1][1][1] + tn * qp.ut;
-            O[0][1][0] = O[0][1][0] + tn * qp.dp;
-            O[0][1][1] = O[0][1][1] + tn * qp.dt;
-        }
-        // centre term for the partner, double-buffered by the position's parity
-        // centre term for the partner.  Its last value was read in the
-        // partner's previous gather, which precedes the partner's arrival at
-        // this position's pair barriers (one is added where the method has
-        // no split exchange).
-        if (!xch) pair_sync(pair_id);
-        sxch[(8 + H) * NT3 + sl] = cterm;
         cp_async_wait_all();
         __syncthreads();
-        if (emit && apply) {
-            const real crecv = sxch[(8 + 1 - H) * NT3 + sl];
-            {
-                const real* vv = sv + ((p & 1) * 2 + H) * 2 * NT3 + sl;
-                vA = vv[0];
-                vB = vv[NT3];
-            }
-            const real* in = sterm + (NTB == 2 ? (p & 1) : 0) * NTERM3 * NT3 + sl;
-            auto add_term = [&](int code) {
-                if (code == 4) {
-                    if (H == 0) {
-                        vA = vA + Qp[0] - tn * (F1[0] - F0[0]) - own_c - crecv;
-                        vB = vB + Qp[1] - tn * (F1[1] - F0[1]);
-                    } else {
-                        vA = vA - crecv;
-                        vB = vB - own_c;
-                    }
-                } else {
-                    const int da = code % 3 - 1, db = code / 3 - 1;
-                    const int u = E1A ? -da : -db, w = E1A ? -db : -da;
-                    const int idx9 = (w + 1) * 3 + (u + 1);
-                    const int nb = idx9 < 4 ? idx9 : idx9 - 1;
-                    const int so = db * T3A + da;
-                    if (H == 0) {
-                        vA = vA + in[(nb * 4 + 0) * NT3 + so] + in[(nb * 4 + 2) * NT3 + so];
-                    } else {
-                        vA = vA + in[(nb * 4 + 1) * NT3 + so];
-                        vB = vB + in[(nb * 4 + 3) * NT3 + so];
-                    }
-                }
-            };
-#pragma unroll
-            for (int k = 0; k < 9; ++k) add_term(k);
-            const long long off = qoffAB + (long long)(p - 1) * a.qs[AXN];
-            qnew[off + CA * a.fstride] = vA;
-            qnew[off + CB * a.fstride] = vB;
+        // -------------------------------------------- D: plane t-1
+        real op = SB[own], ou = SB[PL + own], ov = SB[2 * PL + own], ow = SB[3 * PL + own];
+        SB[own] = bp;
+        SB[PL + own] = bu;
+        SB[2 * PL + own] = bv;
+        SB[3 * PL + own] = bw;
+        if (TRANS && r >= 1 && r < ROWS - 1) {
+            fxp += f6 * (nexzp - SB[4 * PL + own]);
+            fxu += f6 * (nexzu - SB[5 * PL + own]);
+            SB[4 * PL + own] = nexzp;
+            SB[5 * PL + own] = nexzu;
+            nfzw += f6 * ((exzw - __shfl_up_sync(FULL, exzw, 1)) + (eyzw - SE[2 * PL + own - 32]));
+            op -= ((fxp - __shfl_up_sync(FULL, fxp, 1)) + (fyp - SE[own - 32])) + (nfzp - fzp);
+            ou -= fxu - __shfl_up_sync(FULL, fxu, 1);
+            ov -= fyv - SE[PL + own - 32];
+            ow -= nfzw - fzw;
+            // plane t's x faces take the y difference of its edge fluxes
+            fxp = nfxp + f6 * (exyp - SE[3 * PL + own - 32]);
+            fxu = nfxu + f6 * (exyu - SE[4 * PL + own - 32]);
         }
-        if (active) {
-            for (int k = 0; k < 2; ++k)
-                for (int c = 0; c < 2; ++c) { wA[k][c] = wB[k][c]; wB[k][c] = wC[k][c]; }
-            amB[0] = amC[0]; amB[1] = amC[1];
-            apB[0] = apC[0]; apB[1] = apC[1];
-            qLp = qRp; qLn = qRn;
-            F0[0] = F1[0]; F0[1] = F1[1];
+        if (TRANS) {
+            fyp = nfyp;
+            fyv = nfyv + f6 * (exyv - __shfl_up_sync(FULL, exyv, 1));  // ... and its y faces the x difference
+            fzp = nfzp;
+            fzw = nfzw;
+            XZm = XZ;
+            SB[8 * PL + own] = Yy;
         }
-        // one term buffer: every gather of p ends before a publish of p+1
-        if constexpr (NTB == 1) __syncthreads();
+        if (out && t > k0) {
+            const long long o = (long long)(i - 1) + (long long)(j - 1) * a.qs[1] + (long long)(t - 2) * a.qs[2];
+            qnew[o] = op;
+            qnew[o + a.fstride] = ou;
+            qnew[o + 2 * a.fstride] = ov;
+            qnew[o + 3 * a.fstride] = ow;
+        }
+        w0 = w1;
+        w1 = w2;
+        a2zm = a2z;
+        a1z = a1zn;
+        a2z = a2zn;
+        rz = rz1;
+        rz1 = rz2;
+        g0 = g1;
+        const int so = sm;
+        sm = s0;
+        s0 = s1;
+        s1 = s2;
+        s2 = s3;
+        s3 = so;
     }
-    return cfl;
-}
-
-template <class S, int DIR, class M, bool LAST>
-__global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3f_kernel(const Sweep3Args<typename S::real> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    using real = typename S::real;
-    double* red = reinterpret_cast<double*>(reinterpret_cast<real*>(smem_raw) +
-                                            RING3 * NPL3F * NS3 + term3_bufs<real>() * NTERM3 * NT3 +
-                                            (XCH3 + QST3 + VST3) * NT3);
-    ClawCtl* ctl = a.ctl;
-    grid_dependency_sync();
-    if (ctl->done) return;
-    // warps 2k (role 0) and 2k+1 (role 1) share 32 slices
-    const double cfl = ((threadIdx.x >> 5) & 1) ? sweep3f_march<S, DIR, M, 1>(a, smem_raw)
-                                                : sweep3f_march<S, DIR, M, 0>(a, smem_raw);
-    if (LAST) {
-        cta_cfl_and_control(ctl, cfl, red);
-    } else {
-        double c = cfl;
-        for (int off = 16; off > 0; off >>= 1) c = fmax(c, __shfl_xor_sync(0xffffffffu, c, off));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double m = 0.0;
-            for (int w = 0; w < NT3P / 32; ++w) m = fmax(m, red[w]);
-            if (!(m > 0.0)) m = (m != m) ? m : 0.0;
-            atomicMax(&ctl->cfl_bits, (unsigned long long)__double_as_longlong(m));
-        }
-    }
+    const double cd = (double)cmax;
+    const double cfl = fmax(fmax((dt / a.d[0]) * cd, (dt / a.d[1]) * cd), (dt / a.d[2]) * cd);
+    cta_cfl_and_control(ctl, cfl, red);
 }
 
 }  // namespace clawb200
