@@ -11,10 +11,6 @@
 #include "char2d.cuh"
 #include "host.h"
 
-#ifndef CLAW_CHAR_MIN_ROWS
-#define CLAW_CHAR_MIN_ROWS 8  // fewest rows of a work item (small grids: more items, more warps)
-#endif
-
 namespace clawb200 {
 
 template <typename real, int LIM, int BCM, int ORD, int TRN, int LIM2 = LIM>
@@ -58,7 +54,7 @@ struct CharRunner : Runner {
                                                                32 * WARPS2D, smem));
         if (per_sm < 1) return fail(CLAW_E_CUDA, "characteristic kernel cannot be resident");
         const long long full = (long long)nsm * per_sm * WARPS2D;
-        const int nw = row_blocks(full, args.nstrips, g.my, CLAW_CHAR_MIN_ROWS, &args.brows, &args.nblocks);
+        const int nw = row_blocks(full, args.nstrips, g.my, &args.brows, &args.nblocks);
         grid = (nw + WARPS2D - 1) / WARPS2D;
         args.nwarps = nw;
         return 0;

@@ -31,18 +31,20 @@ struct Runner {
     virtual int launches_per_step() const { return 1; }
 };
 
-#ifndef CLAW_STEP2_MIN_ROWS
-#define CLAW_STEP2_MIN_ROWS 16  // fewest rows of a work item of the generic and split 2D kernels
-#endif
-
 // Row-block-major work items of a 2D column-march kernel: as many row blocks
-// as fill `full` resident warps with one item (strip x row block) each, every
-// block at least min_rows high.  Returns the warps to launch.
-inline int row_blocks(long long full, int nstrips, int my, int min_rows, int* brows, int* nblocks) {
+// as fill `full` resident warps with one item (strip x row block) each, down
+// to one row.  A warp's march takes its rows and three or four halo rows one
+// after the other (2-4 us each in the generic FP64 kernel), so while warps
+// are idle shorter blocks shorten the step although they repeat halo rows.
+// Against blocks of at least 16 (generic, split) or 8 rows (characteristic),
+// us per step: annulus 40x120 FP64 95 -> 24, 320x960 106 -> 56; radial FP64
+// 256^2 45 -> 20, 512^2 46 -> 31, contracted 256^2 13.5 -> 10.2, Strang FP64
+// 256^2 61 -> 25; 1024^2, where the blocks are 16 rows either way, the same.
+// Returns the warps to launch.
+inline int row_blocks(long long full, int nstrips, int my, int* brows, int* nblocks) {
     long long nb = full / nstrips;
     if (nb < 1) nb = 1;
-    const long long cap = (my + min_rows - 1) / min_rows;
-    if (nb > cap) nb = cap > 0 ? cap : 1;
+    if (nb > my) nb = my;
     *brows = (int)((my + nb - 1) / nb);
     *nblocks = (my + *brows - 1) / *brows;
     const long long items = (long long)nstrips * *nblocks;

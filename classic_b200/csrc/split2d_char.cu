@@ -51,7 +51,7 @@ struct CharSplitRunner : Runner {
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS2D, smem));
         if (per_sm < 1) return fail(CLAW_E_CUDA, "split characteristic kernel cannot be resident");
         const long long full = (long long)nsm * per_sm * WARPS2D;
-        const int nw = row_blocks(full, args.nstrips, g.my, CLAW_CHAR_MIN_ROWS, &args.brows, &args.nblocks);
+        const int nw = row_blocks(full, args.nstrips, g.my, &args.brows, &args.nblocks);
         grid = (nw + WARPS2D - 1) / WARPS2D;
         args.nwarps = nw;
         return 0;
