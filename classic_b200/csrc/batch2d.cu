@@ -397,7 +397,7 @@ int claw_batch_autotune(claw_batch* b, const double* dt_trial, int repeats, int*
     float best = 1e30f, best_tail = 1e30f;
     int best_ctas = maxc, best_rows = 48;
     for (int ctas = maxc; ctas >= 1 && ctas >= maxc / 2; --ctas) {
-        b->runner->set_shape(48, ctas);
+        b->runner->set_shape(1, ctas);
         float t = 0.f;
         int rc = time_step(trial, n, &t);
         if (rc) return rc;
@@ -411,7 +411,11 @@ int claw_batch_autotune(claw_batch* b, const double* dt_trial, int repeats, int*
         if (rc) return rc;
         if (t < best_tail) { best_tail = t; best_rows = rows; }
     }
-    b->runner->set_shape(best_rows, best_ctas);
+    b->runner->set_shape(1, best_ctas);  // the default height, kept where it is the fastest
+    float t1 = 0.f;
+    const int rc1 = time_step(tail, 1, &t1);
+    if (rc1) return rc1;
+    if (best_tail < t1) b->runner->set_shape(best_rows, best_ctas);
     if (b->gexec) {  // the captured time loop holds the old launch shape
         cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;

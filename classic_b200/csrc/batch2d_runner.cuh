@@ -22,7 +22,7 @@ struct BatchRunner {
     // launch shape: tile height (rows per warp at least) and CTAs per SM
     virtual void set_shape(int min_rows, int ctas_per_sm) = 0;
     virtual int max_ctas_per_sm() const = 0;
-    int min_rows = 48, ctas_per_sm = 0;
+    int min_rows = 1, ctas_per_sm = 0;
 };
 
 template <class S, class M>
@@ -107,7 +107,13 @@ struct BatchRunnerT : BatchRunner {
         b.count = n;
         b.active = active;
         b.err = err;
-        set_shape(48, per_sm);
+        // Tile height 1: every resident warp takes a share of the rows.  While
+        // the instances' rows outnumber the warps the height does not matter
+        // (64 instances of 128..1024: 56.3 ms at any height); when they do not,
+        // a warp's march is the step's time, so the shorter the better (16
+        // contracted Euler instances of 128..384, 47 steps: 9.6 ms at 48 rows,
+        // 5.5 at 16, 5.1 at 4 and below; 3 of 60..200: 4.8 -> 0.58 ms).
+        set_shape(1, per_sm);
         return 0;
     }
 
