@@ -72,6 +72,17 @@ struct Acoustics2D {
         bmasdq[0] = cc * (b1 * zz); bmasdq[mu] = real(0); bmasdq[mv] = -(cc * b1);
         bpasdq[0] = cc * (b2 * zz); bpasdq[mu] = real(0); bpasdq[mv] = cc * b2;
     }
+
+    // The fluctuations flux2 splits carry no transverse velocity, so b1 = -b2
+    // and the two halves of a split mirror each other bit for bit: pressure
+    // parts of opposite sign, equal velocity parts.  up(ixy, asdq, bp) is the
+    // upper half of rpt.
+    static constexpr bool trans_mirror = true;
+    __device__ __forceinline__ void up(int ixy, const real* asdq, real bp[meqn]) const {
+        const int mu = (ixy == 1) ? 1 : 2, mv = (ixy == 1) ? 2 : 1;
+        const real b2 = asdq[0] * hz;
+        bp[0] = cc * (b2 * zz); bp[mu] = real(0); bp[mv] = cc * b2;
+    }
 };
 
 // ------------------------------------------------------------------------
@@ -438,8 +449,8 @@ struct VCAcoustics1D {
         const real zl = auxL[0], cl = auxL[1], zr = auxR[0], cr = auxR[1];
         const real dp = qR[0] - qL[0];
         const real du = qR[1] - qL[1];
-        const real a1 = (zr * du - dp) / (zl + zr);
-        const real a2 = (zl * du + dp) / (zl + zr);
+        const real a1 = div_ieee(zr * du - dp, zl + zr);
+        const real a2 = div_ieee(zl * du + dp, zl + zr);
         wave[0][0] = -(a1 * zl); wave[0][1] = a1;
         wave[1][0] = a2 * zr;    wave[1][1] = a2;
         s[0] = -cl;

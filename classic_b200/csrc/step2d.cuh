@@ -162,6 +162,18 @@ struct solver_ctx<S, std::void_t<typename S::Ctx>> {
     static constexpr bool value = true;
 };
 
+// Optional solver trait: S::trans_mirror with S::up, a transverse split whose
+// lower half is its upper half with the pressure's sign changed; the kernel
+// then forms, sends and keeps the upper half alone: four multiplications and
+// two shuffles a split where both halves took twelve operations and four.
+// With q(c-1) read from the ring when its row is due (not carried, 12
+// registers) the acoustics kernel no longer spills: radial 1024^2 FP64 57 ->
+// 52 us a step.
+template <class S, class = void>
+struct solver_mirror { static constexpr bool value = false; };
+template <class S>
+struct solver_mirror<S, std::void_t<decltype(S::trans_mirror)>> { static constexpr bool value = S::trans_mirror; };
+
 template <class S>
 __device__ __forceinline__ typename solver_ctx<S>::type iface_ctx(const S& s, int ixy,
                                                                   const typename S::real* qL,
@@ -206,6 +218,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     using real = typename S::real;
     constexpr int ME = S::meqn, MW = S::mwaves, MA = S::maux;
     constexpr int MAX = MA > 0 ? MA : 1;
+    constexpr bool MIRROR = solver_mirror<S>::value;
     using R = Ring2D<S>;
     constexpr int W = R::W;
     constexpr unsigned FULL = 0xffffffffu;
@@ -222,6 +235,13 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     const bool capa = M::capa >= 0 ? (M::capa != 0) : (A.capa > 0);
     const bool fwave = M::fwave >= 0 ? (M::fwave != 0) : (A.fwave != 0);
     const int ic = capa ? A.capa - 1 : 0;
+    // the capacity of a cell's aux vector (a run-time index would put it in local memory)
+    auto cap = [&](const real* a) -> real {
+        real v = a[0];
+#pragma unroll
+        for (int k = 1; k < MAX; ++k) v = ic == k ? a[k] : v;
+        return v;
+    };
     bool limit = M::lim > 0;
     if (M::lim < 0)
         limit = (A.mthlim[0] | A.mthlim[1] | A.mthlim[2] | A.mthlim[3] | A.mthlim[4] |
@@ -236,6 +256,12 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     auto phi = [](int ml, real r) -> real {
         if constexpr (M::fast) return phi_limiter_fast<real>(ml, r);
         else return phi_limiter<real>(ml, r);
+    };
+    // limiter ratio; a zero wave's is not used, and dividing by 1 keeps it off
+    // the division's general path
+    auto ratio = [](real n, real nn) -> real {
+        if constexpr (M::fast) return AR::div(n, nn);
+        else return AR::div(n, nn != real(0) ? nn : real(1));
     };
     const int lane = threadIdx.x & 31;
     const int mx = A.mx, my = A.my;
@@ -257,7 +283,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     // x-interface c counts toward the CFL for columns 0..mx, y-interface
     // of column c for columns -1..mx (src/2d/flux2.f90:124-132 over the
     // slices of src/2d/step2.f90:92,173)
-    const bool cx_ok = c >= 0 && c <= mx;
+    const bool cx_ok = c >= 0 && c <= mx && (lane > 0 || !capa);
     const bool cy_ok = c >= -1 && c <= mx;
 
     // wait limit; test hook: strip 0 skips the copy of one row (its wait then
@@ -289,29 +315,27 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     auto slot_ptr = [&](int r) -> const unsigned char* {
         return ring + (int)(seq_of(r) & (RING - 1)) * R::SLOT;
     };
-    // q(c-1, r), q(c, r) with the x and y boundary conditions applied.
-    auto load_q = [&](int r, real* qm, real* qc) {
+    // q of this lane's column (left = false) or the column left of it at row r,
+    // with the x and y boundary conditions applied.
+    auto load_q = [&](int r, bool left, real* q) {
         const real* sq = reinterpret_cast<const real*>(slot_ptr(r));
         bool nyneg;
         const int sr = bc_map(r, my, A.bc[2], A.bc[3], nyneg);
+        const int at = left ? im : icc, src = left ? sm : sc;
+        const bool glob = left ? gm : gc, neg = left ? negm : negc;
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
-            real vm = sq[m * W + im];
-            real vc = sq[m * W + icc];
+            real v = sq[m * W + at];
             if (any_global) {
-                if (gm) vm = qold[m * A.fstride + (long long)sr * A.ld + sm];
-                if (gc) vc = qold[m * A.fstride + (long long)sr * A.ld + sc];
+                if (glob) v = qold[m * A.fstride + (long long)sr * A.ld + src];
             }
-            if (m == 1) { vm = negm ? -vm : vm; vc = negc ? -vc : vc; }
-            if (m == 2 && nyneg) { vm = -vm; vc = -vc; }
-            qm[m] = vm;
-            qc[m] = vc;
+            if (m == 1) v = neg ? -v : v;
+            if (m == 2 && nyneg) v = -v;
+            q[m] = v;
         }
         if constexpr (SRC) {
-            if (K.src == 2) {  // Strang: dt/2 of source on the data the step reads
-                src_radial_cell(A, qm, c - 1, K.src_pre);
-                src_radial_cell(A, qc, c, K.src_pre);
-            }
+            // Strang: dt/2 of source on the data the step reads
+            if (K.src == 2) src_radial_cell(A, q, left ? c - 1 : c, K.src_pre);
         }
     };
     // aux of column (c + dc) at row r (ring already resident).
@@ -323,9 +347,34 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         }
     };
 
+    // dt/dx and dt/dy over the capacity of a cell, in the update's arithmetic
+    // and (FP32 and contracted builds) as the Courant number takes them.  One
+    // division a row and axis: the cell to the left is the lane to the left
+    // (lane 0's interface counts towards no output, and towards the Courant
+    // number in the strip to the left), the rows roll with the march.  Two
+    // divisions a row for twelve: annulus 40 x 120, 25 -> 21 us a step.
+    constexpr bool SAME = sizeof(real) == 8 && !M::fast;
+    struct Scale { real v; double d; };
+    auto scale = [&](real dtd, double dtd_d, const real* a) -> Scale {
+        Scale k{dtd, dtd_d};
+        if (capa) {
+            k.v = AR::div(dtd, cap(a));
+            k.d = SAME ? (double)k.v : dtd_d / (double)cap(a);
+        }
+        return k;
+    };
+    auto scale_left = [&](const Scale& k) -> Scale {
+        Scale l = k;
+        if (capa) {
+            l.v = __shfl_up_sync(FULL, k.v, 1);
+            l.d = SAME ? (double)l.v : __shfl_up_sync(FULL, k.d, 1);
+        }
+        return l;
+    };
+    Scale ky_p{dtdy, dtdy_d}, ky_t{dtdy, dtdy_d};  // rows t-1, t
+
     // ---- march state ----
-    real qm_t[ME], qc_t[ME];        // row t
-    real qm_n[ME], qc_n[ME];        // row t+1
+    real qc_t[ME], qc_n[ME];        // rows t, t+1
     real qc_p[ME];                  // q(c, t-1)
     real Ax_prev[ME], q2_prev[ME];  // x-slice increments carried to row t
     // y-interface t (between rows t-1 and t): raw waves and fluctuations
@@ -348,17 +397,18 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     if (!wait_row(rfirst)) { failed = true; fail_row = rfirst; }
     if (!failed && !wait_row(rfirst + 1)) { failed = true; fail_row = rfirst + 1; }
     if (!failed) {
-        load_q(rfirst, qm_t, qc_t);
-        load_q(rfirst + 1, qm_n, qc_n);
+        load_q(rfirst, false, qc_t);
+        load_q(rfirst + 1, false, qc_n);
         real a_c[MAX], a_cn[MAX];
         aux_at(rfirst, 0, a_c);
         aux_at(rfirst + 1, 0, a_cn);
         cy = iface_ctx(A.solver, 2, qc_t, qc_n);
         if constexpr (solver_ctx<S>::value) A.solver.rpn_ctx(2, cy, qc_t, qc_n, wy, sy, amy, apy);
         else A.solver.rpn(2, qc_t, qc_n, a_c, a_cn, wy, sy, amy, apy);
+        ky_p = scale(dtdy, dtdy_d, a_c);
+        ky_t = scale(dtdy, dtdy_d, a_cn);
         if (cy_ok && rfirst + 1 >= 0) {
-            const double dt0 = capa ? dtdy_d / (double)a_c[ic] : dtdy_d;
-            const double dt1 = capa ? dtdy_d / (double)a_cn[ic] : dtdy_d;
+            const double dt0 = ky_p.d, dt1 = ky_t.d;
             double em = 0.0;
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw)
@@ -368,7 +418,6 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
             qc_p[m] = qc_t[m];
-            qm_t[m] = qm_n[m];
             qc_t[m] = qc_n[m];
         }
     }
@@ -376,7 +425,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
     for (int t = r0 - 1; t <= r0 + nr && !failed; ++t) {
         // ---------------- read row t+1 ----------------
         if (!wait_row(t + 1)) { failed = true; fail_row = t + 1; break; }
-        load_q(t + 1, qm_n, qc_n);
+        load_q(t + 1, false, qc_n);
         real a_m[MAX], a_c[MAX], a_cn[MAX], a_p[MAX], a_cp[MAX], a_mp[MAX], a_pp[MAX], a_mn[MAX];
         aux_at(t, -1, a_m);       // (c-1, t)
         aux_at(t, 0, a_c);        // (c,   t)
@@ -390,15 +439,15 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         // ======== x-slice t: interface c (between columns c-1, c) ========
         real q3[ME];
         {
-            real w[MW][ME], s[MW], amdq[ME], apdq[ME];
+            real w[MW][ME], s[MW], amdq[ME], apdq[ME], qm_t[ME];
+            load_q(t, true, qm_t);  // (row t stays in the ring until the next iteration)
             const auto cx = iface_ctx(A.solver, 1, qm_t, qc_t);
             if constexpr (solver_ctx<S>::value) A.solver.rpn_ctx(1, cx, qm_t, qc_t, w, s, amdq, apdq);
             else A.solver.rpn(1, qm_t, qc_t, a_m, a_c, w, s, amdq, apdq);
-            const real dtm = capa ? AR::div(dtdx, a_m[ic]) : dtdx;  // dtdx1d(i-1)
-            const real dtc = capa ? AR::div(dtdx, a_c[ic]) : dtdx;  // dtdx1d(i)
+            const Scale kc = scale(dtdx, dtdx_d, a_c), km = scale_left(kc);
+            const real dtm = km.v, dtc = kc.v;  // dtdx1d(i-1), dtdx1d(i)
             {
-                const double dm = capa ? dtdx_d / (double)a_m[ic] : dtdx_d;
-                const double dc = capa ? dtdx_d / (double)a_c[ic] : dtdx_d;
+                const double dm = km.d, dc = kc.d;
                 double em = 0.0;
 #pragma unroll
                 for (int mw = 0; mw < MW; ++mw)
@@ -442,7 +491,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                         const int ml = lim_of(mw);
                         if (ml == 0) continue;
                         const real dl = __shfl_up_sync(FULL, dotr[mw], 1);
-                        const real r = AR::div(s[mw] > real(0) ? dl : dotr[mw], wn2[mw]);
+                        const real r = ratio(s[mw] > real(0) ? dl : dotr[mw], wn2[mw]);
                         const real ph = wn2[mw] != real(0) ? phi(ml, r) : real(1);
 #pragma unroll
                         for (int m = 0; m < ME; ++m)
@@ -477,21 +526,23 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                     }
                 }
                 real bm[ME], bp[ME];
-                if constexpr (solver_ctx<S>::value) A.solver.rpt_ctx(1, 1, cx, amdq, bm, bp);
+                if constexpr (MIRROR) A.solver.up(1, amdq, bp);
+                else if constexpr (solver_ctx<S>::value) A.solver.rpt_ctx(1, 1, cx, amdq, bm, bp);
                 else A.solver.rpt(1, 1, qm_t, qc_t, a_mp, a_m, a_mn, amdq, bm, bp);
                 const real hm = real(0.5) * dtm, hc = real(0.5) * dtc;
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
                     if (S::trans_zero(1, m)) continue;
-                    s3[m] = -(hm * bm[m]);  // gadd(:,1,i-1) from this interface
+                    if constexpr (!MIRROR) s3[m] = -(hm * bm[m]);  // gadd(:,1,i-1) from this interface
                     s4[m] = -(hm * bp[m]);  // gadd(:,2,i-1)
                 }
-                if constexpr (solver_ctx<S>::value) A.solver.rpt_ctx(1, 2, cx, apdq, bm, bp);
+                if constexpr (MIRROR) A.solver.up(1, apdq, bp);
+                else if constexpr (solver_ctx<S>::value) A.solver.rpt_ctx(1, 2, cx, apdq, bm, bp);
                 else A.solver.rpt(1, 2, qm_t, qc_t, a_cp, a_c, a_cn, apdq, bm, bp);
 #pragma unroll
                 for (int m = 0; m < ME; ++m) {
                     if (S::trans_zero(1, m)) continue;
-                    g1b[m] = hc * bm[m];
+                    if constexpr (!MIRROR) g1b[m] = hc * bm[m];
                     g2b[m] = hc * bp[m];
                 }
             }
@@ -507,10 +558,10 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                     dF = r2 - F[m];
                 }
                 if (!tz) {
-                    const real r3 = __shfl_down_sync(FULL, s3[m], 1);
                     const real r4 = __shfl_down_sync(FULL, s4[m], 1);
-                    G1 = r3 - g1b[m];
                     G2 = r4 - g2b[m];
+                    if constexpr (MIRROR) G1 = m == 0 ? -G2 : G2;
+                    else G1 = __shfl_down_sync(FULL, s3[m], 1) - g1b[m];
                 }
                 real q2, Ax = real(0), Bx = real(0);
                 if (!capa) {
@@ -523,9 +574,9 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                         Bx = dtdy * G1;
                     }
                 } else {
-                    q2 = ((qc_t[m] + Ax_prev[m]) + qa) - AR::div(dtdx * dF + dtdy * (G2 - G1), a_c[ic]);
-                    Ax = AR::div(dtdy * G2, a_cn[ic]);
-                    Bx = AR::div(dtdy * G1, a_cp[ic]);
+                    q2 = ((qc_t[m] + Ax_prev[m]) + qa) - AR::div(dtdx * dF + dtdy * (G2 - G1), cap(a_c));
+                    Ax = AR::div(dtdy * G2, cap(a_cn));
+                    Bx = AR::div(dtdy * G1, cap(a_cp));
                 }
                 q3[m] = (!tz || capa) ? q2_prev[m] - Bx : q2_prev[m];  // x-part of (c, t-1)
                 q2_prev[m] = q2;
@@ -538,17 +589,16 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         const auto cyn = iface_ctx(A.solver, 2, qc_t, qc_n);
         if constexpr (solver_ctx<S>::value) A.solver.rpn_ctx(2, cyn, qc_t, qc_n, wn, sn, amn, apn);
         else A.solver.rpn(2, qc_t, qc_n, a_c, a_cn, wn, sn, amn, apn);
+        const Scale ky_n = scale(dtdy, dtdy_d, a_cn);
         {
-            const double dt0 = capa ? dtdy_d / (double)a_c[ic] : dtdy_d;
-            const double dt1 = capa ? dtdy_d / (double)a_cn[ic] : dtdy_d;
+            const double dt0 = ky_t.d, dt1 = ky_n.d;
             double em = 0.0;
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw)
                 em = dmax(em, dmax(dt1 * (double)sn[mw], -dt0 * (double)sn[mw]));
             cfl = (cy_ok && t + 1 <= my) ? dmax(cfl, em) : cfl;
         }
-        const real dty_p = capa ? AR::div(dtdy, a_cp[ic]) : dtdy;  // dtdy1d(t-1)
-        const real dty_t = capa ? AR::div(dtdy, a_c[ic]) : dtdy;   // dtdy1d(t)
+        const real dty_p = ky_p.v, dty_t = ky_t.v;  // dtdy1d(t-1), dtdy1d(t)
         real cqy[ME], Fy[ME], dotr_y[MW];
 #pragma unroll
         for (int m = 0; m < ME; ++m) { cqy[m] = real(0); Fy[m] = real(0); }
@@ -578,7 +628,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                         nn = first ? wy[mw][m] * wy[mw][m] : nn + wy[mw][m] * wy[mw][m];
                         first = false;
                     }
-                    const real r = AR::div(sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw], nn);
+                    const real r = ratio(sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw], nn);
                     const real ph = nn != real(0) ? phi(ml, r) : real(1);
 #pragma unroll
                     for (int m = 0; m < ME; ++m)
@@ -615,7 +665,10 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                     apy[m] = apy[m] - cqy[m];
                 }
             }
-            if constexpr (solver_ctx<S>::value) {
+            if constexpr (MIRROR) {
+                A.solver.up(2, amy, bpa);
+                A.solver.up(2, apy, bpb);
+            } else if constexpr (solver_ctx<S>::value) {
                 A.solver.rpt_ctx(2, 1, cy, amy, bma, bpa);
                 A.solver.rpt_ctx(2, 2, cy, apy, bmb, bpb);
             } else {
@@ -632,8 +685,8 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
             const bool wz = S::wave_zero(2, m), tz = S::trans_zero(2, m) || trans <= 0;
             const real qa = wz ? real(0) : P1[m] - dty_p * amo[m];
             const real dF = wz ? real(0) : Fy[m] - Fy_prev[m];
-            const real G1 = tz ? real(0) : -(hp * bma[m]) - P3[m];
             const real G2 = tz ? real(0) : -(hp * bpa[m]) - P4[m];
+            const real G1 = tz ? real(0) : MIRROR ? (m == 0 ? -G2 : G2) : -(hp * bma[m]) - P3[m];
             real q6;
             if (!capa) {
                 real q5 = q3[m];
@@ -643,10 +696,10 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                 else if (!tz) q5 = q5 + (-(dtdx * (G2 - G1)));
                 q6 = tz ? q5 : q5 - __shfl_down_sync(FULL, dtdx * G1, 1);  // from column c+1
             } else {
-                const real Al = __shfl_up_sync(FULL, AR::div(dtdx * G2, a_pp[ic]), 1);
-                const real Br = __shfl_down_sync(FULL, AR::div(dtdx * G1, a_mp[ic]), 1);
+                const real Al = __shfl_up_sync(FULL, AR::div(dtdx * G2, cap(a_pp)), 1);
+                const real Br = __shfl_down_sync(FULL, AR::div(dtdx * G1, cap(a_mp)), 1);
                 const real q4 = q3[m] + Al;
-                const real q5 = (q4 + qa) - AR::div(dtdy * dF + dtdx * (G2 - G1), a_cp[ic]);
+                const real q5 = (q4 + qa) - AR::div(dtdy * dF + dtdx * (G2 - G1), cap(a_cp));
                 q6 = q5 - Br;
             }
             qo[m] = q6;
@@ -662,16 +715,17 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
             P1[m] = S::wave_zero(2, m) ? real(0) : -(dty_t * apo[m]);
-            P3[m] = S::trans_zero(2, m) ? real(0) : ht * bmb[m];
+            P3[m] = S::trans_zero(2, m) || MIRROR ? real(0) : ht * bmb[m];
             P4[m] = S::trans_zero(2, m) ? real(0) : ht * bpb[m];
             Fy_prev[m] = Fy[m];
             amy[m] = amn[m];
             apy[m] = apn[m];
             qc_p[m] = qc_t[m];
-            qm_t[m] = qm_n[m];
             qc_t[m] = qc_n[m];
         }
         cy = cyn;
+        ky_p = ky_t;
+        ky_t = ky_n;
 #pragma unroll
         for (int mw = 0; mw < MW; ++mw) {
             dotl_y[mw] = dotr_y[mw];

@@ -146,7 +146,7 @@ __device__ __forceinline__ void split_xslice(const Step2Args<S>& A, const typena
                 const int ml = M::lim >= 0 ? M::lim : A.mthlim[mw];
                 const real dl = __shfl_up_sync(FULL, dotr[mw], 1);
                 if (ml == 0) continue;
-                const real r = (s[mw] > real(0) ? dl : dotr[mw]) / wn2[mw];
+                const real r = div_ieee(s[mw] > real(0) ? dl : dotr[mw], wn2[mw] != real(0) ? wn2[mw] : real(1));
                 const real ph = wn2[mw] != real(0) ? phi_limiter<real>(ml, r) : real(1);
 #pragma unroll
                 for (int m = 0; m < ME; ++m)
@@ -179,7 +179,7 @@ __device__ __forceinline__ void split_xslice(const Step2Args<S>& A, const typena
         if (update && !S::wave_zero(1, m)) {
             const real qa = qadd[m] - r1;
             const real dF = r2 - F[m];
-            v = capa ? (v + qa) - dtdx * dF / ac[ic] : (v + qa) - dtdx * dF;
+            v = capa ? (v + qa) - div_ieee(dtdx * dF, ac[ic]) : (v + qa) - dtdx * dF;
         }
         xq[m] = v;
     }
@@ -389,7 +389,7 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
                         nn = first ? wy[mw][m] * wy[mw][m] : nn + wy[mw][m] * wy[mw][m];
                         first = false;
                     }
-                    const real r = (sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw]) / nn;
+                    const real r = div_ieee(sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw], nn != real(0) ? nn : real(1));
                     const real ph = nn != real(0) ? phi_limiter<real>(ml, r) : real(1);
 #pragma unroll
                     for (int m = 0; m < ME; ++m)
@@ -424,7 +424,7 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
             if (ro >= 0 && ro < my && !S::wave_zero(2, m)) {
                 const real qa = P1[m] - dty_p * amy[m];
                 const real dF = Fy[m] - Fy_prev[m];
-                v = capa ? (v + qa) - K.dtdy * dF / aux_p[ic] : (v + qa) - K.dtdy * dF;
+                v = capa ? (v + qa) - div_ieee(K.dtdy * dF, aux_p[ic]) : (v + qa) - K.dtdy * dF;
             }
             yb[m] = v;
         }
