@@ -78,13 +78,10 @@ long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 template <class S>
 struct Runner1D : Runner {
     Step1Args<S> args;
-    int smem = 0;
-    typename S::real* iface = nullptr;
+    int smem = 0, threads = 64;
+    void (*kernel)(const Step1Args<S>) = nullptr;
 
     explicit Runner1D(const S& s) { std::memset(&args, 0, sizeof(args)); args.solver = s; }
-    ~Runner1D() override {
-        if (iface) cudaFree(iface);
-    }
 
     int prepare(const claw_config& cfg, const Geometry& g) override {
         args.q[0] = static_cast<typename S::real*>(g.q[0]);
@@ -108,23 +105,23 @@ struct Runner1D : Runner {
         int dev = 0, optin = 0;
         CUDA_TRY(cudaGetDevice(&dev));
         CUDA_TRY(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        long long bytes = step1_smem_bytes<S>(g.mx, true);
-        if (bytes + 1024 > optin) {
-            // the interface arrays move to an L2-resident global buffer
-            bytes = step1_smem_bytes<S>(g.mx, false);
-            if (bytes + 1024 > optin)
-                return fail(CLAW_E_UNSUPPORTED, "1D grid of %d cells exceeds the single-CTA kernel", g.mx);
-            CUDA_TRY(cudaMalloc(&iface, (size_t)step1_iface_doubles<S>(g.mx) * sizeof(typename S::real)));
-        }
-        args.iface = iface;
-        smem = (int)bytes;
-        CUDA_TRY(cudaFuncSetAttribute(step1_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem));
+        // a warp per strip of cells while the CTA has room, and the controller's
+        constexpr int most = step1_threads<S>();
+        threads = std::min(most, 32 * ((g.mx + STRIP1 - 1) / STRIP1 + 1));
+        const long long bytes = step1_smem_bytes<S>(g.mx);
+        const bool smq = bytes + 1024 <= optin;
+        smem = smq ? (int)bytes : 0;
+        bool mc = cfg.order == 2 && cfg.capa_index == 0 && !cfg.use_fwaves && args.src_split == 0;
+        for (int k = 0; k < cfg.num_waves; ++k) mc = mc && cfg.limiter[k] == 4;
+        if (!smq) kernel = &step1_kernel<S, Method1Any, false, most>;
+        else if (threads > 512) kernel = mc ? &step1_kernel<S, Method1MC, true, most> : &step1_kernel<S, Method1Any, true, most>;
+        else kernel = mc ? &step1_kernel<S, Method1MC, true, 512> : &step1_kernel<S, Method1Any, true, 512>;
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         return 0;
     }
 
     cudaError_t launch(cudaStream_t s) override {
-        step1_kernel<S><<<1, STEP1_THREADS, smem, s>>>(args);
+        kernel<<<1, threads, smem, s>>>(args);
         return cudaGetLastError();
     }
 };

@@ -5,16 +5,32 @@
 // next dt is chosen before the Courant check, unlike claw2).
 //
 // 1D grids in this code family are small (hundreds to ~2000 cells), so the
-// B200 shape is one CTA holding the grid, its ghost cells, the saved copy for
-// rejected steps and all interface quantities in shared memory; each time
-// step is four barrier-separated phases and the dt controller runs in thread
-// 0.  One launch replaces ~10^3 step launches and host round trips.
+// B200 shape is one CTA that keeps q in shared memory (two copies: a step
+// reads one and writes the other, so a rejected step is one not switched to).
+// One launch replaces ~10^3 step launches and host round trips.
+//
+// What bounds a step is the latency of its dependent chain, so the chain is
+// kept short and split in two.  A warp holds 32 neighbouring cells, two of
+// them halo on each side, and writes 28: waves, limiter ratios, correction
+// fluxes and fluctuations stay in registers and cross lanes by shuffle.  Waves
+// and limited waves do not need dt, so while a warp of its own folds the last
+// step's Courant maxima and runs claw1's dt controller (two divisions), the
+// others solve the next step's Riemann problems on the new q; a rejected step
+// solves the old q's again.  Two barriers per step.
 #pragma once
 #include "common.cuh"
 
 namespace clawb200 {
 
-constexpr int STEP1_THREADS = 512;
+constexpr int STRIP1 = 28;  // cells a warp writes
+
+// Threads of the CTA at most: 512 leave a thread 128 registers; a two-wave
+// system fits the 64 that 1024 threads leave, which grids of more than 16
+// strips take.
+template <class S>
+__host__ __device__ constexpr int step1_threads() {
+    return S::mwaves >= 3 ? 512 : 1024;
+}
 
 template <class S>
 struct Step1Args {
@@ -30,263 +46,288 @@ struct Step1Args {
     // Strang; the radial term of examples/acoustics_2d_radial/1drad/src1.f
     int src_split;
     double src_nd1, src_bulk, xlower;  // ndim - 1, bulk, xlower
-    // per-interface waves, speeds and fluctuations: in shared memory when
-    // null, else this global buffer of step1_iface_doubles(mx) reals (grids
-    // whose interface arrays do not fit the CTA's shared memory; the buffer
-    // stays in L2, and __syncthreads orders the CTA's global accesses too)
-    typename S::real* iface;
     ClawCtl* ctl;
     S solver;
 };
 
-// src1.f:18-23 on cells 0..mx+1 (i = 1..mx+2): p -= dt (ndim-1) bulk / x_i u.
-// Thread tid owns the cells k = tid mod blockDim, as the update phases do.
+// q's two copies and aux in shared memory
 template <class S>
-__device__ __forceinline__ void step1_source(const Step1Args<S>& A, typename S::real* qs, int n,
-                                             double dts) {
-    using real = typename S::real;
-    for (int k = threadIdx.x; k < A.mx + 2; k += blockDim.x) {
-        const double xcell = A.xlower + ((double)(k + 1) - 0.5) * A.dx;
-        const double coef = dts * A.src_nd1 * A.src_bulk / xcell;
-        qs[k + 2] = qs[k + 2] - (real)(coef * (double)qs[n + k + 2]);
-    }
+long long step1_smem_bytes(int mx) {
+    return ((long long)2 * S::meqn * mx + (long long)S::maux * (mx + 4)) * (long long)sizeof(typename S::real);
 }
 
-// per-interface wave/s/amdq/apdq (f reuses amdq)
-template <class S>
-__host__ __device__ constexpr long long step1_iface_doubles(int mx) {
-    return (long long)(S::mwaves * S::meqn + S::mwaves + 2 * S::meqn) * (mx + 4);
+// Largest of the warp's values, each >= 0: their bit patterns order as they do.
+__device__ __forceinline__ double warp_max_nonneg(double c) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(c);
+    const unsigned hi = (unsigned)(b >> 32);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+    return __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
 }
 
-template <class S>
-__host__ __device__ constexpr long long step1_smem_doubles(int mx, bool iface_in_smem) {
-    // q, aux, dtdx (+ the interface arrays), reduction; the copy kept for a
-    // rejected step lives in the output buffer
-    return (long long)(S::meqn + S::maux + 1) * (mx + 4) + (iface_in_smem ? step1_iface_doubles<S>(mx) : 0) +
-           32;
-}
+// Methods compiled in: MC on every wave at order 2 without capacity, f-waves
+// or source (taken branches cost a lone warp 30-100 cycles each), and one that
+// reads everything at run time.
+struct Method1MC {
+    static constexpr int lim = 4;
+};
+struct Method1Any {
+    static constexpr int lim = -1;
+};
 
-template <class S>
-long long step1_smem_bytes(int mx, bool iface_in_smem) {
-    return step1_smem_doubles<S>(mx, iface_in_smem) * (long long)sizeof(typename S::real) + 64 * 8;
-}
-
-template <class S>
-__global__ void __launch_bounds__(STEP1_THREADS, 1) step1_kernel(const __grid_constant__ Step1Args<S> A) {
+// SMQ: q and aux in shared memory; else (grids too large for it) the two
+// copies are the handle's own buffers in global memory, L2-resident, whose
+// accesses __syncthreads orders within the CTA just the same.  The last warp
+// is the controller's.
+template <class S, class M, bool SMQ, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) step1_kernel(const __grid_constant__ Step1Args<S> A) {
     using real = typename S::real;
     constexpr int ME = S::meqn, MW = S::mwaves, MA = S::maux;
     constexpr int MAX = MA > 0 ? MA : 1;
+    constexpr bool ANY = M::lim < 0;
+    constexpr unsigned FULL = 0xffffffffu;
     ClawCtl* ctl = A.ctl;
-    const int mx = A.mx, n = mx + 4;  // cell k (0-based) lives at k+2
-    const int ne = mx + 4;            // interface e in [-1, mx+1] lives at e+1
+    const int mx = A.mx, n = mx + 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    real* qs = reinterpret_cast<real*>(smem_raw);
-    real* as = qs + ME * n;
-    real* dtdx = as + MA * n;
-    real* wv = A.iface ? A.iface : dtdx + n;  // [MW][ME][ne]
-    real* sv = wv + MW * ME * ne;   // [MW][ne]
-    real* amd = sv + MW * ne;       // [ME][ne]
-    real* apd = amd + ME * ne;
-    real* fl = amd;                 // [ME][ne], once the Godunov update has used amdq
-    __shared__ double red[STEP1_THREADS / 32];
-    __shared__ double sh_dt, sh_cfl;
-    __shared__ int sh_state;  // 0 continue, 1 retry, 2 stop
-
-    const int tid = threadIdx.x;
+    __shared__ double red[32];
+    __shared__ double sh_dt, sh_dtdx;
+    __shared__ int sh_act;
+    enum { STEP = 0, RETRY = 1, STOP_NEW = 2, STOP_OLD = 3 };
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = (blockDim.x >> 5) - 1;
+    const int nstrips = (mx + STRIP1 - 1) / STRIP1;
     const int cur = ctl->cur;
-    real* __restrict__ qsave = A.q[cur ^ 1];  // interior copy for a rejected step
+    real* sq = reinterpret_cast<real*>(smem_raw);  // [2][ME][mx]
+    real* sa = sq + 2 * ME * mx;                   // [MA][n]
+    const long long fs = SMQ ? mx : A.fstride, afs = SMQ ? n : A.afstride;
+    if constexpr (SMQ) {
+        const real* qin = A.q[cur];
+        for (int i = tid; i < ME * mx; i += blockDim.x) sq[i] = qin[(i / mx) * A.fstride + i % mx];
+        for (int i = tid; i < MA * n; i += blockDim.x) sa[i] = A.aux[(i / n) * A.afstride + i % n];
+    }
     // a single step (claw_step) is step1 alone: accepted whatever its Courant
     // number, without the source steps that claw1 wraps around it
     const bool single = ctl->mode == CTL_SINGLE;
-    const int src_split = single ? 0 : A.src_split;
-    const real* qin = A.q[cur];
-    for (int i = tid; i < ME * mx; i += blockDim.x) {
-        const int m = i / mx, k = i % mx;
-        qs[m * n + k + 2] = qin[m * A.fstride + k];
-    }
-    for (int i = tid; i < MA * n; i += blockDim.x) as[i] = A.aux[(i / n) * A.afstride + (i % n)];
-    double t = ctl->t, dt = ctl->dt;
-    const double tstart = ctl->tstart, tend = ctl->tend;
+    const int src_split = ANY && !single ? A.src_split : 0;
     const double dxd = A.dx;
-    bool limit = false;
-    for (int k = 0; k < MW; ++k) limit |= A.mthlim[k] != 0;
+    int buf = SMQ ? 0 : cur;  // q's copy the step reads
     __syncthreads();
 
-    double cflmax = 0.0, dtmin = ctl->dtmin, dtmaxs = ctl->dtmax, cfl = 0.0;
-    int nacc = 0, nrej = 0;
-    bool stop = false;
-    const int maxn = ctl->maxn;
-    for (int step = 0; step < maxn && !stop; ++step) {
-        const double told = t;
-        if (told + dt > tend && tstart < tend) dt = tend - told;
-        for (int i = tid; i < ME * mx; i += blockDim.x)
-            qsave[(i / mx) * A.fstride + i % mx] = qs[(i / mx) * n + i % mx + 2];
-        __syncthreads();
+    if (warp == nwarps) {  // ------------------------------- controller
+        const bool dt_variable = ctl->dt_variable != 0;
+        const double tstart = ctl->tstart, tend = ctl->tend, dt_max = ctl->dt_max, cfl_max = ctl->cfl_max,
+                     cfl_desired = ctl->cfl_desired;
+        const int maxn = ctl->maxn;
+        double t = ctl->t, dt = ctl->dt, dtmin = ctl->dtmin, dtmaxs = ctl->dtmax, cfl = 0.0, cflmax = 0.0;
+        double told = t;
+        int nacc = 0, nrej = 0, act = STEP;
+        bool fresh = true;  // a new step, not a retry
         for (;;) {
-            t = told + dt;
-            // ---- bc1 (src/1d/bc1.f): ghosts -1,-2 and mx,mx+1; wall negates q(2)
-            if (tid < 4 * ME) {
-                const int side = tid / (2 * ME), r = tid % (2 * ME), ibc = 1 + r / ME, m = r % ME;
-                const int bcode = A.bc[side];
-                int dst, src;
-                if (side == 0) {
-                    dst = -ibc;
-                    src = bcode == BC_PERIODIC ? mx - ibc : (bcode == BC_WALL ? ibc - 1 : 0);
+            if (act < STOP_NEW) {
+                if (fresh) {
+                    told = t;
+                    if (told + dt > tend && tstart < tend) dt = tend - told;
+                }
+                t = told + dt;
+                if (lane == 0) {
+                    sh_dt = dt;
+                    sh_dtdx = dt / dxd;
+                }
+            }
+            if (lane == 0) sh_act = act;
+            __syncthreads();
+            if (act >= STOP_NEW) break;
+            __syncthreads();
+            cfl = warp_max_nonneg(lane < nwarps ? red[lane] : 0.0);
+            // claw1: choose the next dt first (src/1d/claw1.f:520-529) ...
+            if (dt_variable) {
+                if (cfl > 0.0) {
+                    dt = fmin(dt_max, dt * cfl_desired / cfl);
+                    dtmin = fmin(dt, dtmin);
+                    dtmaxs = fmax(dt, dtmaxs);
                 } else {
-                    dst = mx - 1 + ibc;
-                    src = bcode == BC_PERIODIC ? ibc - 1 : (bcode == BC_WALL ? mx - ibc : mx - 1);
+                    dt = dt_max;
                 }
-                real v = qs[m * n + src + 2];
-                if (bcode == BC_WALL && m == 1) v = -v;
-                qs[m * n + dst + 2] = v;
             }
-            for (int k = tid; k < n; k += blockDim.x) {
-                if (A.capa > 0) dtdx[k] = (real)(dt / (dxd * (double)as[(A.capa - 1) * n + k]));
-                else dtdx[k] = (real)(dt / dxd);
+            // ... then check the Courant number (src/1d/claw1.f:533-554)
+            if (single || cfl <= cfl_max) {
+                cflmax = fmax(cfl, cflmax);
+                ++nacc;
+                fresh = true;
+                act = t >= tend || nacc >= maxn ? STOP_NEW : STEP;
+            } else {
+                t = told;
+                fresh = false;
+                if (dt_variable) {
+                    ++nrej;
+                    act = RETRY;
+                } else {
+                    cflmax = fmax(cfl, cflmax);
+                    act = STOP_OLD;
+                }
             }
-            __syncthreads();
-            if (src_split == 2) {  // Strang: dt/2 of source before the step
-                step1_source(A, qs, n, dt / 2.0);
-                __syncthreads();
+        }
+        if (lane == 0) {
+            ctl->t = t;
+            ctl->dt = dt;
+            ctl->cflmax_seen = cflmax;
+            ctl->cfl_last = cfl;
+            ctl->dtmin = dtmin;
+            ctl->dtmax = dtmaxs;
+            ctl->n = nacc;
+            ctl->nrej = nrej;
+            ctl->cur = SMQ ? cur ^ 1 : (cur ^ (nacc & 1));
+            ctl->done = 1;
+        }
+        buf = (SMQ ? 0 : cur) ^ (nacc & 1);
+    } else {  // ----------------------------------------------- cells
+        const bool order2 = ANY ? A.order != 1 : true;
+        const bool many = nstrips > nwarps;  // several strips per warp
+        // the source before a Strang step needs dt
+        const bool late = many || src_split == 2;
+        // this lane's cell of a strip, its source cell under bc1 (src/1d/bc1.f;
+        // a wall negates q(2)); once, unless warps take several strips
+        int x0 = 0, x = 0, sx = 0;
+        bool neg = false;
+        real a[MAX], aL[MAX];
+        auto cells = [&](int strip) {
+            x0 = strip * STRIP1 + lane - 2;
+            x = min(x0, mx + 1);
+            sx = x;
+            neg = false;
+            if (x < 0) {
+                neg = A.bc[0] == BC_WALL;
+                sx = A.bc[0] == BC_PERIODIC ? mx + x : (neg ? -1 - x : 0);
+            } else if (x >= mx) {
+                neg = A.bc[1] == BC_WALL;
+                sx = A.bc[1] == BC_PERIODIC ? x - mx : (neg ? 2 * mx - 1 - x : mx - 1);
             }
-            // ---- rp1 at interfaces e = -1 .. mx+1 (src/1d/step1.f90:82) + CFL
-            double c_loc = 0.0;
-            for (int e = tid - 1; e <= mx + 1; e += blockDim.x) {
-                real qL[ME], qR[ME], aL[MAX], aR[MAX];
-                for (int m = 0; m < ME; ++m) { qL[m] = qs[m * n + e + 1]; qR[m] = qs[m * n + e + 2]; }
-                for (int k = 0; k < MA; ++k) { aL[k] = as[k * n + e + 1]; aR[k] = as[k * n + e + 2]; }
-                real w[MW][ME], s[MW], am[ME], ap[ME];
-                A.solver.rp1(qL, qR, aL, aR, w, s, am, ap);
+#pragma unroll
+            for (int k = 0; k < MA; ++k) {
+                a[k] = SMQ ? sa[k * n + x + 2] : A.aux[k * afs + x + 2];
+                aL[k] = __shfl_up_sync(FULL, a[k], 1);
+            }
+        };
+        cells(warp);
+        // src1.f:18-23 at cell xc (0-based, right ghosts included): p -= dt (ndim-1) bulk / x_i u
+        auto source = [&](real* q, int xc, double dts) {
+            const double xcell = A.xlower + ((double)(xc + 1) - 0.5) * dxd;
+            const double coef = dts * A.src_nd1 * A.src_bulk / xcell;
+            q[0] = q[0] - (real)(coef * (double)q[ME > 1 ? 1 : 0]);
+        };
+        double dt = 0.0, dtdx_d = 0.0;
+        // q of this lane's cell, and the interface left of it: speeds,
+        // fluctuations, limited waves (src/1d/step1.f90:82, inlinelimiter)
+        real q[ME], w[MW][ME], s[MW], am[ME], ap[ME];
+        auto waves = [&](int b) {
+            const real* rd = SMQ ? sq + b * ME * mx : A.q[b];
+            real qL[ME];
+#pragma unroll
+            for (int m = 0; m < ME; ++m) q[m] = rd[m * fs + sx];
+            if (ME > 1) q[ME > 1 ? 1 : 0] = neg ? -q[ME > 1 ? 1 : 0] : q[ME > 1 ? 1 : 0];
+            if (ANY && src_split == 2 && x >= 0) source(q, x, dt / 2.0);  // Strang: dt/2 before the step
+#pragma unroll
+            for (int m = 0; m < ME; ++m) qL[m] = __shfl_up_sync(FULL, q[m], 1);
+            A.solver.rp1(qL, q, aL, a, w, s, am, ap);
+            if (order2) {
+                // the waves' ratios side by side: their divisions overlap
+                real nn[MW], r[MW];
+#pragma unroll
                 for (int mw = 0; mw < MW; ++mw) {
-                    for (int m = 0; m < ME; ++m) wv[(mw * ME + m) * ne + e + 1] = w[mw][m];
-                    sv[mw * ne + e + 1] = s[mw];
-                }
-                for (int m = 0; m < ME; ++m) { amd[m * ne + e + 1] = am[m]; apd[m * ne + e + 1] = ap[m]; }
-                if (e >= 0 && e <= mx) {
-                    const double dR = (double)dtdx[e + 2], dL = (double)dtdx[e + 1];
-                    for (int mw = 0; mw < MW; ++mw)
-                        c_loc = fmax(fmax(c_loc, dR * (double)s[mw]), -dL * (double)s[mw]);
-                }
-            }
-            __syncthreads();
-            // ---- Godunov update of cells 0..mx-1 (in place) and the limited
-            //      correction flux f at interfaces 0..mx
-            for (int k = tid; k < mx; k += blockDim.x) {
-                const real d = dtdx[k + 2];
-                for (int m = 0; m < ME; ++m)
-                    qs[m * n + k + 2] = (qs[m * n + k + 2] - d * apd[m * ne + k + 1]) - d * amd[m * ne + k + 2];
-            }
-            if (A.order != 1) {
-                __syncthreads();  // f overwrites amdq
-                for (int e = tid; e <= mx; e += blockDim.x) {
-                    real w[MW][ME];
-                    for (int mw = 0; mw < MW; ++mw)
-                        for (int m = 0; m < ME; ++m) w[mw][m] = wv[(mw * ME + m) * ne + e + 1];
-                    if (limit) {
-                        for (int mw = 0; mw < MW; ++mw) {
-                            const int ml = A.mthlim[mw];
-                            if (ml == 0) continue;
-                            real nn = real(0), dl = real(0), dr = real(0);
-                            for (int m = 0; m < ME; ++m) {
-                                const real wl = wv[(mw * ME + m) * ne + e];
-                                const real wr = wv[(mw * ME + m) * ne + e + 2];
-                                nn = nn + w[mw][m] * w[mw][m];
-                                dr = dr + w[mw][m] * wr;
-                                dl = dl + wl * w[mw][m];
-                            }
-                            if (nn == real(0)) continue;
-                            const real r = (sv[mw * ne + e + 1] > real(0) ? dl : dr) / nn;
-                            const real ph = phi_limiter<real>(ml, r);
-                            for (int m = 0; m < ME; ++m) w[mw][m] = ph * w[mw][m];
-                        }
+                    real dr = real(0);
+                    nn[mw] = real(0);
+#pragma unroll
+                    for (int m = 0; m < ME; ++m) {
+                        const real wn = __shfl_down_sync(FULL, w[mw][m], 1);
+                        nn[mw] = nn[mw] + w[mw][m] * w[mw][m];
+                        dr = dr + w[mw][m] * wn;
                     }
-                    const real ave = real(0.5) * (dtdx[e + 1] + dtdx[e + 2]);
-                    real f[ME];
+                    const real dl = __shfl_up_sync(FULL, dr, 1);
+                    // a zero wave is left as it is; its ratio is not used
+                    r[mw] = div_ieee(s[mw] > real(0) ? dl : dr, nn[mw] != real(0) ? nn[mw] : real(1));
+                }
+#pragma unroll
+                for (int mw = 0; mw < MW; ++mw) {
+                    const real p = phi_limiter<real>(ANY ? A.mthlim[mw] : M::lim, r[mw]);
+                    const real ph = nn[mw] != real(0) ? p : real(1);
+#pragma unroll
+                    for (int m = 0; m < ME; ++m) w[mw][m] = ph * w[mw][m];
+                }
+            }
+        };
+        for (;;) {
+            if (!late) waves(buf);
+            __syncthreads();
+            dt = sh_dt;
+            dtdx_d = sh_dtdx;
+            const int act = sh_act;
+            if (act >= STOP_NEW) break;
+            if (act == RETRY) {
+                buf ^= 1;
+                if (!late) waves(buf);
+            }
+            real* wr = SMQ ? sq + (buf ^ 1) * ME * mx : A.q[buf ^ 1];
+            double c_loc = 0.0;
+            for (int strip = warp; strip < nstrips; strip += nwarps) {
+                if (many) cells(strip);
+                if (late) waves(buf);
+                real d = (real)dtdx_d, dL = d;
+                if (ANY && MA > 0 && A.capa > 0) {
+                    const real cap = A.capa == 1 ? a[0] : a[MAX > 1 ? 1 : 0];
+                    d = (real)(dt / (dxd * (double)cap));
+                    dL = __shfl_up_sync(FULL, d, 1);
+                }
+                if (lane >= 2 && x0 <= mx) {  // interfaces 0 .. mx
+#pragma unroll
+                    for (int mw = 0; mw < MW; ++mw) {  // fmax by select: a NaN leaves c_loc
+                        const double cr = (double)d * (double)s[mw], cl = -(double)dL * (double)s[mw];
+                        c_loc = cr > c_loc ? cr : c_loc;
+                        c_loc = cl > c_loc ? cl : c_loc;
+                    }
+                }
+                // the correction flux f, then the Godunov update and the
+                // correction (src/1d/step1.f90:96-170)
+                real f[ME];
+                if (order2) {
+                    const real ave = real(0.5) * (dL + d);
+#pragma unroll
                     for (int m = 0; m < ME; ++m) f[m] = real(0);
+#pragma unroll
                     for (int mw = 0; mw < MW; ++mw) {
-                        const real sm = sv[mw * ne + e + 1], as_ = fabs(sm);
-                        const real coef = A.fwave ? real(0.5) * copysign(real(1), sm) * (real(1) - as_ * ave)
-                                                  : real(0.5) * as_ * (real(1) - as_ * ave);
+                        const real as_ = fabs(s[mw]);
+                        const real coef = ANY && A.fwave
+                                              ? real(0.5) * copysign(real(1), s[mw]) * (real(1) - as_ * ave)
+                                              : real(0.5) * as_ * (real(1) - as_ * ave);
+#pragma unroll
                         for (int m = 0; m < ME; ++m) f[m] = f[m] + coef * w[mw][m];
                     }
-                    for (int m = 0; m < ME; ++m) fl[m * ne + e + 1] = f[m];
                 }
-            }
-            // CFL reduction
-            for (int off = 16; off > 0; off >>= 1) c_loc = fmax(c_loc, __shfl_xor_sync(0xffffffffu, c_loc, off));
-            if ((tid & 31) == 0) red[tid >> 5] = c_loc;
-            __syncthreads();
-            if (A.order != 1) {
-                for (int k = tid; k < mx; k += blockDim.x) {
-                    const real d = dtdx[k + 2];
-                    for (int m = 0; m < ME; ++m)
-                        qs[m * n + k + 2] = qs[m * n + k + 2] - d * (fl[m * ne + k + 2] - fl[m * ne + k + 1]);
-                }
-            }
-            // source after the step, before the Courant check (claw1.f:499-509)
-            if (src_split == 2) step1_source(A, qs, n, dt / 2.0);
-            if (src_split == 1) step1_source(A, qs, n, dt);
-            if (tid == 0) {
-                double cm = 0.0;
-                for (int w = 0; w < STEP1_THREADS / 32; ++w) cm = fmax(cm, red[w]);
-                sh_cfl = cm;
-                // claw1: choose the next dt first (src/1d/claw1.f:520-529) ...
-                double dtn = dt;
-                if (ctl->dt_variable) {
-                    if (cm > 0.0) {
-                        dtn = fmin(ctl->dt_max, dt * ctl->cfl_desired / cm);
-                        dtmin = fmin(dtn, dtmin);
-                        dtmaxs = fmax(dtn, dtmaxs);
-                    } else {
-                        dtn = ctl->dt_max;
+#pragma unroll
+                for (int m = 0; m < ME; ++m) {
+                    const real amr = __shfl_down_sync(FULL, am[m], 1);
+                    q[m] = (q[m] - d * ap[m]) - d * amr;
+                    if (order2) {
+                        const real fr = __shfl_down_sync(FULL, f[m], 1);
+                        q[m] = q[m] - d * (fr - f[m]);
                     }
                 }
-                sh_dt = dtn;
-                // ... then check the Courant number (src/1d/claw1.f:533-554)
-                if (cm != cm) sh_state = single ? 0 : 3;
-                else if (single || cm <= ctl->cfl_max) sh_state = 0;
-                else sh_state = ctl->dt_variable ? 1 : 2;
+                // source after the step, before the Courant check (claw1.f:499-509)
+                if (ANY && src_split != 0 && x0 >= 0) source(q, x, src_split == 2 ? dt / 2.0 : dt);
+                if (lane >= 2 && lane < 2 + STRIP1 && x0 < mx) {
+#pragma unroll
+                    for (int m = 0; m < ME; ++m) wr[m * fs + x] = q[m];
+                }
             }
+            const double wm = warp_max_nonneg(c_loc > 0.0 ? c_loc : 0.0);
+            if (lane == 0) red[warp] = wm;
             __syncthreads();
-            cfl = sh_cfl;
-            dt = sh_dt;
-            const int st = sh_state;
-            if (st == 0) {
-                cflmax = fmax(cfl, cflmax);
-                break;
-            }
-            t = told;
-            for (int i = tid; i < ME * mx; i += blockDim.x)
-                qs[(i / mx) * n + i % mx + 2] = qsave[(i / mx) * A.fstride + i % mx];
-            __syncthreads();
-            if (st == 1) { ++nrej; continue; }
-            if (st == 3) { if (tid == 0) ctl->err |= CTL_ERR_NAN_CFL; stop = true; break; }
-            cflmax = fmax(cfl, cflmax);
-            stop = true;
-            break;
+            buf ^= 1;
         }
-        if (stop) break;
-        ++nacc;
-        if (t >= tend) break;
-        __syncthreads();
+        if (sh_act == STOP_OLD) buf ^= 1;
     }
-    __syncthreads();
-    real* qout = A.q[cur ^ 1];
-    for (int i = tid; i < ME * mx; i += blockDim.x) {
-        const int m = i / mx, k = i % mx;
-        qout[m * A.fstride + k] = qs[m * n + k + 2];
-    }
-    if (tid == 0) {
-        ctl->t = t;
-        ctl->dt = dt;
-        ctl->cflmax_seen = cflmax;
-        ctl->cfl_last = cfl;
-        ctl->dtmin = dtmin;
-        ctl->dtmax = dtmaxs;
-        ctl->n = nacc;
-        ctl->nrej = nrej;
-        ctl->cur = cur ^ 1;
-        ctl->done = 1;
+    if constexpr (SMQ) {
+        real* qout = A.q[cur ^ 1];
+        const real* qs = sq + buf * ME * mx;
+        for (int i = tid; i < ME * mx; i += blockDim.x) qout[(i / mx) * A.fstride + i % mx] = qs[i];
     }
 }
 
