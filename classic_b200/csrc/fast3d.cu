@@ -25,22 +25,11 @@ struct Step3fRunner : Runner {
         CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * Sh::rows, Sh::smem));
         if (per_sm < 1) return fail(CLAW_E_CUDA, "step3f kernel cannot be resident on an SM");
-        // Segments of planes: the count with the least work in the longest
-        // column of CTAs (waves of CTAs times planes each marches, with 4
-        // planes' worth of start-up: two halo planes and the first copies).
-        const long long tiles = (long long)args.tilesx * args.tilesy, slots = (long long)nsm * per_sm;
-        long long best = -1;
-        for (int n = 1; n <= g.mz; ++n) {
-            const int len = (g.mz + n - 1) / n;
-            const int segs = (g.mz + len - 1) / len;
-            const long long cost = (tiles * segs + slots - 1) / slots * (len + 4);
-            if (best < 0 || cost < best) {
-                best = cost;
-                args.seglen = len;
-                if (tiles * segs > 0x7fffffffLL) return fail(CLAW_E_UNSUPPORTED, "3D grid too large");
-                grid = (int)(tiles * segs);
-            }
-        }
+        const long long tiles = (long long)args.tilesx * args.tilesy;
+        args.seglen = segment_length(tiles, g.mz, (long long)nsm * per_sm);
+        const long long n = tiles * ((g.mz + args.seglen - 1) / args.seglen);
+        if (n > 0x7fffffffLL) return fail(CLAW_E_UNSUPPORTED, "3D grid too large");
+        grid = (int)n;
         return 0;
     }
     cudaError_t launch(cudaStream_t s) override {

@@ -479,8 +479,8 @@ struct VCAcoustics3D {
                                                real s[2], real am[2], real ap[2]) {
         const real dp = pR - pL;
         const real du = uR - uL;
-        const real a1 = (zr * du - dp) / (zl + zr);
-        const real a2 = (zl * du + dp) / (zl + zr);
+        const real a1 = div_ieee(zr * du - dp, zl + zr);
+        const real a2 = div_ieee(zl * du + dp, zl + zr);
         w[0][0] = -(a1 * zl); w[0][1] = a1;
         w[1][0] = a2 * zr;    w[1][1] = a2;
         s[0] = -cl;

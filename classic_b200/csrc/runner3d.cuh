@@ -53,6 +53,26 @@ void fill_sweep3(Sweep3Args<real>& b, const claw_config& cfg, const Geometry& g)
     b.ctl = g.ctl;
 }
 
+// Cells per segment of a 3D march of n cells over `tiles` tiles: the count with
+// the least work in the longest column of CTAs (waves of CTAs on `slots`
+// resident ones, times the cells each marches, with four cells' worth of
+// start-up: halo cells and the first copies).  In 64-cell segments a 64^3 grid
+// was 25 CTAs.
+inline int segment_length(long long tiles, int n, long long slots) {
+    long long best = -1;
+    int length = n;
+    for (int s = 1; s <= n; ++s) {
+        const int len = (n + s - 1) / s;
+        const long long ctas = tiles * ((n + len - 1) / len);
+        const long long cost = (ctas + slots - 1) / slots * (len + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            length = len;
+        }
+    }
+    return length;
+}
+
 // Reference order: one launch per sweep (sweep3p_kernel).
 template <class S, class M>
 struct Runner3D : Runner {
@@ -63,12 +83,17 @@ struct Runner3D : Runner {
 
     int prepare(const claw_config& cfg, const Geometry& g) override {
         const int m[3] = {g.mx, g.my, g.mz};
+        int dev = 0, nsm = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        const long long slots = (long long)nsm * CLAW_SWEEP3_MINB;
         for (int dir = 0; dir < 3; ++dir) {
             const int axa = dir == 0 ? 1 : 0, axb = dir == 2 ? 1 : 2;
             fill_sweep3(args[dir], cfg, g);
             args[dir].tilesA = (m[axa] + T3A - 3) / (T3A - 2);
             args[dir].tilesB = (m[axb] + T3B - 3) / (T3B - 2);
-            args[dir].nseg = (m[dir] + SEG3 - 1) / SEG3;
+            args[dir].seglen = segment_length((long long)args[dir].tilesA * args[dir].tilesB, m[dir], slots);
+            args[dir].nseg = (m[dir] + args[dir].seglen - 1) / args[dir].seglen;
             const long long n = (long long)args[dir].tilesA * args[dir].tilesB * args[dir].nseg;
             if (n > 0x7fffffffLL) return fail(CLAW_E_UNSUPPORTED, "3D grid too large");
             grid[dir] = (int)n;

@@ -3,10 +3,11 @@
 //
 // One kernel per sweep direction.  A CTA owns a T3A x T3B tile of slices of
 // that sweep (the outer ring of the tile is a one-slice halo) and marches the
-// tile along the slice direction, one cell position per iteration; each thread
-// carries one slice's Riemann state (normal solve at interface p+2, limiter
-// and second-order correction at p+1, the transverse and double-transverse
-// splits of p+1, and the gadd/hadd partial sums of cells p and p+1).
+// tile along the slice direction, one cell position per iteration; each slice's
+// Riemann state (normal solve at interface p+2, limiter and second-order
+// correction at p+1, the transverse and double-transverse splits of p+1, and
+// the gadd/hadd partial sums of cells p and p+1) is carried by a pair of
+// threads, the same lane of two neighbouring warps.
 //
 // A cell receives contributions from the nine slices around it.  step3 adds
 // them in the order of its 2x2-block colouring (colour of the slow slice
@@ -25,16 +26,16 @@
 namespace clawb200 {
 
 #ifndef CLAW_T3B
-#define CLAW_T3B 16
+#define CLAW_T3B 12
 #endif
 #ifndef CLAW_SWEEP3_MINB
 #define CLAW_SWEEP3_MINB 1  // resident CTAs per SM the sweep kernels are compiled for
 #endif
 constexpr int T3A = 16, T3B = CLAW_T3B, NT3 = T3A * T3B;   // thread tile, incl. the halo ring
 constexpr int S3A = T3A + 2, S3B = T3B + 2, NS3 = S3A * S3B;  // aux tile, one more ring
-constexpr int SEG3 = 64;                              // cell positions per CTA march
 constexpr int RING3 = 4;                              // aux positions held in shared memory
-constexpr int NTERM3 = 32;                            // published terms per slice and position
+constexpr int NPL3 = 4;                               // aux planes: Z, c, 1/(Z+Z_e1), 1/(Z+Z_e2)
+constexpr int NTERM3 = 39;                            // terms per slice and position: 8 neighbours x 4, centre
 constexpr int BC_PISTON = 10;                         // user BC of acoustics_3d_heterogeneous
 
 template <typename real>
@@ -51,17 +52,21 @@ struct Sweep3Args {
     int order, m3, m4;
     double d[3];         // dx, dy, dz
     double xlower, ylower;
-    int tilesA, tilesB, nseg;
+    int tilesA, tilesB, nseg, seglen;
     ClawCtl* ctl;
 };
 
 constexpr int QST3 = 4;  // staged q planes of NT3 values: [position & 1][p, normal velocity]
 
-// aux ring, two neighbour-term buffers, staged q: 160 KB in FP64, inside the
-// 164 KB shared-memory carveout (the rest of the SM's 256 KB is L1)
+constexpr int XCH3 = 8;   // exchange planes of NT3 values: L [h][2], R [h][2]
+constexpr int VST3 = 8;   // staged values of the cells each role updates: [position & 1][role][2]
+
+// Shared memory is sized to the carveout steps (100, 132, 164, 196, 228 KB);
+// what the carveout leaves is L1, which serves the x-sweep's strided loads and
+// the spills: 121 KB with one buffer of terms (a second CTA barrier a position).
 template <typename real>
 __host__ __device__ constexpr int sweep3_smem_bytes() {
-    return (RING3 * 2 * NS3 + 2 * NTERM3 * NT3 + QST3 * NT3) * (int)sizeof(real) +
+    return (RING3 * NPL3 * NS3 + (NTERM3 + XCH3 + QST3 + VST3) * NT3) * (int)sizeof(real) +
            16 * (int)sizeof(double);
 }
 
@@ -120,37 +125,83 @@ struct Method3D {
 using MethodGeneric3D = Method3D<-1, -1, -1>;
 using MethodMC3D = Method3D<2, 2, 4>;  // transverse_waves 22, MC on both waves
 
-// ------------------------------------------------------------ pair variant ---
-// Each slice's work is split over a thread pair: both
-// threads solve the normal problem, limit and form cqxx (a few dozen
-// operations, duplicated); thread h = 0 then owns flux3's y-like side (the
-// rpt3 splits in e1, the rptt3 splits of the z-like parts in e1, gadd) and
-// h = 1 the z-like side (splits in e2, hadd).  The four combinations each
-// side needs from the other's splits (flux3.f90:363-376 and :488-495) cross
-// by one shuffle, as do the two centre terms.  Half the registers per thread
-// give twice the resident warps of a thread per slice (which needs 255
-// registers).  Operation order per value is flux3's, so results are
-// bit-identical to the serial reference order in FP64 without contraction.
 constexpr int NT3P = 2 * NT3;
 
-template <class S, int DIR, class M, bool LAST>
-__global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const Sweep3Args<typename S::real> a) {
+// x / d, correctly rounded, from r = RN(1/d): q = x r, then q += r (x - d q)
+// twice.  The first correction leaves q within an ulp of x / d; then x - d q is
+// exact and the second rounds correctly (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990,
+// whose theorem asks for a correctly rounded reciprocal and no underflow).
+// Five operations where a division takes its whole latency of 148 cycles; the
+// sums d = Z + Z' repeat over the splits, so a ring element's two reciprocals
+// serve sixteen.  `in` says that x and d are far enough from the ends of the
+// exponent range (|x| in 2^+-896, d in 2^+-100); outside it, the division.
+__device__ __forceinline__ double quot3(double x, double d, double r) {
+    double q = x * r;
+    q = fma(fma(-d, q, x), r, q);
+    return fma(fma(-d, q, x), r, q);
+}
+__device__ __forceinline__ bool quot3_range(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return e - ((1023u - 896u) << 20) < (2u * 896u) << 20 || x == 0.0;
+}
+// the quotients outside that range, out of line: they hardly ever run
+template <class S>
+__device__ __noinline__ typename S::Split split3_far(typename S::real xp, typename S::real zb, typename S::real cb,
+                                                     typename S::real zm, typename S::real za,
+                                                     typename S::real ca) {
+    return S::split(xp, zb, cb, zm, za, ca);
+}
+
+// Role h = 0 owns flux3's y-like side (the rpt3 splits in e1, the rptt3 splits
+// of the z-like parts in e1, gadd), h = 1 the z-like side (splits in e2, hadd);
+// both solve the normal problem, limit and form cqxx (a few dozen operations,
+// duplicated).  A warp's role is a compile-time constant, so shared-memory
+// indexes fold to immediates.  The four combinations each side needs from the
+// other's splits (flux3.f90:363-376 and :488-495) cross through shared memory
+// under a 64-thread named barrier of the warp pair.  Operation order per value
+// is flux3's.
+//
+// A cell adds its terms in step3's colour order, which depends on its slice
+// indexes modulo 4: each thread sorts its neighbours once and keeps the shared
+// memory offsets of its terms in that order, the centre's own terms among them
+// (published like the neighbours'), so the gather is a run of loads and adds.
+//
+// The four rpt3 splits of a position, and the four rptt3 splits after the
+// exchange, are formed side by side so that their quotients overlap.
+//
+// Against pairs of neighbouring lanes with run-time roles, an IEEE division in
+// every quotient, the gather's indexes formed at every position and segments
+// of 64 cells whatever the grid, ms a step: 256^3 15.1 -> 11.0, 128^3 3.0 ->
+// 1.69, 64^3 1.53 -> 0.25.  99 warp instructions a cell and sweep for 151; the
+// FP64 pipe runs at 27 %, latency of dependent FP64 operations bounds it.
+__device__ __forceinline__ void pair_sync(int id) {
+    asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
+
+// The march of one tile of slices for the threads of role H; returns the
+// thread's Courant number.
+template <class S, int DIR, class M, int H>
+__device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::real>& a,
+                                                unsigned char* smem_raw, int* far) {
     using real = typename S::real;
     using Split = typename S::Split;
     constexpr int AXN = DIR, AXA = DIR == 0 ? 1 : 0, AXB = DIR == 2 ? 1 : 2;
     constexpr bool E1A = DIR != 1;
     constexpr int CN = 1 + AXN, CE1 = 1 + (E1A ? AXA : AXB), CE2 = 1 + (E1A ? AXB : AXA);
-    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NPL = NPL3;
+    // shared-memory steps of this role's own split direction and the other
+    constexpr int E1S = E1A ? 1 : S3A, E2S = E1A ? S3A : 1;
+    constexpr int OWNS = H ? E2S : E1S, OTHS = H ? E1S : E2S;
+    constexpr int CA = H ? CE1 : 0, CB = H ? CE2 : CN;  // components this role updates
 
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    real* saux = reinterpret_cast<real*>(smem_raw);  // [RING3][2][NS3]
-    real* sterm = saux + RING3 * 2 * NS3;            // [2][NTERM3][NT3]
-    real* sq = sterm + 2 * NTERM3 * NT3;             // [QST3][NT3]
-    double* red = reinterpret_cast<double*>(sq + QST3 * NT3);
+    real* saux = reinterpret_cast<real*>(smem_raw);  // [RING3][NPL][NS3]
+    real* sterm = saux + RING3 * NPL * NS3;          // [NTERM3][NT3]
+    real* sxch = sterm + NTERM3 * NT3;               // [XCH3][NT3]
+    real* sq = sxch + XCH3 * NT3;                    // [QST3][NT3]
+    real* sv = sq + QST3 * NT3;                      // [VST3][NT3]
 
     ClawCtl* ctl = a.ctl;
-    grid_dependency_sync();
-    if (ctl->done) return;
     const int cur = ctl->cur;
     const real* __restrict__ qold = a.q[cur];
     real* __restrict__ qnew = a.q[cur ^ 1];
@@ -165,6 +216,8 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
     const real S6g = (real(1.0) / real(6.0)) * tn * te2;
     const real S6h = (real(1.0) / real(6.0)) * tn * te1;
     const real dtdxave = real(0.5) * (tn + tn);
+    const real t_own = H ? te2 : te1;
+    const real S6own = H ? S6h : S6g;
 
     const int m3 = M::m3 >= 0 ? M::m3 : a.m3;
     const int m4 = M::m4 >= 0 ? M::m4 : a.m4;
@@ -175,20 +228,26 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
     const int seg = bid % a.nseg, tile = bid / a.nseg;
     const int A0 = 1 + (tile % a.tilesA) * (T3A - 2);
     const int B0 = 1 + (tile / a.tilesA) * (T3B - 2);
-    const int p0 = 1 + seg * SEG3;
-    const int p1 = min(p0 + SEG3, mN + 1);
+    const int p0 = 1 + seg * a.seglen;
+    const int p1 = min(p0 + a.seglen, mN + 1);
     const int tid = threadIdx.x;
-    const int h = tid & 1;           // 0: y-like side (gadd), 1: z-like side (hadd)
-    const int sl = tid >> 1;         // slice within the tile
+    const int warp = tid >> 5;
+    const int sl = (warp >> 1) * 32 + (tid & 31);  // slice within the tile
+    const int pair_id = 1 + (warp >> 1);           // named barrier of the warp pair
     const int ta = sl % T3A, tb = sl / T3A;
     const int A = A0 - 1 + ta, B = B0 - 1 + tb;
     const bool active = A <= mA + 1 && B <= mB + 1;
     const bool apply = active && ta >= 1 && ta <= T3A - 2 && tb >= 1 && tb <= T3B - 2 &&
                        A <= mA && B <= mB;
-    const unsigned amask = __ballot_sync(FULL, active);  // pairs are active together
 
-    unsigned long long perm = 0;
+    // step3's order of the cell's nine contributions (src/3d/step3.f90:151-186:
+    // colour of the slow slice index, colour of the fast one, slow, fast), as
+    // offsets into the published terms: planes off and off + 2.  Role 0's
+    // centre is two entries, (own sums) and (the transverse differences).
+    constexpr int NG = H ? 9 : 10;
+    int goff[NG];
     {
+        unsigned long long perm = 0;
         int code[9], key[9];
         for (int k = 0; k < 9; ++k) {
             const int da = k % 3 - 1, db = k / 3 - 1;
@@ -201,7 +260,21 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
                 int t = key[j]; key[j] = key[j - 1]; key[j - 1] = t;
                 t = code[j]; code[j] = code[j - 1]; code[j - 1] = t;
             }
-        for (int k = 0; k < 9; ++k) perm |= (unsigned long long)code[k] << (4 * k);
+        int kc = 0;  // place of the centre
+        for (int k = 0; k < 9; ++k) {
+            perm |= (unsigned long long)code[k] << (4 * k);
+            if (code[k] == 4) kc = k;
+        }
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            const int k = H == 0 && g > kc ? g - 1 : g;
+            const int cd = (int)((perm >> (4 * k)) & 15ull);
+            const int da = cd % 3 - 1, db = cd / 3 - 1;
+            const int u = E1A ? -da : -db, w = E1A ? -db : -da;
+            const int idx9 = (w + 1) * 3 + (u + 1);
+            const int nb = idx9 < 4 ? idx9 : idx9 - 1;
+            goff[g] = cd == 4 ? (H ? 36 : g == kc ? 32 : 33) * NT3 : (nb * 4 + H) * NT3 + db * T3A + da;
+        }
     }
 
     bool flipA, flipB;
@@ -226,10 +299,9 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             }
         }
     };
-    // Z and c of ring position pos, copied asynchronously: issued at the top
-    // of a position, awaited just before its CTA barrier
+    // Z and c of ring position pos, copied asynchronously
     auto load_aux = [&](int pos) {
-        real* dst = saux + (pos & (RING3 - 1)) * 2 * NS3;
+        real* dst = saux + (pos & (RING3 - 1)) * NPL * NS3;
         const long long pofs = (long long)(pos + 1) * a.as[AXN];
         for (int e = tid; e < NS3; e += NT3P) {
             const int sa = e % S3A, sb = e / S3A;
@@ -239,14 +311,32 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             cp_async_el(dst + NS3 + e, aux + o + a.afstride);
         }
     };
-    // q of this slice at position pos, staged the same way: h = 0 copies p,
-    // h = 1 the normal velocity; boundary conditions apply when the pair takes them
+    // 1 / (Z + Z_next) along A and B of ring position pos, from its landed Z.
+    // The next tile element is the next cell, or the same clamped cell past
+    // the grid's last ghost; the tile's last row and column are never read.
+    auto make_rcp = [&](int pos) {
+        real* dst = saux + (pos & (RING3 - 1)) * NPL * NS3;
+        for (int e = tid; e < NS3; e += NT3P) {
+            const int sa = e % S3A, sb = e / S3A;
+            if (sa == S3A - 1 || sb == S3B - 1) continue;
+            const real z = dst[e];
+            const real dA = z + dst[e + 1], dB = z + dst[e + S3A];
+            const real rA = real(1) / dA, rB = real(1) / dB;
+            // (2^-100 .. 2^100; false for NaN)
+            const bool in = dA > real(7.9e-31) && dA < real(1.2e30) && dB > real(7.9e-31) && dB < real(1.2e30);
+            if (!in) *far = 1;
+            dst[(E1A ? 2 : 3) * NS3 + e] = rA;
+            dst[(E1A ? 3 : 2) * NS3 + e] = rB;
+        }
+    };
+    // q of this slice at position pos: role 0 stages p, role 1 the normal
+    // velocity; boundary conditions are applied when the pair takes them
     auto issue_q = [&](int pos) {
         if (!active) return;
         bool fN;
         const int pm = bc3_src(pos, mN, a.bc[2 * AXN], a.bc[2 * AXN + 1], fN);
-        const long long off = qoffAB + (long long)(pm - 1) * a.qs[AXN] + (h ? CN * a.fstride : 0);
-        cp_async_el(sq + ((pos & 1) * 2 + h) * NT3 + sl, qold + off);
+        const long long off = qoffAB + (long long)(pm - 1) * a.qs[AXN] + (H ? CN * a.fstride : 0);
+        cp_async_el(sq + ((pos & 1) * 2 + H) * NT3 + sl, qold + off);
     };
     auto take_q = [&](int pos, real& qp, real& qn) {
         qp = sq[((pos & 1) * 2) * NT3 + sl];
@@ -263,31 +353,40 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             }
         }
     };
-    // shared-memory steps of this thread's own split direction and the other
     const int sown = (tb + 1) * S3A + (ta + 1);
-    const int e1s = E1A ? 1 : S3A, e2s = E1A ? S3A : 1;
-    const int ownS = h ? e2s : e1s, othS = h ? e1s : e2s;
-    auto Zo = [&](int pos, int o, int w) -> real {
-        return saux[(pos & (RING3 - 1)) * 2 * NS3 + sown + o * ownS + w * othS];
-    };
-    auto Co = [&](int pos, int o, int w) -> real {
-        return saux[(pos & (RING3 - 1)) * 2 * NS3 + NS3 + sown + o * ownS + w * othS];
+    auto plane = [&](int pos, int k) -> const real* {
+        return saux + (pos & (RING3 - 1)) * NPL * NS3 + k * NS3 + sown;
     };
     // split in the own direction of a fluctuation at the cell `w` across
-    auto split_own = [&](real xp, int pos, int w) -> Split {
-        return S::split(xp, Zo(pos, -1, w), Co(pos, -1, w), Zo(pos, 0, w), Zo(pos, 1, w), Co(pos, 1, w));
+    // (S::split with its quotients from the face reciprocals)
+    bool near = true;  // the medium's sums are in range (false is sticky)
+    auto split_near = [&](real xp, int pos, int w) -> Split {
+        const real* Zp = plane(pos, 0);
+        const real* Cp = plane(pos, 1);
+        const real* Rp = plane(pos, 2 + H);  // 1 / (Z + Z_next) along the own direction
+        const real zb = Zp[-OWNS + w * OTHS], zm = Zp[w * OTHS], za = Zp[OWNS + w * OTHS];
+        const real b1 = -quot3(xp, zb + zm, Rp[-OWNS + w * OTHS]);
+        const real b2 = quot3(xp, zm + za, Rp[w * OTHS]);
+        const real c1 = Cp[-OWNS + w * OTHS] * b1, c2 = Cp[OWNS + w * OTHS] * b2;
+        return Split{c1 * zb, -c1, c2 * za, c2};
     };
-    const real t_own = h ? te2 : te1;
-    const real S6own = h ? S6h : S6g;
+    auto split_far = [&](real xp, int pos, int w) -> Split {
+        const real* Zp = plane(pos, 0);
+        const real* Cp = plane(pos, 1);
+        return split3_far<S>(xp, Zp[-OWNS + w * OTHS], Cp[-OWNS + w * OTHS], Zp[w * OTHS], Zp[OWNS + w * OTHS],
+                             Cp[OWNS + w * OTHS]);
+    };
 
     double cfl = 0.0;
     auto solve = [&](int i, real pL, real uL, real pR, real uR, real w[2][2], real am[2], real ap[2]) {
         real s[2];
-        S::rpn(pL, uL, pR, uR, Zo(i - 1, 0, 0), Co(i - 1, 0, 0), Zo(i, 0, 0), Co(i, 0, 0), w, s, am, ap);
+        const real zl = *plane(i - 1, 0), cl = *plane(i - 1, 1);
+        const real zr = *plane(i, 0), cr = *plane(i, 1);
+        S::rpn(pL, uL, pR, uR, zl, cl, zr, cr, w, s, am, ap);
         if (i >= 1 && i <= mN + 1) {
-            for (int k = 0; k < 2; ++k) {
-                const double c = tn_d * (double)s[k];
-                cfl = fmax(fmax(cfl, c), -c);
+            for (int k = 0; k < 2; ++k) {  // fmax by select: a NaN leaves cfl
+                const double c = fabs(tn_d * (double)s[k]);
+                cfl = c > cfl ? c : cfl;
             }
         }
     };
@@ -299,6 +398,10 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
     issue_q(p0 + 1);
     cp_async_wait_all();
     __syncthreads();
+    make_rcp(p0 - 1);
+    make_rcp(p0);
+    __syncthreads();
+    near = *(volatile int*)far == 0;
 
     real wA[2][2], wB[2][2];
     real amB[2], apB[2];
@@ -320,6 +423,12 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
     }
     __syncthreads();
 
+    const bool xch = m3 > 0 && m4 > 0;  // the pair exchanges split combinations
+    // exchange planes: [side L/R][role][value] of NT3 slices each
+    auto xplane = [&](int side, int role, int v) -> real* {
+        return sxch + ((side * 2 + role) * 2 + v) * NT3 + sl;
+    };
+
     for (int p = p0 - 1; p < p1; ++p) {
         const bool emit = p >= p0;
         // position p+3: its ring slot and staged q were last read before the
@@ -328,23 +437,30 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             load_aux(p + 3);
             issue_q(p + 3);
         }
-        const int cA = h ? CE1 : 0, cB = h ? CE2 : CN;  // components this thread updates
+        near = near && *(volatile int*)far == 0;  // (set before the last barrier)
+        // the reciprocals of position p+2 (its Z landed before the last barrier)
+        if (p + 2 <= p1 + 1) make_rcp(p + 2);
+        const real* vsrc = DIR == 0 ? qold : qnew;
         real vA = 0, vB = 0;
-        if (emit && apply) {
-            const long long off = qoffAB + (long long)(p - 1) * a.qs[AXN];
-            const real* src = DIR == 0 ? qold : qnew;
-            vA = src[off + cA * a.fstride];
-            vB = src[off + cB * a.fstride];
+        // the cell values of position p+1, staged for the next position (only
+        // this thread writes that cell, at that position)
+        if (apply && p + 1 >= p0 && p + 1 < p1) {
+            const long long off = qoffAB + (long long)p * a.qs[AXN];
+            real* dv = sv + (((p + 1) & 1) * 2 + H) * 2 * NT3 + sl;
+            cp_async_el(dv, vsrc + off + CA * a.fstride);
+            cp_async_el(dv + NT3, vsrc + off + CB * a.fstride);
         }
         real F1[2] = {0, 0};
         real Qp[2] = {0, 0};
-        real wC[2][2], amC[2], apC[2], qRp = 0, qRn = 0;
-        real cterm = 0, own_c = 0;  // centre terms: sent to the partner / kept
+        real wC[2][2] = {}, amC[2] = {}, apC[2] = {}, qRp = 0, qRn = 0;
+        real cq[2] = {0, 0};
+        Split ma = {0, 0, 0, 0}, mp = {0, 0, 0, 0}, qm = {0, 0, 0, 0}, qp = {0, 0, 0, 0};
+        const int L = p, R = p + 1;
         if (active) {
             take_q(p + 2, qRp, qRn);
             solve(p + 2, qLp, qLn, qRp, qRn, wC, amC, apC);
             real wl[2][2];
-            const real sB[2] = {-Co(p, 0, 0), Co(p + 1, 0, 0)};
+            const real sB[2] = {-*plane(p, 1), *plane(p + 1, 1)};
             for (int k = 0; k < 2; ++k) {
                 wl[k][0] = wB[k][0];
                 wl[k][1] = wB[k][1];
@@ -354,14 +470,13 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
                     if (wn2 != real(0)) {
                         const real dl = wA[k][0] * wB[k][0] + wA[k][1] * wB[k][1];
                         const real dr = wB[k][0] * wC[k][0] + wB[k][1] * wC[k][1];
-                        const real r = (sB[k] > real(0) ? dl : dr) / wn2;
+                        const real r = div_ieee(sB[k] > real(0) ? dl : dr, wn2);
                         const real phi = phi_limiter<real>(lim, r);
                         wl[k][0] = phi * wB[k][0];
                         wl[k][1] = phi * wB[k][1];
                     }
                 }
             }
-            real cq[2] = {0, 0};
             if (order == 2) {
                 for (int k = 0; k < 2; ++k) {
                     const real as_ = fabs(sB[k]);
@@ -377,143 +492,164 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             Qs[0] = real(0) - tn * apB[0];
             Qs[1] = real(0) - tn * apB[1];
 
-            const int L = p, R = p + 1;
-            // ---- cell p: the amdq side of interface p+1 completes gadd/hadd
+            // ---- the four rpt3 splits of interface p+1, side by side (their
+            // quotients overlap): A-dq and cqxx at cell p, A+dq and cqxx at p+1
             if (m3 > 0) {
-                const Split ma = split_own(amB[0], L, 0);
-                Split qm = {0, 0, 0, 0};
-                if (m3 == 2) qm = split_own(cq[0], L, 0);
+                if (near && quot3_range(amB[0]) && quot3_range(apB[0]) && quot3_range(cq[0])) {
+                    ma = split_near(amB[0], L, 0);
+                    mp = split_near(apB[0], R, 0);
+                    if (m3 == 2) {
+                        qm = split_near(cq[0], L, 0);
+                        qp = split_near(cq[0], R, 0);
+                    }
+                } else {
+                    ma = split_far(amB[0], L, 0);
+                    mp = split_far(apB[0], R, 0);
+                    if (m3 == 2) {
+                        qm = split_far(cq[0], L, 0);
+                        qp = split_far(cq[0], R, 0);
+                    }
+                }
+                if (m4 > 0) {
+                    // the combinations the partner splits (flux3.f90:363-376, 488-495)
+                    real x1 = ma.up, x3 = ma.dp, x0 = mp.up, x2 = mp.dp;
+                    if (m4 == 2) {
+                        x1 = ma.up + real(3) * qm.up;
+                        x3 = ma.dp + real(3) * qm.dp;
+                        x0 = mp.up - real(3) * qp.up;
+                        x2 = mp.dp - real(3) * qp.dp;
+                    }
+                    *xplane(0, H, 0) = x1;
+                    *xplane(0, H, 1) = x3;
+                    *xplane(1, H, 0) = x0;
+                    *xplane(1, H, 1) = x2;
+                }
+                // cell p: the amdq side of interface p+1 completes gadd/hadd
                 O[0][1][0] = O[0][1][0] - H5 * ma.dp;
                 O[0][1][1] = O[0][1][1] - H5 * ma.dt;
                 O[1][1][0] = O[1][1][0] - H5 * ma.up;
                 O[1][1][1] = O[1][1][1] - H5 * ma.ut;
-                if (m4 > 0) {
-                    // the combinations the partner splits (flux3.f90:363-376, 488-495)
-                    real x1 = ma.up, x3 = ma.dp;
-                    if (m4 == 2) {
-                        x1 = ma.up + real(3) * qm.up;
-                        x3 = ma.dp + real(3) * qm.dp;
-                    }
-                    const real y1 = __shfl_xor_sync(amask, x1, 1);
-                    const real y3 = __shfl_xor_sync(amask, x3, 1);
-                    const Split tpm = split_own(y1, L, 1), tmm = split_own(y3, L, -1);
-                    O[1][1][0] = O[1][1][0] + S6own * (tpm.up - tmm.up);
-                    O[1][1][1] = O[1][1][1] + S6own * (tpm.ut - tmm.ut);
-                    O[0][1][0] = O[0][1][0] + S6own * (tpm.dp - tmm.dp);
-                    O[0][1][1] = O[0][1][1] + S6own * (tpm.dt - tmm.dt);
-                    O[1][2][0] = O[1][2][0] - S6own * tpm.up;
-                    O[1][2][1] = O[1][2][1] - S6own * tpm.ut;
-                    O[0][2][0] = O[0][2][0] - S6own * tpm.dp;
-                    O[0][2][1] = O[0][2][1] - S6own * tpm.dt;
-                    O[1][0][0] = O[1][0][0] + S6own * tmm.up;
-                    O[1][0][1] = O[1][0][1] + S6own * tmm.ut;
-                    O[0][0][0] = O[0][0][0] + S6own * tmm.dp;
-                    O[0][0][1] = O[0][0][1] + S6own * tmm.dt;
+            }
+        }
+        Split tpp = {0, 0, 0, 0}, tmp = {0, 0, 0, 0};
+        if (xch) {
+            pair_sync(pair_id);
+            if (active) {
+                const real y1 = *xplane(0, 1 - H, 0), y3 = *xplane(0, 1 - H, 1);
+                const real y0 = *xplane(1, 1 - H, 0), y2 = *xplane(1, 1 - H, 1);
+                Split tpm, tmm;
+                if (near && quot3_range(y0) && quot3_range(y1) && quot3_range(y2) && quot3_range(y3)) {
+                    tpm = split_near(y1, L, 1);
+                    tmm = split_near(y3, L, -1);
+                    tpp = split_near(y0, R, 1);
+                    tmp = split_near(y2, R, -1);
+                } else {
+                    tpm = split_far(y1, L, 1);
+                    tmm = split_far(y3, L, -1);
+                    tpp = split_far(y0, R, 1);
+                    tmp = split_far(y2, R, -1);
                 }
-                if (m3 == 2) {
-                    O[1][1][0] = O[1][1][0] - tn * qm.up;
-                    O[1][1][1] = O[1][1][1] - tn * qm.ut;
-                    O[0][1][0] = O[0][1][0] - tn * qm.dp;
-                    O[0][1][1] = O[0][1][1] - tn * qm.dt;
-                }
+                O[1][1][0] = O[1][1][0] + S6own * (tpm.up - tmm.up);
+                O[1][1][1] = O[1][1][1] + S6own * (tpm.ut - tmm.ut);
+                O[0][1][0] = O[0][1][0] + S6own * (tpm.dp - tmm.dp);
+                O[0][1][1] = O[0][1][1] + S6own * (tpm.dt - tmm.dt);
+                O[1][2][0] = O[1][2][0] - S6own * tpm.up;
+                O[1][2][1] = O[1][2][1] - S6own * tpm.ut;
+                O[0][2][0] = O[0][2][0] - S6own * tpm.dp;
+                O[0][2][1] = O[0][2][1] - S6own * tpm.dt;
+                O[1][0][0] = O[1][0][0] + S6own * tmm.up;
+                O[1][0][1] = O[1][0][1] + S6own * tmm.ut;
+                O[0][0][0] = O[0][0][0] + S6own * tmm.dp;
+                O[0][0][1] = O[0][0][1] + S6own * tmm.dt;
+            }
+        }
+        if (active) {
+            if (m3 == 2) {
+                O[1][1][0] = O[1][1][0] - tn * qm.up;
+                O[1][1][1] = O[1][1][1] - tn * qm.ut;
+                O[0][1][0] = O[0][1][0] - tn * qm.dp;
+                O[0][1][1] = O[0][1][1] - tn * qm.dt;
             }
             if (emit) {
                 // terms for the eight neighbours: own offset o (the side), other w (the level)
-                real* out = sterm + (p & 1) * NTERM3 * NT3 + sl;
+                real* out = sterm + sl;
+#pragma unroll
                 for (int w = -1; w <= 1; ++w)
+#pragma unroll
                     for (int o = -1; o <= 1; ++o) {
                         if (o == 0 && w == 0) continue;
-                        const int de1 = h ? w : o, de2 = h ? o : w;
+                        const int de1 = H ? w : o, de2 = H ? o : w;
                         const int idx9 = (de2 + 1) * 3 + (de1 + 1);
                         const int nb = idx9 < 4 ? idx9 : idx9 - 1;
+#pragma unroll
                         for (int c = 0; c < 2; ++c) {
                             const real tv = o < 0 ? -(t_own * O[0][w + 1][c])
                                           : o == 0 ? -(t_own * (O[1][w + 1][c] - O[0][w + 1][c]))
                                                    : t_own * O[1][w + 1][c];
-                            out[(nb * 4 + 2 * h + c) * NT3] = tv;
+                            out[(nb * 4 + 2 * H + c) * NT3] = tv;
                         }
                     }
-                // centre: h = 0 keeps te1*dG_p and sends te1*dG_e1; h = 1
-                // keeps te2*dH_e2 and sends te2*dH_p
+                // centre: h = 0 subtracts its own sums, te1*dG_p and te2*dH_p
+                // from p and sends te1*dG_e1; h = 1 subtracts te2*dH_e2 and
+                // sends te2*dH_p
                 const real dp_ = t_own * (O[1][1][0] - O[0][1][0]);
                 const real dv_ = t_own * (O[1][1][1] - O[0][1][1]);
-                cterm = h ? dp_ : dv_;
-                own_c = h ? dv_ : dp_;
+                if (H == 0) {
+                    out[32 * NT3] = Qp[0];
+                    out[34 * NT3] = -(tn * (F1[0] - F0[0]));
+                    out[33 * NT3] = -dp_;
+                    out[36 * NT3] = -dv_;
+                } else {
+                    out[35 * NT3] = -dp_;
+                    out[38 * NT3] = -dv_;
+                }
             }
             // ---- cell p+1: the apdq side of interface p+1 starts gadd/hadd
-            for (int s_ = 0; s_ < 2; ++s_)
-                for (int l = 0; l < 3; ++l)
-                    for (int c = 0; c < 2; ++c) O[s_][l][c] = 0;
-            if (m3 > 0) {
-                const Split mp = split_own(apB[0], R, 0);
-                Split qp = {0, 0, 0, 0};
-                if (m3 == 2) qp = split_own(cq[0], R, 0);
-                O[0][1][0] = O[0][1][0] - H5 * mp.dp;
-                O[0][1][1] = O[0][1][1] - H5 * mp.dt;
-                O[1][1][0] = O[1][1][0] - H5 * mp.up;
-                O[1][1][1] = O[1][1][1] - H5 * mp.ut;
-                if (m4 > 0) {
-                    real x0 = mp.up, x2 = mp.dp;
-                    if (m4 == 2) {
-                        x0 = mp.up - real(3) * qp.up;
-                        x2 = mp.dp - real(3) * qp.dp;
-                    }
-                    const real y0 = __shfl_xor_sync(amask, x0, 1);
-                    const real y2 = __shfl_xor_sync(amask, x2, 1);
-                    const Split tpp = split_own(y0, R, 1), tmp = split_own(y2, R, -1);
-                    O[1][1][0] = O[1][1][0] + S6own * (tpp.up - tmp.up);
-                    O[1][1][1] = O[1][1][1] + S6own * (tpp.ut - tmp.ut);
-                    O[0][1][0] = O[0][1][0] + S6own * (tpp.dp - tmp.dp);
-                    O[0][1][1] = O[0][1][1] + S6own * (tpp.dt - tmp.dt);
-                    O[1][2][0] = O[1][2][0] - S6own * tpp.up;
-                    O[1][2][1] = O[1][2][1] - S6own * tpp.ut;
-                    O[0][2][0] = O[0][2][0] - S6own * tpp.dp;
-                    O[0][2][1] = O[0][2][1] - S6own * tpp.dt;
-                    O[1][0][0] = O[1][0][0] + S6own * tmp.up;
-                    O[1][0][1] = O[1][0][1] + S6own * tmp.ut;
-                    O[0][0][0] = O[0][0][0] + S6own * tmp.dp;
-                    O[0][0][1] = O[0][0][1] + S6own * tmp.dt;
-                }
-                if (m3 == 2) {
-                    O[1][1][0] = O[1][1][0] + tn * qp.up;
-                    O[1][1][1] = O[1][1][1] + tn * qp.ut;
-                    O[0][1][0] = O[0][1][0] + tn * qp.dp;
-                    O[0][1][1] = O[0][1][1] + tn * qp.dt;
-                }
+            // (0 - x written as -x: the same value)
+            O[0][1][0] = -(H5 * mp.dp);
+            O[0][1][1] = -(H5 * mp.dt);
+            O[1][1][0] = -(H5 * mp.up);
+            O[1][1][1] = -(H5 * mp.ut);
+            O[1][1][0] = O[1][1][0] + S6own * (tpp.up - tmp.up);
+            O[1][1][1] = O[1][1][1] + S6own * (tpp.ut - tmp.ut);
+            O[0][1][0] = O[0][1][0] + S6own * (tpp.dp - tmp.dp);
+            O[0][1][1] = O[0][1][1] + S6own * (tpp.dt - tmp.dt);
+            O[1][2][0] = -(S6own * tpp.up);
+            O[1][2][1] = -(S6own * tpp.ut);
+            O[0][2][0] = -(S6own * tpp.dp);
+            O[0][2][1] = -(S6own * tpp.dt);
+            O[1][0][0] = S6own * tmp.up;
+            O[1][0][1] = S6own * tmp.ut;
+            O[0][0][0] = S6own * tmp.dp;
+            O[0][0][1] = S6own * tmp.dt;
+            if (m3 == 2) {
+                O[1][1][0] = O[1][1][0] + tn * qp.up;
+                O[1][1][1] = O[1][1][1] + tn * qp.ut;
+                O[0][1][0] = O[0][1][0] + tn * qp.dp;
+                O[0][1][1] = O[0][1][1] + tn * qp.dt;
             }
         }
-        const real crecv = __shfl_xor_sync(FULL, cterm, 1);
         cp_async_wait_all();
         __syncthreads();
         if (emit && apply) {
-            const real* in = sterm + (p & 1) * NTERM3 * NT3;
-            for (int k = 0; k < 9; ++k) {
-                const int code = (int)((perm >> (4 * k)) & 15ull);
-                if (code == 4) {
-                    if (h == 0) {
-                        vA = vA + Qp[0] - tn * (F1[0] - F0[0]) - own_c - crecv;
-                        vB = vB + Qp[1] - tn * (F1[1] - F0[1]);
-                    } else {
-                        vA = vA - crecv;
-                        vB = vB - own_c;
-                    }
-                } else {
-                    const int da = code % 3 - 1, db = code / 3 - 1;
-                    const int u = E1A ? -da : -db, w = E1A ? -db : -da;
-                    const int idx9 = (w + 1) * 3 + (u + 1);
-                    const int nb = idx9 < 4 ? idx9 : idx9 - 1;
-                    const int src = sl + db * T3A + da;
-                    if (h == 0) {
-                        vA = vA + in[(nb * 4 + 0) * NT3 + src] + in[(nb * 4 + 2) * NT3 + src];
-                    } else {
-                        vA = vA + in[(nb * 4 + 1) * NT3 + src];
-                        vB = vB + in[(nb * 4 + 3) * NT3 + src];
-                    }
+            const real* vv = sv + ((p & 1) * 2 + H) * 2 * NT3 + sl;
+            vA = vv[0];
+            vB = vv[NT3];
+            const real* in = sterm + sl;
+            if (H == 0) {
+#pragma unroll
+                for (int g = 0; g < NG; ++g) vA = vA + in[goff[g]] + in[goff[g] + 2 * NT3];
+                vB = vB + Qp[1] - tn * (F1[1] - F0[1]);
+            } else {
+#pragma unroll
+                for (int g = 0; g < NG; ++g) {
+                    vA = vA + in[goff[g]];
+                    vB = vB + in[goff[g] + 2 * NT3];
                 }
             }
             const long long off = qoffAB + (long long)(p - 1) * a.qs[AXN];
-            qnew[off + cA * a.fstride] = vA;
-            qnew[off + cB * a.fstride] = vB;
+            qnew[off + CA * a.fstride] = vA;
+            qnew[off + CB * a.fstride] = vB;
         }
         if (active) {
             for (int k = 0; k < 2; ++k)
@@ -523,15 +659,34 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
             qLp = qRp; qLn = qRn;
             F0[0] = F1[0]; F0[1] = F1[1];
         }
+        // one term buffer: every gather of p ends before a publish of p+1
+        __syncthreads();
     }
+    return cfl;
+}
 
+template <class S, int DIR, class M, bool LAST>
+__global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const Sweep3Args<typename S::real> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using real = typename S::real;
+    double* red = reinterpret_cast<double*>(reinterpret_cast<real*>(smem_raw) +
+                                            RING3 * NPL3 * NS3 + (NTERM3 + XCH3 + QST3 + VST3) * NT3);
+    __shared__ int far;  // some Z + Z' of the tile is out of quot3's range
+    ClawCtl* ctl = a.ctl;
+    grid_dependency_sync();
+    if (ctl->done) return;
+    if (threadIdx.x == 0) far = 0;  // (a CTA barrier precedes the first reciprocal)
+    // warps 2k (role 0) and 2k+1 (role 1) share 32 slices
+    const double cfl = ((threadIdx.x >> 5) & 1) ? sweep3p_march<S, DIR, M, 1>(a, smem_raw, &far)
+                                                : sweep3p_march<S, DIR, M, 0>(a, smem_raw, &far);
     if (LAST) {
         cta_cfl_and_control(ctl, cfl, red);
     } else {
-        for (int off = 16; off > 0; off >>= 1) cfl = fmax(cfl, __shfl_xor_sync(FULL, cfl, off));
-        if ((tid & 31) == 0) red[tid >> 5] = cfl;
+        double c = cfl;
+        for (int off = 16; off > 0; off >>= 1) c = fmax(c, __shfl_xor_sync(0xffffffffu, c, off));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
         __syncthreads();
-        if (tid == 0) {
+        if (threadIdx.x == 0) {
             double m = 0.0;
             for (int w = 0; w < NT3P / 32; ++w) m = fmax(m, red[w]);
             if (!(m > 0.0)) m = (m != m) ? m : 0.0;

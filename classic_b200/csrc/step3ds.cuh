@@ -127,7 +127,7 @@ __device__ __forceinline__ void ds3_flux(const Split3Args<real>& a, const real (
         if (lim > 0) {
             const real wn2 = w[k][0] * w[k][0] + w[k][1] * w[k][1];
             if (wn2 != real(0)) {
-                const real r = (s[k] > real(0) ? dl[k] : dr[k]) / wn2;
+                const real r = div_ieee(s[k] > real(0) ? dl[k] : dr[k], wn2);
                 const real phi = phi_limiter<real>(lim, r);
                 w0 = phi * w[k][0];
                 w1 = phi * w[k][1];
