@@ -129,6 +129,7 @@ SIGNATURES = {
     # learned corrector kernels (include/claw_nn.h)
     "nn_conv3x3_forward": (ctypes.c_int, [_P, _P, _P, _P, _P] + [ctypes.c_int] * 7 + [_P]),
     "nn_conv3x3_wgrad": (ctypes.c_int, [_P] * 6 + [ctypes.c_int] * 5 + [_P]),
+    "nn_conv3x3_dgrad": (ctypes.c_int, [_P] * 4 + [ctypes.c_int] * 5 + [_P]),
     "nn_device_error": (ctypes.c_int, [ctypes.c_int]),
     "nn_flip_weights": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int, _P]),
     "nn_gelu_backward": (ctypes.c_int, [_P, _P, _P, ctypes.c_longlong, _P]),
@@ -136,6 +137,8 @@ SIGNATURES = {
                                    ctypes.c_float, _P]),
     "nn_adam": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_longlong] + [ctypes.c_float] * 4 +
                 [ctypes.c_int, _P]),
+    "nn_adam_multi": (ctypes.c_int, [ctypes.c_int] + [_P] * 6 + [ctypes.c_float] * 4 +
+                      [ctypes.c_int, _P]),
     "nn_block_average": (ctypes.c_int, [_P, ctypes.c_longlong, ctypes.c_longlong, _P,
                                         ctypes.c_longlong, ctypes.c_longlong] + [ctypes.c_int] * 4 +
                          [_P]),

@@ -123,7 +123,6 @@ class ConvNet:
         nblk = n * (h // 16) * (w // 16)
         c["partial"] = torch.empty(nblk * 32 * 9 * 32, dtype=torch.float32, device="cuda")
         c["pdb"] = torch.empty(nblk * 32, dtype=torch.float32, device="cuda")
-        c["wt"] = torch.empty(32 * 9 * 32, dtype=torch.bfloat16, device="cuda")
         c["loss"] = torch.zeros(1, dtype=torch.float64, device="cuda")
         self._cache = c
         return c
@@ -151,44 +150,30 @@ class ConvNet:
         n, h, w, _ = dy.shape
         c = self._cache
         st = _stream()
-        d = dy
+        dz = dy  # the last layer has no activation
         for k in range(len(LAYERS) - 1, -1, -1):
             cin, cout, act = LAYERS[k]
-            if act:
-                dz = c["d32a"] if d is not c["d32a"] else c["d32b"]
-                check(self.lib.nn_gelu_backward(_p(d), _p(c["zs"][k]), _p(dz), d.numel(), st),
-                      "nn_gelu_backward")
-            else:
-                dz = d
             a_in = c["x"] if k == 0 else c["acts"][k - 1]
             check(self.lib.nn_conv3x3_wgrad(_p(a_in), _p(dz), _p(c["partial"]), _p(c["pdb"]),
                                             _p(self.gw[k]), _p(self.gb[k]), n, h, w, cin, cout, st),
                   "nn_conv3x3_wgrad")
-            if k > 0:
-                check(self.lib.nn_flip_weights(_p(self.w16[k]), _p(c["wt"]), cout, cin, st),
-                      "nn_flip_weights")
+            if k > 0:  # through this layer's weights and the activation below them
                 dx = c["d32b"] if dz is c["d32a"] else c["d32a"]
-                check(self.lib.nn_conv3x3_forward(_p(dz), _p(c["wt"]), _p(self._zero_bias(cin)),
-                                                  _p(dx), None, n, h, w, cout, cin, 0, 0, st),
-                      "nn_conv3x3_forward (data gradient)")
-                d = dx
-
-    def _zero_bias(self, n):
-        torch = _torch()
-        if not hasattr(self, "_zb"):
-            self._zb = torch.zeros(64, device="cuda")
-        return self._zb
+                check(self.lib.nn_conv3x3_dgrad(_p(dz), _p(self.w16[k]), _p(c["zs"][k - 1]), _p(dx), n, h, w,
+                                                cin, cout, st), "nn_conv3x3_dgrad")
+                dz = dx
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1
-        st = _stream()
-        for k in range(len(LAYERS)):
-            check(self.lib.nn_adam(_p(self.w32[k]), _p(self.gw[k]), _p(self.m[k]), _p(self.v[k]),
-                                   _p(self.w16[k]), self.w32[k].numel(), lr, b1, b2, eps,
-                                   self.step_count, st), "nn_adam")
-            check(self.lib.nn_adam(_p(self.b[k]), _p(self.gb[k]), _p(self.mb[k]), _p(self.vb[k]),
-                                   None, self.b[k].numel(), lr, b1, b2, eps, self.step_count, st),
-                  "nn_adam")
+        w, g = self.w32 + self.b, self.gw + self.gb
+        m, v = self.m + self.mb, self.v + self.vb
+        w16 = list(self.w16) + [None] * len(self.b)
+        count = len(w)
+        ptrs = [(ctypes.c_void_p * count)(*(None if t is None else t.data_ptr() for t in lst))
+                for lst in (w, g, m, v, w16)]
+        sizes = (ctypes.c_longlong * count)(*(t.numel() for t in w))
+        check(self.lib.nn_adam_multi(count, *ptrs, sizes, lr, b1, b2, eps, self.step_count, _stream()),
+              "nn_adam_multi")
 
     def loss_grad(self, pred, target, delta=0.0):
         """MSE (delta = 0) or Huber loss on the 4 output channels (NaN targets

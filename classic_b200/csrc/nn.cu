@@ -45,9 +45,6 @@ __device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], const 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-__device__ __forceinline__ uint32_t ld32(const __nv_bfloat16* p) {
-    return *reinterpret_cast<const uint32_t*>(p);
-}
 __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
@@ -75,22 +72,6 @@ __device__ __forceinline__ float gelu_grad(float z) {
     const float t = tanh_hw(GELU_K0 * fmaf(GELU_K1 * z, z * z, z));
     const float du = GELU_K0 * fmaf(3.0f * GELU_K1 * z, z, 1.0f);
     return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * du;
-}
-
-// Load a HALO x HALO x CP input tile (zero outside the image) into shared
-// memory with a row pitch of CP + 8 elements (conflict-free fragment loads).
-template <int CP>
-__device__ __forceinline__ void load_halo(__nv_bfloat16* xs, const __nv_bfloat16* x, int n, int h,
-                                          int w, int y0, int x0) {
-    constexpr int CH = CP / 8;  // 16-byte chunks per pixel
-    for (int e = threadIdx.x; e < HALO * HALO * CH; e += NTHREADS) {
-        const int pix = e / CH, ck = e % CH;
-        const int gy = y0 + pix / HALO - 1, gx = x0 + pix % HALO - 1;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (gy >= 0 && gy < h && gx >= 0 && gx < w)
-            v = *reinterpret_cast<const uint4*>(x + (((long long)n * h + gy) * w + gx) * CP + ck * 8);
-        *reinterpret_cast<uint4*>(xs + pix * (CP + 8) + ck * 8) = v;
-    }
 }
 
 // ------------------------------------------------- forward conv, tcgen05 ---
@@ -193,11 +174,16 @@ __host__ __device__ constexpr int smem_bytes() {
 }
 }  // namespace tcp
 
-template <int CIN, int COUT, int ACT, bool OUTF32, bool SAVEZ>
+// DGRAD: the data gradient of a layer.  The weights are the layer's own
+// [CIN][9][COUT], read flipped and transposed as they are staged (no
+// flip_weights launch), and with zin the epilogue multiplies by GELU'(z) of the
+// layer below, rounding to BF16 before and after as the separate pass does.
+template <int CIN, int COUT, int ACT, bool OUTF32, bool SAVEZ, bool DGRAD = false>
 __global__ void __launch_bounds__(tcp::NTH, 1) conv3x3_fwd_tcp(const __nv_bfloat16* __restrict__ x,
                                                             const __nv_bfloat16* __restrict__ wt,
                                                             const float* __restrict__ bias, void* out,
-                                                            float* __restrict__ zsave, int n, int h,
+                                                            float* __restrict__ zsave,
+                                                            const float* __restrict__ zin, int n, int h,
                                                             int w, const __grid_constant__ CUtensorMap tmx) {
     using namespace tc;
     static_assert(CIN % 16 == 0 && (COUT == 16 || COUT == 32), "UMMA M128: N in {16, 32}, K in steps of 16");
@@ -278,8 +264,18 @@ __global__ void __launch_bounds__(tcp::NTH, 1) conv3x3_fwd_tcp(const __nv_bfloat
             float z[16], yv[16];
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
-                z[q] = __uint_as_float(rr[c0 + q]) + bs[c0 + q];
+                z[q] = DGRAD ? __uint_as_float(rr[c0 + q]) : __uint_as_float(rr[c0 + q]) + bs[c0 + q];
                 yv[q] = ACT ? gelu(z[q]) : z[q];
+            }
+            if (DGRAD && zin) {
+#pragma unroll
+                for (int q = 0; q < 16; q += 4) {
+                    const float4 zl = *reinterpret_cast<const float4*>(zin + pix * COUT + c0 + q);
+                    const float zv[4] = {zl.x, zl.y, zl.z, zl.w};
+#pragma unroll
+                    for (int r4 = 0; r4 < 4; ++r4)
+                        yv[q + r4] = __bfloat162float(__float2bfloat16_rn(yv[q + r4])) * gelu_grad(zv[r4]);
+                }
             }
             if (SAVEZ) {
 #pragma unroll
@@ -308,12 +304,23 @@ __global__ void __launch_bounds__(tcp::NTH, 1) conv3x3_fwd_tcp(const __nv_bfloat
     // the first two halo copies fly while the weights are staged
     load_tile(first, 0);
     load_tile(first + stride, 1);
-    for (int e = tid; e < COUT * 9 * KC; e += tcp::NTH) {  // wt[co][tap][ci] -> [tap][kc][co]
-        const int co = e / (9 * KC), r = e % (9 * KC), tap = r / KC, kc = r % KC;
-        *reinterpret_cast<uint4*>(Bs + (tap * KC + kc) * BPLANE + co * 16) =
-            *reinterpret_cast<const uint4*>(wt + ((long long)co * 9 + tap) * CIN + kc * 8);
+    if (DGRAD) {
+        for (int e = tid; e < COUT * 9 * KC; e += tcp::NTH) {  // w[ci][8 - tap][co] -> [tap][kc][co]
+            const int co = e % COUT, r = e / COUT, tap = r / KC, kc = r % KC;
+            const __nv_bfloat16* src = wt + ((kc * 8) * 9 + 8 - tap) * COUT + co;
+            uint32_t v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = pack2(src[2 * i * 9 * COUT], src[(2 * i + 1) * 9 * COUT]);
+            *reinterpret_cast<uint4*>(Bs + (tap * KC + kc) * BPLANE + co * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+    } else {
+        for (int e = tid; e < COUT * 9 * KC; e += tcp::NTH) {  // wt[co][tap][ci] -> [tap][kc][co]
+            const int co = e / (9 * KC), r = e % (9 * KC), tap = r / KC, kc = r % KC;
+            *reinterpret_cast<uint4*>(Bs + (tap * KC + kc) * BPLANE + co * 16) =
+                *reinterpret_cast<const uint4*>(wt + ((long long)co * 9 + tap) * CIN + kc * 8);
+        }
+        for (int e = tid; e < COUT; e += tcp::NTH) bs[e] = bias[e];
     }
-    for (int e = tid; e < COUT; e += tcp::NTH) bs[e] = bias[e];
     clawb200::fence_proxy_async_smem();  // the tensor core reads the weights these threads wrote
     fence_before();
     __syncthreads();  // barriers initialised, weights in place, TMEM allocated
@@ -371,91 +378,173 @@ __global__ void __launch_bounds__(tcp::NTH, 1) conv3x3_fwd_tcp(const __nv_bfloat
 
 
 // ------------------------------------------------------- weight gradient ---
-// partial[blk][co][tap*CIN + ci] = sum over the tile's pixels p of
-//   dz[p, co] * x[p + off(tap), ci];  pdb[blk][co] = sum_p dz[p, co].
-// GEMM M = COUT (dz transposed in shared memory), N = 9*CIN (im2col of the
-// halo tile), K = the tile's 256 pixels.
+// dw[co][tap*CIN + ci] = sum over pixels p of dz[p, co] * x[p + off(tap), ci],
+// db[co] = sum_p dz[p, co].  A GEMM with M = COUT, N = 9 x CIN and K = all the
+// pixels: too narrow in M (16 or 32) for a tcgen05 MMA, so mma.sync, one partial
+// result per 16x16-pixel tile (K = its 256 pixels), added over the tiles in
+// order by reduce_tiles.  A CTA takes every gridDim.x-th tile, the next one
+// arriving by cp.async meanwhile.  Nine warps are the nine taps, each COUT x CIN
+// of outputs; a tenth adds dz's channels for db.  Both operands lie in shared
+// memory as they come, [pixel][channel], and ldmatrix's transposed form hands
+// them to the MMA as [channel][pixel] fragments: no transposed copy, four
+// ldmatrix and eight MMAs per 16 pixels.
+//
+// 16 x 64^2, 32 -> 32 channels, under ncu: 24.8 + 51 us (2-byte fragment loads,
+// one thread adding a tile's dz after another, 36 blocks adding the partials
+// with a few loads in flight each) -> 11.1 + 6.0 us, the same sums in the same
+// order.  What is left is latency: 256 tiles on 148 SMs, one chain of additions
+// a column.
+constexpr int WTHREADS = 10 * 32;
+
+__device__ __forceinline__ void ldsm_x4_t(uint32_t r[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
+}
+// 16 bytes global -> shared, asynchronously; zeros where in is false
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(clawb200::smem_u32(dst)), "l"(src),
+                 "r"(in ? 16 : 0)
+                 : "memory");
+}
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(NTHREADS) conv3x3_wgrad(const __nv_bfloat16* __restrict__ x,
-                                                           const __nv_bfloat16* __restrict__ dz,
-                                                           float* __restrict__ partial,
-                                                           float* __restrict__ pdb, int h, int w) {
-    constexpr int XP = CIN + 8, DP = NPIX + 8;
-    constexpr int MT = COUT / 16, NT = 9 * CIN / 8, TILES = MT * NT, TPW = (TILES + 7) / 8;
+__host__ __device__ constexpr int wgrad_stage() {  // bytes: halo tile, then dz tile, rows padded against bank conflicts
+    return HALO * HALO * (CIN + 8) * 2 + NPIX * (COUT + 8) * 2;
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(WTHREADS) conv3x3_wgrad(const __nv_bfloat16* __restrict__ x,
+                                                          const __nv_bfloat16* __restrict__ dz,
+                                                          float* __restrict__ partial,
+                                                          float* __restrict__ pdb, int h, int w,
+                                                          int ntiles, bool dz16) {
+    constexpr int XP = CIN + 8, DP = COUT + 8, XC = CIN / 8, DC = COUT / 8;
+    constexpr int MT = COUT / 16, NT = CIN / 16;  // 16-wide tiles of co and of ci
     extern __shared__ __align__(16) unsigned char smem[];
-    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem);
-    __nv_bfloat16* dzt = xs + HALO * HALO * XP;  // [COUT][NPIX + 8]
-    const int n = blockIdx.z, y0 = blockIdx.y * TILE, x0 = blockIdx.x * TILE;
-    const long long blk = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    load_halo<CIN>(xs, x, n, h, w, y0, x0);
-    for (int e = threadIdx.x; e < NPIX * COUT; e += NTHREADS) {
-        const int p = e / COUT, co = e % COUT;
-        const long long pix = ((long long)n * h + y0 + p / TILE) * w + x0 + p % TILE;
-        dzt[co * DP + p] = dz[pix * COUT + co];
-    }
-    __syncthreads();
-    if (threadIdx.x < COUT) {
-        float s = 0.f;
-        for (int p = 0; p < NPIX; ++p) s += __bfloat162float(dzt[threadIdx.x * DP + p]);
-        pdb[blk * COUT + threadIdx.x] = s;
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tid = threadIdx.x, lane = tid & 31, tap = tid >> 5;
+    const int ky = tap / 3, kx = tap % 3;
+    const int tx = w / TILE, timg = tx * (h / TILE);
+    auto load = [&](int tile, int st) {
+        __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smem + st * wgrad_stage<CIN, COUT>());
+        __nv_bfloat16* ds = xs + HALO * HALO * XP;
+        const int img = tile / timg, r = tile % timg;
+        const int y0 = (r / tx) * TILE, x0 = (r % tx) * TILE;
+        const __nv_bfloat16* xi = x + (long long)img * h * w * CIN;
+        const __nv_bfloat16* di = dz + (long long)img * h * w * COUT;
+        for (int e = tid; e < HALO * HALO * XC; e += WTHREADS) {
+            const int pix = e / XC, ck = e % XC;
+            const int gy = y0 + pix / HALO - 1, gx = x0 + pix % HALO - 1;
+            const bool in = gy >= 0 && gy < h && gx >= 0 && gx < w;
+            cp_async16(xs + pix * XP + ck * 8, in ? xi + ((long long)gy * w + gx) * CIN + ck * 8 : xi, in);
+        }
+        for (int e = tid; e < NPIX * DC; e += WTHREADS) {
+            const int pix = e / DC, ck = e % DC;
+            const __nv_bfloat16* src = di + ((long long)(y0 + pix / TILE) * w + x0 + pix % TILE) * COUT + ck * 8;
+            if (dz16) cp_async16(ds + pix * DP + ck * 8, src, true);
+            else  // dz does not start on 16 bytes
+                for (int k = 0; k < 8; ++k) ds[pix * DP + ck * 8 + k] = src[k];
+        }
+    };
+    // ldmatrix row of this lane: matrix lane / 8, row lane % 8
+    const int mr = lane & 7, mi = lane >> 3;
     const int g = lane >> 2, t = lane & 3;
-    float acc[TPW][4];
+    int st = 0;
+    if ((int)blockIdx.x < ntiles) load(blockIdx.x, 0);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, st ^= 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();  // the tile landed; every warp is done with the other stage
+        if (tile + (int)gridDim.x < ntiles) load(tile + gridDim.x, st ^ 1);
+        const __nv_bfloat16* xs = reinterpret_cast<const __nv_bfloat16*>(smem + st * wgrad_stage<CIN, COUT>());
+        const __nv_bfloat16* ds = xs + HALO * HALO * XP;
+        if (tap == 9) {  // the tenth warp: db's share of the tile, pixel by pixel
+            const int co = lane % COUT;
+            float sum = 0.f;
+#pragma unroll 32
+            for (int p = 0; p < NPIX; ++p) sum += __bfloat162float(ds[p * DP + co]);
+            if (lane < COUT) pdb[(long long)tile * COUT + co] = sum;
+            continue;
+        }
+        float acc[MT][2 * NT][4];
 #pragma unroll
-    for (int i = 0; i < TPW; ++i)
+        for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[i][k] = 0.f;
-#pragma unroll 1
-    for (int k0 = 0; k0 < NPIX; k0 += 16) {
-        // pixels k0+2t, k0+2t+1 (b0) and k0+2t+8, +9 (b1): all in tile row k0/16
-        const int prow = k0 / TILE;
+            for (int j = 0; j < 2 * NT; ++j)
 #pragma unroll
-        for (int i = 0; i < TPW; ++i) {
-            const int tile = warp + 8 * i;
-            if (tile >= TILES) break;
-            const int mt = tile / NT, nt = tile % NT;
-            const int co = mt * 16 + g;
-            const __nv_bfloat16* ap = dzt + co * DP + k0 + 2 * t;
-            const uint32_t a[4] = {ld32(ap), ld32(ap + 8 * DP), ld32(ap + 8), ld32(ap + 8 * DP + 8)};
-            const int tap = (nt * 8) / CIN, ci = (nt * 8) % CIN + g;
-            const int ky = tap / 3, kx = tap % 3;
-            const __nv_bfloat16* xr = xs + ((prow + ky) * HALO + kx) * XP + ci;
-            const int c0 = 2 * t;  // tile column of the first pixel of b0
-            uint32_t b[2];
-            b[0] = pack2(xr[(c0)*XP], xr[(c0 + 1) * XP]);
-            b[1] = pack2(xr[(c0 + 8) * XP], xr[(c0 + 9) * XP]);
-            mma_bf16(acc[i], a, b);
+                for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
+        // A (co x pixel): matrices (k 0-7, m 0-7), (k 0-7, m 8-15), (k 8-15, m 0-7), (k 8-15, m 8-15)
+        const uint32_t a0 = clawb200::smem_u32(ds + ((mi >> 1) * 8 + mr) * DP + (mi & 1) * 8);
+        // B (pixel x ci): matrices (k 0-7, n 0-7), (k 8-15, n 0-7), (k 0-7, n 8-15), (k 8-15, n 8-15)
+        const uint32_t b0 = clawb200::smem_u32(xs + (ky * HALO + kx + (mi & 1) * 8 + mr) * XP + (mi >> 1) * 8);
+#pragma unroll 4
+        for (int row = 0; row < TILE; ++row) {  // 16 pixels: one row of the tile
+            uint32_t a[MT][4], b[NT][4];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) ldsm_x4_t(a[i], a0 + (row * TILE * DP + i * 16) * 2);
+#pragma unroll
+            for (int j = 0; j < NT; ++j) ldsm_x4_t(b[j], b0 + (row * HALO * XP + j * 16) * 2);
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    mma_bf16(acc[i][2 * j], a[i], b[j]);
+                    mma_bf16(acc[i][2 * j + 1], a[i], b[j] + 2);
+                }
+        }
+        float* out = partial + (long long)tile * (COUT * 9 * CIN) + tap * CIN;
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < 2 * NT; ++j) {
+                const int c = j * 8 + 2 * t, r0 = i * 16 + g;
+                out[r0 * 9 * CIN + c] = acc[i][j][0];
+                out[r0 * 9 * CIN + c + 1] = acc[i][j][1];
+                out[(r0 + 8) * 9 * CIN + c] = acc[i][j][2];
+                out[(r0 + 8) * 9 * CIN + c + 1] = acc[i][j][3];
+            }
+    }
+}
+
+// dw[j] = sum over tiles of partial[tile][j] and db[c] of pdb[tile][c], tile
+// after tile; the last block takes db.  A column's additions are one chain, so
+// its loads must not wait for it: they go through shared memory by cp.async,
+// 64 tiles a stage, two stages ahead of the sum.
+constexpr int RT_ROWS = 64, RT_STAGES = 3;
+__global__ void __launch_bounds__(64) reduce_tiles(const float* __restrict__ partial, float* __restrict__ dw,
+                                                   const float* __restrict__ pdb, float* __restrict__ db,
+                                                   long long count, int len, int cout) {
+    __shared__ float sh[RT_STAGES][RT_ROWS][64];
+    const bool bias = blockIdx.x == gridDim.x - 1;
+    const int j = bias ? threadIdx.x : blockIdx.x * 64 + threadIdx.x;
+    const int n = bias ? cout : len;
+    if (j >= n) return;  // (a thread reads only what it copied itself)
+    const float* src = (bias ? pdb : partial) + j;
+    auto load = [&](long long chunk) {
+        const long long b0 = chunk * RT_ROWS;
+        const int rows = (int)min((long long)RT_ROWS, count - b0);
+        float* dst = &sh[chunk % RT_STAGES][0][threadIdx.x];
+        for (int k = 0; k < rows; ++k)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(clawb200::smem_u32(dst + k * 64)),
+                         "l"(src + (b0 + k) * n)
+                         : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(0);
+    load(1);  // (empty past the last tile, like the ones below)
+    float v = 0.f;
+    for (long long chunk = 0; chunk * RT_ROWS < count; ++chunk) {
+        load(chunk + 2);
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+        const int rows = (int)min((long long)RT_ROWS, count - chunk * RT_ROWS);
+        const float* p = &sh[chunk % RT_STAGES][0][threadIdx.x];
+        if (rows == RT_ROWS) {
+#pragma unroll 16
+            for (int k = 0; k < RT_ROWS; ++k) v += p[k * 64];
+        } else {
+            for (int k = 0; k < rows; ++k) v += p[k * 64];
         }
     }
-    float* out = partial + blk * (long long)(COUT * 9 * CIN);
-#pragma unroll
-    for (int i = 0; i < TPW; ++i) {
-        const int tile = warp + 8 * i;
-        if (tile >= TILES) break;
-        const int mt = tile / NT, nt = tile % NT;
-        const int col = nt * 8 + 2 * t;
-        const int r0 = mt * 16 + g, r1 = r0 + 8;
-        out[r0 * 9 * CIN + col] = acc[i][0];
-        out[r0 * 9 * CIN + col + 1] = acc[i][1];
-        out[r1 * 9 * CIN + col] = acc[i][2];
-        out[r1 * 9 * CIN + col + 1] = acc[i][3];
-    }
-}
-
-template <int CIN, int COUT>
-constexpr int wgrad_smem() {
-    return HALO * HALO * (CIN + 8) * 2 + COUT * (NPIX + 8) * 2;
-}
-
-// sum over tiles: dst[j] = sum_b src[b][j]
-__global__ void reduce_tiles(const float* __restrict__ src, float* __restrict__ dst, long long nblk,
-                             int len) {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < len; j += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (long long b = 0; b < nblk; ++b) s += src[b * len + j];
-        dst[j] = s;
-    }
+    (bias ? db : dw)[j] = v;
 }
 
 // Wt[ci][tap][co] = W[co][8 - tap][ci]: the data gradient's weights
@@ -477,29 +566,43 @@ __global__ void gelu_backward(const __nv_bfloat16* __restrict__ dy, const float*
 
 // MSE over the first nc of cp channels: dy = 2 (pred - target) / count,
 // loss accumulated in FP64 (one atomic per block)
-__global__ void mse_grad(const float* __restrict__ pred, const float* __restrict__ target,
-                         __nv_bfloat16* __restrict__ dy, double* __restrict__ loss, long long npix,
-                         int cp, int nc, float inv_count, float delta) {
+// A thread per pixel: nc channels of arithmetic, then the pixel's cp BF16 values
+// in 16-byte stores (16 x 64^2: 10.7 -> 3 us against a thread per value with a
+// 64-bit division each).
+__global__ void __launch_bounds__(NTHREADS) mse_grad(const float* __restrict__ pred,
+                                                     const float* __restrict__ target,
+                                                     __nv_bfloat16* __restrict__ dy, double* __restrict__ loss,
+                                                     long long npix, int cp, int nc, float inv_count,
+                                                     float delta) {
     __shared__ double red[NTHREADS / 32];
     double acc = 0.0;
-    const long long n = npix * cp;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-         e += (long long)gridDim.x * blockDim.x) {
-        const long long p = e / cp;
-        const int c = (int)(e % cp);
-        float g = 0.f;
+    auto grad = [&](long long p, int c) -> __nv_bfloat16 {
         const float tg = c < nc ? target[p * nc + c] : 0.f;
-        if (c < nc && tg == tg) {  // a NaN target masks the pixel out
-            const float d = pred[e] - tg;
-            if (delta > 0.f && fabsf(d) > delta) {  // Huber: linear beyond delta
-                acc += 2.0 * (double)delta * (double)fabsf(d) - (double)delta * (double)delta;
-                g = 2.f * copysignf(delta, d) * inv_count;
-            } else {
-                acc += (double)d * (double)d;
-                g = 2.f * d * inv_count;
-            }
+        if (c >= nc || tg != tg) return __float2bfloat16_rn(0.f);  // a NaN target masks the value out
+        const float d = pred[p * cp + c] - tg;
+        if (delta > 0.f && fabsf(d) > delta) {  // Huber: linear beyond delta
+            acc += 2.0 * (double)delta * (double)fabsf(d) - (double)delta * (double)delta;
+            return __float2bfloat16_rn(2.f * copysignf(delta, d) * inv_count);
         }
-        dy[e] = __float2bfloat16_rn(g);
+        acc += (double)d * (double)d;
+        return __float2bfloat16_rn(2.f * d * inv_count);
+    };
+    const bool wide = cp % 8 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
+    for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npix;
+         p += (long long)gridDim.x * blockDim.x) {
+        if (wide) {
+            for (int c = 0; c < cp; c += 8) {
+                uint32_t v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const __nv_bfloat16 lo = grad(p, c + 2 * k);
+                    v[k] = pack2(lo, grad(p, c + 2 * k + 1));
+                }
+                *reinterpret_cast<uint4*>(dy + p * cp + c) = make_uint4(v[0], v[1], v[2], v[3]);
+            }
+        } else {
+            for (int c = 0; c < cp; ++c) dy[p * cp + c] = grad(p, c);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -511,10 +614,24 @@ __global__ void mse_grad(const float* __restrict__ pred, const float* __restrict
     }
 }
 
-__global__ void adam_step(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                          float* __restrict__ v, __nv_bfloat16* __restrict__ w16, long long n,
-                          float lr, float b1, float b2, float eps, float c1, float c2) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+// Adam on up to ADAM_MAX tensors, tensor blockIdx.y (the network's ten tensors
+// in one launch instead of ten of 4 us).
+constexpr int ADAM_MAX = 16;
+struct AdamTensors {
+    float* w[ADAM_MAX];
+    const float* g[ADAM_MAX];
+    float* m[ADAM_MAX];
+    float* v[ADAM_MAX];
+    __nv_bfloat16* w16[ADAM_MAX];
+    long long n[ADAM_MAX];
+};
+__global__ void adam_step(const __grid_constant__ AdamTensors T, float lr, float b1, float b2, float eps,
+                          float c1, float c2) {
+    const int k = blockIdx.y;
+    float *w = T.w[k], *m = T.m[k], *v = T.v[k];
+    const float* g = T.g[k];
+    __nv_bfloat16* w16 = T.w16[k];
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < T.n[k];
          e += (long long)gridDim.x * blockDim.x) {
         const float ge = g[e];
         const float me = b1 * m[e] + (1.f - b1) * ge;
@@ -692,11 +809,11 @@ int halo_map(CUtensorMap* map, const void* x, int n, int h, int w, int c) {
     return r == CUDA_SUCCESS ? 0 : NN_E_CUDA;
 }
 
-template <int CIN, int COUT, int ACT, bool OUTF32, bool SAVEZ>
+template <int CIN, int COUT, int ACT, bool OUTF32, bool SAVEZ, bool DGRAD = false>
 int launch_fwd(const void* x, const void* w, const float* b, void* y, float* z, int n, int h,
-               int wd, cudaStream_t s) {
+               int wd, cudaStream_t s, const float* zin = nullptr) {
     constexpr int SM = tcp::smem_bytes<CIN, COUT>();
-    auto k = conv3x3_fwd_tcp<CIN, COUT, ACT, OUTF32, SAVEZ>;
+    auto k = conv3x3_fwd_tcp<CIN, COUT, ACT, OUTF32, SAVEZ, DGRAD>;
     // One persistent CTA per SM (the driver's limit for a TMEM-allocating
     // kernel).  The function attributes and the resident CTA count are set up
     // once per device and instantiation (0 = not yet); a launch that fails
@@ -743,9 +860,9 @@ int launch_fwd(const void* x, const void* w, const float* b, void* y, float* z, 
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k, xb, wb, b, y, z, n, h, wd, map);
+        e = cudaLaunchKernelEx(&cfg, k, xb, wb, b, y, z, zin, n, h, wd, map);
 #else
-        k<<<grid, tcp::NTH, SM, s>>>(xb, wb, b, y, z, n, h, wd, map);
+        k<<<grid, tcp::NTH, SM, s>>>(xb, wb, b, y, z, zin, n, h, wd, map);
         e = cudaGetLastError();
 #endif
         if (e == cudaSuccess) return 0;
@@ -756,15 +873,25 @@ int launch_fwd(const void* x, const void* w, const float* b, void* y, float* z, 
 }
 
 template <int CIN, int COUT>
-int launch_wgrad(const void* x, const void* dz, float* partial, float* pdb, int n, int h, int wd,
-                 cudaStream_t s) {
-    constexpr int SM = wgrad_smem<CIN, COUT>();
+int launch_wgrad(const void* x, const void* dz, float* partial, float* pdb, float* dw, float* db, int n, int h,
+                 int wd, cudaStream_t s) {
+    constexpr int SM = 2 * wgrad_stage<CIN, COUT>();
     auto k = conv3x3_wgrad<CIN, COUT>;
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SM) != cudaSuccess)
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SM) != cudaSuccess)
         return NN_E_CUDA;
-    k<<<dim3(wd / TILE, h / TILE, n), NTHREADS, SM, s>>>(static_cast<const __nv_bfloat16*>(x),
-                                                          static_cast<const __nv_bfloat16*>(dz),
-                                                          partial, pdb, h, wd);
+    const long long tiles = (long long)n * (h / TILE) * (wd / TILE);
+    if (tiles > 0x7fffffffLL) return NN_E_UNSUPPORTED;
+    // equal shares of tiles, two CTAs per SM (93 KB of shared memory each)
+    const long long per = (tiles + 2 * nsm - 1) / (2 * nsm);
+    const int grid = (int)((tiles + per - 1) / per);
+    k<<<grid, WTHREADS, SM, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(dz),
+                                 partial, pdb, h, wd, (int)tiles,
+                                 (reinterpret_cast<uintptr_t>(dz) & 15u) == 0);
+    constexpr int len = COUT * 9 * CIN;
+    reduce_tiles<<<len / 64 + 1, 64, 0, s>>>(partial, dw, pdb, db, tiles, len, COUT);
     return cudaGetLastError() == cudaSuccess ? 0 : NN_E_CUDA;
 }
 
@@ -799,17 +926,23 @@ int nn_conv3x3_wgrad(const void* x, const void* dz, float* partial, float* pdb, 
                      float* db, int n, int h, int wd, int cin, int cout, void* stream) {
     if (!x || !dz || !partial || !pdb || !dw || !db || !shape_ok(n, h, wd)) return NN_E_INVALID;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    int rc;
-    if (cin == 16 && cout == 32) rc = launch_wgrad<16, 32>(x, dz, partial, pdb, n, h, wd, s);
-    else if (cin == 32 && cout == 32) rc = launch_wgrad<32, 32>(x, dz, partial, pdb, n, h, wd, s);
-    else if (cin == 32 && cout == 16) rc = launch_wgrad<32, 16>(x, dz, partial, pdb, n, h, wd, s);
-    else return NN_E_UNSUPPORTED;
-    if (rc) return rc;
-    const long long nblk = (long long)n * (h / TILE) * (wd / TILE);
-    const int len = cout * 9 * cin;
-    reduce_tiles<<<(len + 255) / 256, 256, 0, s>>>(partial, dw, nblk, len);
-    reduce_tiles<<<1, 256, 0, s>>>(pdb, db, nblk, cout);
-    return cudaGetLastError() == cudaSuccess ? 0 : NN_E_CUDA;
+    if (cin == 16 && cout == 32) return launch_wgrad<16, 32>(x, dz, partial, pdb, dw, db, n, h, wd, s);
+    if (cin == 32 && cout == 32) return launch_wgrad<32, 32>(x, dz, partial, pdb, dw, db, n, h, wd, s);
+    if (cin == 32 && cout == 16) return launch_wgrad<32, 16>(x, dz, partial, pdb, dw, db, n, h, wd, s);
+    return NN_E_UNSUPPORTED;
+}
+
+int nn_conv3x3_dgrad(const void* dz, const void* w, const float* z, void* dx, int n, int h, int wd, int cin,
+                     int cout, void* stream) {
+    if (!dz || !w || !dx || !shape_ok(n, h, wd)) return NN_E_INVALID;
+    if ((reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(z)) & 15u) return NN_E_INVALID;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // a convolution from cout to cin channels
+    if (cin == 32 && cout == 32)
+        return launch_fwd<32, 32, 0, false, false, true>(dz, w, nullptr, dx, nullptr, n, h, wd, s, z);
+    if (cin == 32 && cout == 16)
+        return launch_fwd<16, 32, 0, false, false, true>(dz, w, nullptr, dx, nullptr, n, h, wd, s, z);
+    return NN_E_UNSUPPORTED;
 }
 
 int nn_device_error(int clear) {
@@ -841,19 +974,37 @@ int nn_mse_grad(const float* pred, const float* target, void* dy, double* loss, 
                 int cp, int nc, float delta, void* stream) {
     if (!pred || !target || !dy || !loss || npix <= 0 || nc > cp || delta < 0.f) return NN_E_INVALID;
     const float inv = 1.0f / (float)(npix * nc);
-    mse_grad<<<grid_for(npix * cp), NTHREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+    mse_grad<<<grid_for(npix), NTHREADS, 0, static_cast<cudaStream_t>(stream)>>>(
         pred, target, static_cast<__nv_bfloat16*>(dy), loss, npix, cp, nc, inv, delta);
+    return cudaGetLastError() == cudaSuccess ? 0 : NN_E_CUDA;
+}
+
+int nn_adam_multi(int count, float* const* w, const float* const* g, float* const* m, float* const* v,
+                  void* const* w16, const long long* n, float lr, float b1, float b2, float eps, int step,
+                  void* stream) {
+    if (count < 1 || count > ADAM_MAX || !w || !g || !m || !v || !w16 || !n || step < 1) return NN_E_INVALID;
+    AdamTensors T = {};
+    long long most = 0;
+    for (int k = 0; k < count; ++k) {
+        if (!w[k] || !g[k] || !m[k] || !v[k] || n[k] < 0) return NN_E_INVALID;
+        T.w[k] = w[k];
+        T.g[k] = g[k];
+        T.m[k] = m[k];
+        T.v[k] = v[k];
+        T.w16[k] = static_cast<__nv_bfloat16*>(w16[k]);
+        T.n[k] = n[k];
+        most = std::max(most, n[k]);
+    }
+    float c1 = 1.f, c2 = 1.f;
+    for (int k = 0; k < step && k < 100000; ++k) { c1 *= b1; c2 *= b2; }
+    adam_step<<<dim3(grid_for(most), count), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        T, lr, b1, b2, eps, 1.f - c1, 1.f - c2);
     return cudaGetLastError() == cudaSuccess ? 0 : NN_E_CUDA;
 }
 
 int nn_adam(float* w, const float* g, float* m, float* v, void* w16, long long n, float lr,
             float b1, float b2, float eps, int step, void* stream) {
-    if (!w || !g || !m || !v || n < 0 || step < 1) return NN_E_INVALID;
-    float c1 = 1.f, c2 = 1.f;
-    for (int k = 0; k < step && k < 100000; ++k) { c1 *= b1; c2 *= b2; }
-    adam_step<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, g, m, v, static_cast<__nv_bfloat16*>(w16), n, lr, b1, b2, eps, 1.f - c1, 1.f - c2);
-    return cudaGetLastError() == cudaSuccess ? 0 : NN_E_CUDA;
+    return nn_adam_multi(1, &w, &g, &m, &v, &w16, &n, lr, b1, b2, eps, step, stream);
 }
 
 int nn_block_average(const double* fine, long long ldf, long long fsf, double* coarse, long long ldc,

@@ -32,6 +32,14 @@ int nn_conv3x3_forward(const void* x, const void* w, const float* b, void* y, fl
  * partial / pdb: scratch of n*(h/16)*(wd/16) blocks x (cout*9*cin) / cout floats. */
 int nn_conv3x3_wgrad(const void* x, const void* dz, float* partial, float* pdb, float* dw,
                      float* db, int n, int h, int wd, int cin, int cout, void* stream);
+/* The data gradient of a layer with weights w [cout][9][cin] (BF16, as the
+ * forward pass takes them): dx = the adjoint convolution of dz [n][h][w][cout],
+ * BF16 [n][h][w][cin], times GELU'(z) when z (FP32 pre-activation of the layer
+ * below, [n][h][w][cin]) is given -- nn_flip_weights, nn_conv3x3_forward and
+ * nn_gelu_backward in one launch, the same roundings.  (cin, cout): (32,32),
+ * (32,16). */
+int nn_conv3x3_dgrad(const void* dz, const void* w, const float* z, void* dx, int n, int h, int wd,
+                     int cin, int cout, void* stream);
 /* Device-side error flags of these kernels (bit 0: a wait on the tensor-core
  * accumulator gave up, and that launch left its output unwritten); clear != 0
  * resets them.  Synchronises with the device. */
@@ -50,6 +58,11 @@ int nn_mse_grad(const float* pred, const float* target, void* dy, double* loss, 
 /* One Adam step on FP32 weights (step >= 1); w16 (optional) receives the BF16 copy. */
 int nn_adam(float* w, const float* g, float* m, float* v, void* w16, long long n, float lr,
             float b1, float b2, float eps, int step, void* stream);
+
+/* The same on count (1..16) tensors in one launch; w16[k] may be NULL. */
+int nn_adam_multi(int count, float* const* w, const float* const* g, float* const* m, float* const* v,
+                  void* const* w16, const long long* n, float lr, float b1, float b2, float eps, int step,
+                  void* stream);
 
 /* Solver glue on FP64 SoA fields [meqn][my][ld] (field pitch fs):
  * coarse = r x r block average of fine. */
