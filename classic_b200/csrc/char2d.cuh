@@ -187,11 +187,20 @@ step2_char_kernel(const __grid_constant__ CharArgs<real> A) {
     constexpr int W = R::W;
     constexpr unsigned FULL = 0xffffffffu;
     ClawCtl* ctl = A.ctl;
-    __shared__ double red[WARPS2D];
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* ring = smem + warp * R::WARP_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WARPS2D * R::WARP_BYTES) + warp * RING;
+    if (lane == 0) {
+        for (int sl = 0; sl < RING; ++sl) mbar_init(&bars[sl], 1);
+        fence_barrier_init();
+    }
+    __syncwarp();
     grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dtd = *(volatile double*)&ctl->dt;
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dtd = hd.dt;
     const double dtdx_d = dtd / A.dx, dtdy_d = dtd / A.dy;
     const real dtdx = (real)dtdx_d, dtdy = (real)dtdy_d;
     const real* __restrict__ qold = A.q[cur];
@@ -219,26 +228,15 @@ step2_char_kernel(const __grid_constant__ CharArgs<real> A) {
     const real cZh = real(0.5) * c;                                  // cZ over 2Z
     const real dtdx2 = real(0.5) * dtdx, dtdy2 = real(0.5) * dtdy;  // dt/d on Fp' differences
 
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char* ring = smem + warp * R::WARP_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WARPS2D * R::WARP_BYTES) + warp * RING;
-    if (lane == 0) {
-        for (int sl = 0; sl < RING; ++sl) mbar_init(&bars[sl], 1);
-        fence_barrier_init();
-    }
-    __syncwarp();
     const int mx = A.mx, my = A.my;
-    const unsigned long long wait_ns = ctl_wait_ns(ctl);
+    const unsigned long long wait_ns = hd.wait_ns;
     bool failed = false;
     uint32_t seq_base = 0;
-    bool any_work = false;
 
     const int gw = blockIdx.x * WARPS2D + warp;
     const int items = A.nstrips * A.nblocks;
 
     for (int item = gw; gw < A.nwarps && item < items && !failed; item += A.nwarps) {
-        any_work = true;
         const int strip = item % A.nstrips;
         const int r0 = (item / A.nstrips) * A.brows;
         const int nr = min(A.brows, my - r0);
@@ -247,7 +245,7 @@ step2_char_kernel(const __grid_constant__ CharArgs<real> A) {
         const int x0 = b - R::XQ;
         const int rfirst = r0 - 2, rlast = r0 + nr + 1;
         const int nrows = rlast - rfirst + 1;
-        const int skip1 = strip == 0 ? *(volatile const int*)&ctl->skip_row : 0;  // test hook
+        const int skip1 = strip == 0 ? hd.skip_row : 0;  // test hook
 
         auto seq_of = [&](int r) -> uint32_t { return seq_base + (uint32_t)(r - rfirst); };
         auto issue = [&](int r) {
@@ -533,8 +531,8 @@ step2_char_kernel(const __grid_constant__ CharArgs<real> A) {
     }
     // Courant number as flux2 forms it (dt/dx * c over x-interfaces, dt/dy * c
     // over y-interfaces; the speeds are constant)
-    const double cfl = any_work ? fmax(dtdx_d * (double)c, dtdy_d * (double)c) : 0.0;
-    cta_cfl_and_control(ctl, cfl, red);
+    const double cfl = fmax(dtdx_d * (double)c, dtdy_d * (double)c);
+    cta_count_and_control(ctl, failed, [&](const CtlIn&) { return cfl > 0.0 || cfl != cfl ? cfl : 0.0; });
 }
 
 }  // namespace clawb200

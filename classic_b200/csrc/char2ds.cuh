@@ -104,11 +104,20 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
     constexpr int XQS = STRANG ? (sizeof(real) == 8 ? 6 : 8) : R::XQ;
     constexpr int LEFT = STRANG ? 4 : 2;
     ClawCtl* ctl = A.ctl;
-    __shared__ double red[3 * WARPS2D];
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* ring = smem + warp * R::WARP_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WARPS2D * R::WARP_BYTES) + warp * RING;
+    if (lane == 0) {
+        for (int sl = 0; sl < RING; ++sl) mbar_init(&bars[sl], 1);
+        fence_barrier_init();
+    }
+    __syncwarp();
     grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dtd = *(volatile double*)&ctl->dt;
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dtd = hd.dt;
     // the sweeps' lengths as dimsp2 takes them (src/2d/dimsp2.f:52-62)
     const double dta = STRANG ? dtd / 2.0 : dtd;
     const double dtdx_a_d = dta / A.dx, dtdy_d = dtd / A.dy, dtdx_c_d = (dtd / 2.0) / A.dx;
@@ -124,25 +133,14 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
     real* __restrict__ qnew = A.q[cur ^ 1];
     const CUtensorMap* tmq = &A.tmq[cur];
 
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char* ring = smem + warp * R::WARP_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WARPS2D * R::WARP_BYTES) + warp * RING;
-    if (lane == 0) {
-        for (int sl = 0; sl < RING; ++sl) mbar_init(&bars[sl], 1);
-        fence_barrier_init();
-    }
-    __syncwarp();
     const int mx = A.mx, my = A.my;
-    const unsigned long long wait_ns = ctl_wait_ns(ctl);
+    const unsigned long long wait_ns = hd.wait_ns;
     bool failed = false;
     uint32_t seq_base = 0;
-    bool any_work = false;
     const int gw = blockIdx.x * WARPS2D + warp;
     const int items = A.nstrips * A.nblocks;
 
     for (int item = gw; gw < A.nwarps && item < items && !failed; item += A.nwarps) {
-        any_work = true;
         const int strip = item % A.nstrips;
         const int r0 = (item / A.nstrips) * A.brows;
         const int nr = min(A.brows, my - r0);
@@ -151,7 +149,7 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
         const int x0 = b - XQS;
         const int rfirst = r0 - 2, rlast = r0 + nr + 1;
         const int nrows = rlast - rfirst + 1;
-        const int skip1 = strip == 0 ? *(volatile const int*)&ctl->skip_row : 0;  // test hook
+        const int skip1 = strip == 0 ? hd.skip_row : 0;  // test hook
 
         auto seq_of = [&](int r) -> uint32_t { return seq_base + (uint32_t)(r - rfirst); };
         auto issue = [&](int r) {
@@ -339,9 +337,10 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
     // the sweeps' Courant numbers as step2ds forms them over every interface
     // (dt_sweep/dx c; the speeds are constant), combined as dimsp2 combines them
     const double cd = (double)c;
-    const double c3[3] = {any_work ? dtdx_a_d * cd : 0.0, any_work ? dtdy_d * cd : 0.0,
-                          any_work ? dtdx_c_d * cd : 0.0};
-    cta_split_cfl_and_control(ctl, c3, STRANG ? 3 : 2, red);
+    auto known = [&](double v) { return v > 0.0 || v != v ? v : 0.0; };
+    cta_count_and_control(ctl, failed, [&](const CtlIn& in) {
+        return split_cfl(in, STRANG ? 3 : 2, known(dtdx_a_d * cd), known(dtdy_d * cd), known(dtdx_c_d * cd));
+    });
 }
 
 }  // namespace clawb200

@@ -13,29 +13,30 @@ namespace clawb200 {
 // Every step kernel reads dt / cur at entry; the last CTA to finish a step
 // folds the CFL maximum and runs the accept/reject + next-dt logic here, so a
 // whole time loop runs without a host round trip per step.
-struct ClawCtl {
-    double t, told, dt, tstart, tend;
+struct alignas(128) ClawCtl {
+    // first line: read by every warp at a step's start (step_head: the first
+    // 32 bytes), written by the controller alone
+    double dt;
+    unsigned long long wait_ns;    // limit of a device-side wait (0: the 2 s default)
+    int done;
+    int cur;                       // index of the buffer holding the current q
+    int mode;                      // CTL_ADVANCE or CTL_SINGLE
+    int skip_row;                  // test hook: 1 + the row whose copy strip 0 skips (0: none)
+    double t, told, tstart, tend;
     double dt_max, cfl_max, cfl_desired;
     double cflmax_seen, dtmin, dtmax, cfl_last;
-    unsigned long long cfl_bits;   // atomicMax target (bit pattern of a double >= 0)
-    unsigned int ctas_done;        // last-CTA counter, reset by the last CTA
-    int cur;                       // index of the buffer holding the current q
-    int n, maxn, nrej;             // accepted steps, step limit, rejected steps
-    int done, info;
-    int mode;                      // CTL_ADVANCE or CTL_SINGLE
-    int dt_variable;
-    int err;                       // device error flags (CTL_ERR_*)
-    int skip_row;                  // test hook: 1 + the row whose copy strip 0 skips (0: none)
+    int info, dt_variable;
+    // second line: what the CTAs of a step publish
+    alignas(128) unsigned long long cfl_bits;  // atomicMax target (bit pattern of a double >= 0)
     unsigned long long cfl_sweep[2];  // dimensional splitting: Courant maxima of the
                                       // y-sweep and of Strang's last x-sweep
-    unsigned long long wait_ns;    // limit of a device-side wait (0: the 2 s default)
+    unsigned int ctas_done;        // last-CTA counter, reset by the last CTA
+    int err;                       // device error flags (CTL_ERR_*)
+    int n, maxn, nrej;             // accepted steps, step limit, rejected steps
 };
+static_assert(sizeof(ClawCtl) == 256, "two lines");
 
 constexpr unsigned long long WAIT_NS_DEFAULT = 2000000000ull;
-__device__ __forceinline__ unsigned long long ctl_wait_ns(const ClawCtl* c) {
-    const unsigned long long w = *(volatile const unsigned long long*)&c->wait_ns;
-    return w ? w : WAIT_NS_DEFAULT;
-}
 
 enum { CTL_ADVANCE = 0, CTL_SINGLE = 1 };
 
@@ -43,53 +44,95 @@ enum { CTL_ADVANCE = 0, CTL_SINGLE = 1 };
 enum { BC_USER = 0, BC_EXTRAP = 1, BC_PERIODIC = 2, BC_WALL = 3 };
 enum { CTL_ERR_TMA_TIMEOUT = 1, CTL_ERR_NAN_CFL = 2 };
 
+// What a step kernel reads of the control block at its start: two 16-byte loads
+// a warp, in flight together.  (Testing `done` before loading the rest took two
+// or three L2 round trips of 0.35 us, and the block's line serves every warp of
+// the grid, so its loads are few and its atomics lie elsewhere.)
+struct StepHead {
+    int done, cur, mode, skip_row;
+    double dt;
+    unsigned long long wait_ns;
+};
+__device__ __forceinline__ StepHead step_head(const ClawCtl* c) {
+    unsigned long long d, w;
+    StepHead h;
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(d), "=l"(w) : "l"(c) : "memory");
+    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(h.done), "=r"(h.cur), "=r"(h.mode), "=r"(h.skip_row)
+                 : "l"(&c->done)
+                 : "memory");
+    h.dt = __longlong_as_double((long long)d);
+    h.wait_ns = w ? w : WAIT_NS_DEFAULT;
+    return h;
+}
+
+// The controller's operands, loaded together by the last CTA beside the Courant
+// number.
+struct CtlIn {
+    double told, dt, tend, tstart, dt_max, cfl_max, cfl_desired, cflmax_seen, dtmin, dtmax;
+    int mode, dt_variable, cur, n, maxn, nrej;
+};
+__device__ __forceinline__ CtlIn ctl_in(const ClawCtl* c) {
+    const volatile ClawCtl* v = c;
+    return CtlIn{v->told, v->dt, v->tend, v->tstart, v->dt_max, v->cfl_max, v->cfl_desired, v->cflmax_seen,
+                 v->dtmin, v->dtmax, v->mode, v->dt_variable, v->cur, v->n, v->maxn, v->nrej};
+}
+
 // Controller step: identical decisions to claw2's main loop.  Runs in exactly
-// one thread after every CTA of the step has published its CFL maximum.
-__device__ __forceinline__ void ctl_finish_step(ClawCtl* c) {
-    const double cfl = __longlong_as_double((long long)atomicAdd(&c->cfl_bits, 0ull));
-    c->cfl_bits = 0ull;
+// one thread after every CTA of the step has published its Courant maximum
+// (cfl; its slot is the caller's to clear) and its error flag (err).  The next
+// launch sees the block when this grid is complete.
+__device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, double cfl, int err) {
     c->ctas_done = 0u;
     c->cfl_last = cfl;
-    if (c->err) {  // a device wait gave up: the step's output is incomplete
+    if (err) {  // a device wait gave up: the step's output is incomplete
         c->done = 1;
         return;
     }
-    if (c->mode == CTL_SINGLE) {
-        c->cur ^= 1;
+    if (s.mode == CTL_SINGLE) {
+        c->cur = s.cur ^ 1;
         return;
     }
     if (cfl != cfl) {  // NaN: stop instead of retrying forever
-        c->err |= CTL_ERR_NAN_CFL;
+        c->err = err | CTL_ERR_NAN_CFL;
         c->done = 1;
         return;
     }
-    c->t = c->told + c->dt;
-    if (cfl <= c->cfl_max) {
-        c->cflmax_seen = fmax(cfl, c->cflmax_seen);
-        c->cur ^= 1;
-        if (c->dt_variable) {
-            if (cfl == 0.0) c->dt = c->dt_max;
-            else c->dt = fmin(c->dt_max, c->dt * c->cfl_desired / cfl);
-            c->dtmin = fmin(c->dt, c->dtmin);
-            c->dtmax = fmax(c->dt, c->dtmax);
+    const double t = s.told + s.dt;
+    double dt = s.dt;
+    if (cfl <= s.cfl_max) {
+        c->t = t;
+        c->cflmax_seen = fmax(cfl, s.cflmax_seen);
+        c->cur = s.cur ^ 1;
+        if (s.dt_variable) {
+            if (cfl == 0.0) dt = s.dt_max;
+            else dt = fmin(s.dt_max, s.dt * s.cfl_desired / cfl);
+            c->dtmin = fmin(dt, s.dtmin);
+            c->dtmax = fmax(dt, s.dtmax);
         }
-        c->n += 1;
-        if (c->t >= c->tend || c->n >= c->maxn) {
+        c->n = s.n + 1;
+        if (t >= s.tend || s.n + 1 >= s.maxn) {
             c->done = 1;
         } else {
-            c->told = c->t;
-            if (c->told + c->dt > c->tend && c->tstart < c->tend) c->dt = c->tend - c->told;
+            c->told = t;
+            if (t + dt > s.tend && s.tstart < s.tend) dt = s.tend - t;
         }
+        c->dt = dt;
     } else {
-        c->t = c->told;
-        c->nrej += 1;
-        if (c->dt_variable) {
-            c->dt = fmin(c->dt_max, c->dt * c->cfl_desired / cfl);
+        c->t = s.told;
+        c->nrej = s.nrej + 1;
+        if (s.dt_variable) {
+            c->dt = fmin(s.dt_max, s.dt * s.cfl_desired / cfl);
         } else {
-            c->cflmax_seen = fmax(cfl, c->cflmax_seen);
+            c->cflmax_seen = fmax(cfl, s.cflmax_seen);
             c->done = 1;
         }
     }
+}
+
+// The step's folded Courant maximum, its slot cleared for the next step.
+__device__ __forceinline__ double take_cfl(unsigned long long* slot) {
+    return __longlong_as_double((long long)atomicExch(slot, 0ull));
 }
 
 // Publish one CTA's CFL maximum and, in the last CTA, run the controller.
@@ -108,8 +151,29 @@ __device__ __forceinline__ void cta_cfl_and_control(ClawCtl* ctl, double cfl, do
         const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
         if (prev == gridDim.x - 1) {
             __threadfence();
-            ctl_finish_step(ctl);
-            __threadfence();
+            const CtlIn in = ctl_in(ctl);
+            const int err = *(volatile int*)&ctl->err;
+            ctl_finish_step(ctl, in, take_cfl(&ctl->cfl_bits), err);
+        }
+    }
+}
+
+// The same for a step whose Courant number every CTA knows (constant speeds):
+// nothing is folded, so a CTA only counts itself in.  A fence there waits for
+// the CTA's last stores of q, at the end of every step; the count needs none
+// unless a device wait gave up, whose flag it then orders.  Contracted FP64, us
+// a step: 64^2 8.3 -> 6.4, 1024^2 18.4 -> 16.8, 4096^2 165.7 -> 160.6.
+template <class F>
+__device__ __forceinline__ void cta_count_and_control(ClawCtl* ctl, bool failed, F cfl_of) {
+    const int any = __syncthreads_or(failed);
+    if (threadIdx.x == 0) {
+        if (any) __threadfence();
+        unsigned prev;
+        asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(&ctl->ctas_done) : "memory");
+        if (prev == gridDim.x - 1) {
+            const CtlIn in = ctl_in(ctl);
+            const int err = *(volatile int*)&ctl->err;
+            ctl_finish_step(ctl, in, cfl_of(in), err);
         }
     }
 }

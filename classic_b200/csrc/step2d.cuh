@@ -191,12 +191,18 @@ struct StepConsts {
     const CUtensorMap* tmq;        // TMA map of qold
     int src;                       // source split of this launch (0 in claw_step / batches)
     double src_pre, src_post;      // source time steps before / after the step
+    unsigned long long wait_ns;    // limit of a device-side wait
+    int skip_row;                  // test hook (ClawCtl)
 };
 
 template <class S>
-__device__ __forceinline__ StepConsts<S> step_consts(const Step2Args<S>& A, int cur, double dtd) {
+__device__ __forceinline__ StepConsts<S> step_consts(const Step2Args<S>& A, const StepHead& hd) {
     using real = typename S::real;
+    const int cur = hd.cur;
+    const double dtd = hd.dt;
     StepConsts<S> k;
+    k.wait_ns = hd.wait_ns;
+    k.skip_row = hd.skip_row;
     k.dtdx = (real)(dtd / A.dx);
     k.dtdy = (real)(dtd / A.dy);
     k.dtdx_d = dtd / A.dx;
@@ -288,8 +294,8 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
 
     // wait limit; test hook: strip 0 skips the copy of one row (its wait then
     // runs out, nothing faults)
-    const unsigned long long wait_ns = ctl_wait_ns(ctl);
-    const int skip1 = strip == 0 ? *(volatile const int*)&ctl->skip_row : 0;
+    const unsigned long long wait_ns = K.wait_ns;
+    const int skip1 = strip == 0 ? K.skip_row : 0;
     auto seq_of = [&](int r) -> uint32_t { return seq_base + (uint32_t)(r - rfirst); };
     auto issue = [&](int r) {
         if (skip1 != 0 && r == skip1 - 1) return;
@@ -761,12 +767,7 @@ __global__ void __launch_bounds__(32 * WARPS2D, step2_minb<S>::value)
 step2_kernel(const __grid_constant__ Step2Args<S> A) {
     ClawCtl* ctl = A.ctl;
     __shared__ double red[WARPS2D];
-    grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dtd = *(volatile double*)&ctl->dt;
     using R = Ring2D<S>;
-
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* ring = smem + warp * R::WARP_BYTES;
@@ -776,6 +777,9 @@ step2_kernel(const __grid_constant__ Step2Args<S> A) {
         fence_barrier_init();
     }
     __syncwarp();
+    grid_dependency_sync();
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
 
     const int my = A.my;
     double cfl = 0.0;
@@ -785,9 +789,9 @@ step2_kernel(const __grid_constant__ Step2Args<S> A) {
     const long long gw = (long long)blockIdx.x * WARPS2D + warp;
     long long u0 = (gw < A.nwarps) ? gw * A.units / A.nwarps : 0;
     const long long u1 = (gw < A.nwarps) ? (gw + 1) * A.units / A.nwarps : 0;
-    StepConsts<S> K = step_consts(A, cur, dtd);
+    StepConsts<S> K = step_consts(A, hd);
     // claw2 wraps the source steps around step2; a single step (claw_step) is step2 alone
-    if (SRC && ctl->mode == CTL_ADVANCE) K.src = A.src_split;
+    if (SRC && hd.mode == CTL_ADVANCE) K.src = A.src_split;
 
     if (A.brows > 0) {
         const int items = A.nstrips * A.nblocks;
@@ -893,9 +897,7 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
         while (pre[k + 1] <= u0) ++k;
         const Step2Args<S>& A = B.inst[k];
         ClawCtl* ctl = B.ctls + k;
-        const int cur = *(volatile int*)&ctl->cur;
-        const double dtd = *(volatile double*)&ctl->dt;
-        const StepConsts<S> K = step_consts(A, cur, dtd);
+        const StepConsts<S> K = step_consts(A, step_head(ctl));
         const long long off = u0 - pre[k];
         const int my = A.my;
         const int strip = (int)(off / my), r0 = (int)(off % my);
@@ -913,9 +915,10 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
             const unsigned prev = atomicAdd(&ctl->ctas_done, (unsigned)nr);
             if (prev + (unsigned)nr == (unsigned)B.units[k]) {
                 __threadfence();
-                ctl_finish_step(ctl);
-                if (ctl->done) atomicSub(B.active, 1);
-                __threadfence();
+                const CtlIn in = ctl_in(ctl);
+                const int err = *(volatile int*)&ctl->err;
+                ctl_finish_step(ctl, in, take_cfl(&ctl->cfl_bits), err);
+                if (*(volatile int*)&ctl->done) atomicSub(B.active, 1);
             }
         }
         __syncwarp();

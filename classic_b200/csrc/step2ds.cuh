@@ -484,6 +484,16 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
     seq_base += (uint32_t)nrows;
 }
 
+// dimsp2's Courant number of nsw sweeps (src/2d/dimsp2.f:65-96).
+__device__ __forceinline__ double split_cfl(const CtlIn& in, int nsw, double ca, double cb, double cc) {
+    // a NaN in any sweep stays NaN (the controller stops on it)
+    auto nmax = [](double a, double b2) { return a != a ? a : (b2 != b2 ? b2 : fmax(a, b2)); };
+    if (ca > in.cfl_max) return ca;
+    if (nsw > 2 && cb > in.cfl_max) return cb;
+    const double cfl = nmax(ca, cb);
+    return nsw > 2 ? nmax(cfl, cc) : cfl;
+}
+
 // Fold the per-sweep Courant maxima of every CTA; the last CTA combines them
 // as dimsp2 does and runs the controller.
 __device__ __forceinline__ void cta_split_cfl_and_control(ClawCtl* ctl, const double* c3, int nsw,
@@ -507,26 +517,12 @@ __device__ __forceinline__ void cta_split_cfl_and_control(ClawCtl* ctl, const do
         const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
         if (prev == gridDim.x - 1) {
             __threadfence();
-            const double ca = __longlong_as_double((long long)atomicAdd(&ctl->cfl_bits, 0ull));
-            const double cb = __longlong_as_double((long long)atomicAdd(&ctl->cfl_sweep[0], 0ull));
-            const double cc = nsw > 2
-                                  ? __longlong_as_double((long long)atomicAdd(&ctl->cfl_sweep[1], 0ull))
-                                  : 0.0;
-            ctl->cfl_sweep[0] = 0ull;
-            ctl->cfl_sweep[1] = 0ull;
-            // src/2d/dimsp2.f:65-96
-            // a NaN in any sweep stays NaN (the controller stops on it)
-            auto nmax = [](double a, double b2) { return a != a ? a : (b2 != b2 ? b2 : fmax(a, b2)); };
-            double cfl;
-            if (ca > ctl->cfl_max) cfl = ca;
-            else if (nsw > 2 && cb > ctl->cfl_max) cfl = cb;
-            else {
-                cfl = nmax(ca, cb);
-                if (nsw > 2) cfl = nmax(cfl, cc);
-            }
-            ctl->cfl_bits = (unsigned long long)__double_as_longlong(cfl);
-            ctl_finish_step(ctl);
-            __threadfence();
+            const CtlIn in = ctl_in(ctl);
+            const int err = *(volatile int*)&ctl->err;
+            const double ca = take_cfl(&ctl->cfl_bits), cb = take_cfl(&ctl->cfl_sweep[0]);
+            const double cc = nsw > 2 ? take_cfl(&ctl->cfl_sweep[1]) : 0.0;
+            const double cfl = split_cfl(in, nsw, ca, cb, cc);
+            ctl_finish_step(ctl, in, cfl, err);
         }
     }
 }
@@ -540,11 +536,6 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
     using real = typename S::real;
     ClawCtl* ctl = A.ctl;
     __shared__ double red[3 * WARPS2D];
-    grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dtd = *(volatile double*)&ctl->dt;
-
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* ring = smem + warp * L::WARP_BYTES;
@@ -554,6 +545,12 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
         fence_barrier_init();
     }
     __syncwarp();
+    grid_dependency_sync();
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dtd = hd.dt;
+
 
     SplitConsts<S> K;
     const double dta = STRANG ? dtd / 2.0 : dtd;  // src/2d/dimsp2.f:52-62
@@ -567,7 +564,7 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
     K.qnew = A.q[cur ^ 1];
     K.tmq = &A.tmq[cur];
     // claw2 wraps the source steps around the split step; claw_step runs it alone
-    K.src = (SRC && ctl->mode == CTL_ADVANCE) ? A.src_split : 0;
+    K.src = (SRC && hd.mode == CTL_ADVANCE) ? A.src_split : 0;
     K.src_pre = dtd / 2.0;
     K.src_post = dtd;
 

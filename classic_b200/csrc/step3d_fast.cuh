@@ -114,10 +114,11 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     const Sweep3Args<real>& a = A.g;
     ClawCtl* ctl = a.ctl;
     grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dt = *(volatile double*)&ctl->dt;
     const double tbc = *(volatile double*)&ctl->told;
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dt = hd.dt;
     const real* __restrict__ qold = a.q[cur];
     real* __restrict__ qnew = a.q[cur ^ 1];
     const real* __restrict__ aux = a.aux;

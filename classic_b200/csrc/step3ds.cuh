@@ -150,9 +150,10 @@ __global__ void __launch_bounds__(32 * DS3_WARPS) split3_x_kernel(const Split3Ar
     __shared__ double red[DS3_WARPS];
     ClawCtl* ctl = a.ctl;
     grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dt = *(volatile double*)&ctl->dt;
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dt = hd.dt;
     const double tbc = *(volatile double*)&ctl->told;
     const real* __restrict__ q = a.q[cur];
     real* __restrict__ P = a.P;
@@ -230,9 +231,10 @@ __global__ void __launch_bounds__(32 * DS3_WARPS, 2) split3_yz_kernel(const Spli
     __shared__ double red[DS3_WARPS];
     ClawCtl* ctl = a.ctl;
     grid_dependency_sync();
-    if (*(volatile int*)&ctl->done) return;
-    const int cur = *(volatile int*)&ctl->cur;
-    const double dt = *(volatile double*)&ctl->dt;
+    const StepHead hd = step_head(ctl);
+    if (hd.done) return;
+    const int cur = hd.cur;
+    const double dt = hd.dt;
     const double tbc = *(volatile double*)&ctl->told;
     const real* __restrict__ q = a.q[cur];
     real* __restrict__ qn = a.qw[cur ^ 1];
@@ -370,20 +372,17 @@ __global__ void __launch_bounds__(32 * DS3_WARPS, 2) split3_yz_kernel(const Spli
         const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
         if (prev == gridDim.x - 1) {
             __threadfence();
-            const double cx = __longlong_as_double((long long)atomicAdd(&ctl->cfl_bits, 0ull));
-            const double cy = __longlong_as_double((long long)atomicAdd(&ctl->cfl_sweep[0], 0ull));
-            const double cz = __longlong_as_double((long long)atomicAdd(&ctl->cfl_sweep[1], 0ull));
-            ctl->cfl_sweep[0] = 0ull;
-            ctl->cfl_sweep[1] = 0ull;
+            const CtlIn in = ctl_in(ctl);
+            const int err = *(volatile int*)&ctl->err;
+            const double cx = take_cfl(&ctl->cfl_bits), cy = take_cfl(&ctl->cfl_sweep[0]),
+                         cz = take_cfl(&ctl->cfl_sweep[1]);
             // src/3d/dimsp3.f:55-84; a NaN in any sweep stays NaN
             auto nmax = [](double x, double y) { return x != x ? x : (y != y ? y : fmax(x, y)); };
             double c;
-            if (cx > ctl->cfl_max) c = cx;
-            else if (cy > ctl->cfl_max) c = cy;
+            if (cx > in.cfl_max) c = cx;
+            else if (cy > in.cfl_max) c = cy;
             else c = nmax(nmax(cx, cy), cz);
-            ctl->cfl_bits = (unsigned long long)__double_as_longlong(c);
-            ctl_finish_step(ctl);
-            __threadfence();
+            ctl_finish_step(ctl, in, c, err);
         }
     }
 }
