@@ -18,6 +18,7 @@
 #include "riemann.cuh"
 #include "step2d.cuh"
 #include "batch2d_runner.cuh"
+#include "fieldcopy.cuh"
 
 using namespace clawb200;
 
@@ -78,6 +79,8 @@ struct claw_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     long long launches = 0;
     int device = 0;
+    double* stage = nullptr;  // dense device copy of one instance's q (fieldcopy.cuh)
+    size_t stage_n = 0;
 
     // Frees everything the batch holds, so an error part-way through
     // claw_batch_create leaks nothing.
@@ -91,6 +94,7 @@ struct claw_batch {
                 if (gg.q[s]) cudaFree(gg.q[s]);
             if (gg.aux) cudaFree(gg.aux);
         }
+        if (stage) cudaFree(stage);
         if (ctl_d) cudaFree(ctl_d);
         if (ctl_h) cudaFreeHost(ctl_h);
         if (flags_d) cudaFree(flags_d);
@@ -173,7 +177,14 @@ int claw_batch_create(const claw_config* cfgs, int count, claw_batch** out) {
         }
         g.ctl = b->ctl_d + k;
     }
-    int rc = b->runner->prepare(b->g, cfgs, b->ctl_d, b->flags_d, b->flags_d + 1);
+    size_t largest = 0;
+    for (const Geometry& g : b->g) {
+        const size_t n = (size_t)g.meqn * g.mx * g.my;
+        if (n * sizeof(double) <= STAGE_BYTES) largest = std::max(largest, n);
+    }
+    int rc = make_stage(&b->stage, &b->stage_n, {largest}, false);
+    if (rc) return rc;
+    rc = b->runner->prepare(b->g, cfgs, b->ctl_d, b->flags_d, b->flags_d + 1);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(b->stream));
     *out = b.release();
@@ -188,17 +199,8 @@ int claw_batch_destroy(claw_batch* b) {
 static int batch_fields(claw_batch* b, int k, double* host, bool to_device) {
     const Geometry& g = b->g[k];
     const int cur = b->ctl_h[k].cur;
-    for (int m = 0; m < g.meqn; ++m) {
-        char* d = static_cast<char*>(g.q[cur]) + (size_t)m * g.fstride * 8;
-        double* hp = host + (size_t)m * g.mx * g.my;
-        if (to_device)
-            CUDA_TRY(cudaMemcpy2DAsync(d, g.ld * 8, hp, g.mx * 8, g.mx * 8, g.my,
-                                       cudaMemcpyHostToDevice, b->stream));
-        else
-            CUDA_TRY(cudaMemcpy2DAsync(hp, g.mx * 8, d, g.ld * 8, g.mx * 8, g.my,
-                                       cudaMemcpyDeviceToHost, b->stream));
-    }
-    return 0;
+    return copy_fields(static_cast<double*>(g.q[cur]), g.ld, g.fstride, host, g.meqn, g.mx, g.my, b->stage,
+                       b->stage_n, to_device, b->stream);
 }
 
 int claw_batch_set_q(claw_batch* b, int k, const double* q) {

@@ -15,6 +15,7 @@
 
 #include "../../include/claw_b200.h"
 #include "common.cuh"
+#include "fieldcopy.cuh"
 #include "host.h"
 #include "riemann.cuh"
 #include "step1d.cuh"
@@ -337,17 +338,6 @@ bool solver_shape(int id, SolverShape* sh) {
     }
 }
 
-__global__ void widen_to_double(const float* src, double* dst, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        dst[i] = (double)src[i];
-}
-__global__ void narrow_to_float(const double* src, float* dst, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x)
-        dst[i] = (float)src[i];
-}
-
 }  // namespace
 
 struct claw_handle {
@@ -356,7 +346,8 @@ struct claw_handle {
     int cur = 0;
     cudaStream_t stream = nullptr;
     ClawCtl* ctl_h = nullptr;  // pinned mirror
-    double* stage = nullptr;   // device staging (doubles) for FP32 conversion
+    double* stage = nullptr;   // dense device copy of a field block (fieldcopy.cuh)
+    size_t stage_n = 0;
     std::unique_ptr<Runner> runner;
     cudaGraphExec_t gexec = nullptr;
     int gsteps = 0;
@@ -396,6 +387,13 @@ const char* claw_last_error(void) { return g_err.c_str(); }
 const char* claw_build_info(void) {
     return "clawb200 sm_100a; fp64 path built with --fmad=false (reference operation order)";
 }
+
+// doubles in the caller's arrays
+static long long aux_rows(const Geometry& g) {
+    return (long long)(g.dim >= 2 ? g.my + 4 : 1) * (g.dim >= 3 ? g.mz + 4 : 1);
+}
+static size_t q_count(const Geometry& g) { return (size_t)g.meqn * g.mx * g.my * g.mz; }
+static size_t aux_count(const Geometry& g) { return g.maux * (size_t)(g.mx + 4) * aux_rows(g); }
 
 static int validate(const claw_config* c, SolverShape* sh) {
     if (!c) return fail(CLAW_E_INVALID, "null config");
@@ -497,10 +495,8 @@ int claw_create(const claw_config* cfg, claw_handle** out) {
     std::memset(h->ctl_h, 0, sizeof(ClawCtl));
     h->ctl_h->done = 1;
     CUDA_TRY(cudaMemcpyAsync(g.ctl, h->ctl_h, sizeof(ClawCtl), cudaMemcpyHostToDevice, h->stream));
-    if (g.es == 4) {
-        const size_t n = std::max((size_t)g.fstride * g.meqn, (size_t)g.afstride * g.maux);
-        CUDA_TRY(cudaMalloc(&h->stage, n * sizeof(double)));
-    }
+    rc = make_stage(&h->stage, &h->stage_n, {q_count(g), aux_count(g)}, g.es == 4);
+    if (rc) return rc;
     h->runner = g.es == 8 ? make_runner<double>(*cfg) : make_runner<float>(*cfg);
     if (!h->runner) return fail(CLAW_E_UNSUPPORTED, "no kernel for solver %d", cfg->solver_id);
     if (cfg->b4step_id == CLAW_B4STEP_REVERSING) {
@@ -521,53 +517,21 @@ int claw_destroy(claw_handle* h) {
     return 0;
 }
 
-// Copy a dense host field block [nfields][rows][width] to a pitched device array.
-static int copy_fields(claw_handle* h, void* dev, long long pitch_el, long long fpitch_el,
-                       const double* host, int nfields, long long width, long long rows,
-                       bool to_device) {
-    const Geometry& g = h->g;
-    if (g.es == 8) {
-        for (int m = 0; m < nfields; ++m) {
-            char* d = static_cast<char*>(dev) + (size_t)m * fpitch_el * 8;
-            const double* hp = host + (size_t)m * width * rows;
-            if (to_device)
-                CUDA_TRY(cudaMemcpy2DAsync(d, pitch_el * 8, hp, width * 8, width * 8, rows,
-                                           cudaMemcpyHostToDevice, h->stream));
-            else
-                CUDA_TRY(cudaMemcpy2DAsync(const_cast<double*>(hp), width * 8, d, pitch_el * 8,
-                                           width * 8, rows, cudaMemcpyDeviceToHost, h->stream));
-        }
-    } else {
-        // FP32 storage: stage as doubles on the device, convert there.
-        const long long n = (long long)nfields * fpitch_el;
-        for (int m = 0; m < nfields; ++m) {
-            double* sd = h->stage + (size_t)m * fpitch_el;
-            const double* hp = host + (size_t)m * width * rows;
-            if (to_device)
-                CUDA_TRY(cudaMemcpy2DAsync(sd, pitch_el * 8, hp, width * 8, width * 8, rows,
-                                           cudaMemcpyHostToDevice, h->stream));
-        }
-        if (to_device) {
-            narrow_to_float<<<592, 256, 0, h->stream>>>(h->stage, static_cast<float*>(dev), n);
-        } else {
-            widen_to_double<<<592, 256, 0, h->stream>>>(static_cast<const float*>(dev), h->stage, n);
-            for (int m = 0; m < nfields; ++m) {
-                const double* sd = h->stage + (size_t)m * fpitch_el;
-                double* hp = const_cast<double*>(host) + (size_t)m * width * rows;
-                CUDA_TRY(cudaMemcpy2DAsync(hp, width * 8, sd, pitch_el * 8, width * 8, rows,
-                                           cudaMemcpyDeviceToHost, h->stream));
-            }
-        }
-        CUDA_TRY(cudaGetLastError());
-    }
-    return 0;
+static int copy_block(claw_handle* h, void* dev, long long pitch, long long fpitch, const double* host,
+                      int nfields, long long width, long long rows, bool in) {
+    double* hp = const_cast<double*>(host);  // written only when !in
+    if (h->g.es == 8)
+        return copy_fields(static_cast<double*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage,
+                           h->stage_n, in, h->stream);
+    return copy_fields(static_cast<float*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage,
+                       h->stage_n, in, h->stream);
 }
 
 int claw_set_q(claw_handle* h, const double* q) {
     if (!h || !q) return fail(CLAW_E_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(h->device));
     const Geometry& g = h->g;
-    int rc = copy_fields(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, true);
+    int rc = copy_block(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, true);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return 0;
@@ -577,7 +541,7 @@ int claw_get_q(claw_handle* h, double* q) {
     if (!h || !q) return fail(CLAW_E_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(h->device));
     const Geometry& g = h->g;
-    int rc = copy_fields(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, false);
+    int rc = copy_block(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, false);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return 0;
@@ -588,8 +552,8 @@ int claw_set_aux(claw_handle* h, const double* aux) {
     const Geometry& g = h->g;
     if (g.maux == 0) return 0;
     CUDA_TRY(cudaSetDevice(h->device));
-    const long long rows = (long long)(g.dim >= 2 ? g.my + 4 : 1) * (g.dim >= 3 ? g.mz + 4 : 1);
-    int rc = copy_fields(h, g.aux, g.ald, g.afstride, aux, g.maux, g.mx + 4, rows, true);
+    const long long rows = aux_rows(g);
+    int rc = copy_block(h, g.aux, g.ald, g.afstride, aux, g.maux, g.mx + 4, rows, true);
     if (rc) return rc;
     if (g.aux_base)  // the before-step routine scales from this copy
         CUDA_TRY(cudaMemcpyAsync(g.aux_base, g.aux, (size_t)g.afstride * g.maux * g.es,

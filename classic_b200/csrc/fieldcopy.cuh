@@ -1,0 +1,100 @@
+// Host arrays to and from the pitched device fields.
+//
+// A caller's array is dense [nfields][rows][width] doubles, usually pageable;
+// the device rows are padded and may be FP32.  The driver copies a pageable 2D
+// block row by row and field by field.  us for Euler's four fields, in / out of
+// the device, against one dense copy to or from a device buffer with a kernel
+// that lays the rows out: 72^2 57 / 62 against 30 / 34, 200^2 113 / 140 against
+// 89 / 107, 384^2 327 / 367 against 270 / 275, 700^2 813 / 861 against 820 /
+// 800.  So FP64 blocks of several fields take the buffer up to STAGE_BYTES.  A
+// single field, a 1D grid and up to 64 KB in are cheaper directly (annulus
+// 40x120: 28 against 38; 40^2 42 against 43 to 58; one unpadded field of 64^2
+// 17 against 29 for a 1D copy), and where no row is padded the whole block is
+// one copy (four of 128^2 out: 90 against 54).  FP32 blocks need the buffer for the conversion
+// at any size.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <initializer_list>
+
+#include "common.cuh"
+#include "host.h"
+
+namespace clawb200 {
+
+constexpr size_t STAGE_BYTES = 8u << 20;
+
+// one element a thread, rows over blockIdx.y; row r of field m is dense row
+// m*rows + r
+template <class real, bool IN>
+__global__ void __launch_bounds__(256)
+copy_rows(double* dense, real* dev, long long pitch, long long fpitch, long long width, long long rows,
+          long long nrows) {
+    const long long x = blockIdx.x * 256ll + threadIdx.x;
+    if (x >= width) return;
+    for (long long k = blockIdx.y; k < nrows; k += gridDim.y) {
+        const long long m = k / rows, r = k - m * rows;
+        real* d = dev + m * fpitch + r * pitch + x;
+        if constexpr (IN) *d = (real)dense[k * width + x];
+        else dense[k * width + x] = (double)*d;
+    }
+}
+
+// Queue the copy of nfields fields on the stream (the caller waits for it).
+// `stage` holds stage_n doubles; FP64 blocks of more go directly.
+template <class real>
+int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int nfields, long long width,
+                long long rows, double* stage, size_t stage_n, bool in, cudaStream_t st) {
+    const long long nrows = nfields * rows;
+    const size_t n = (size_t)nrows * width;
+    const auto kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    if constexpr (sizeof(real) == 8) {
+        const bool small_in = in && n * 8 <= 65536;
+        if (pitch == width && fpitch == width * rows && !small_in) {
+            if (in) CUDA_TRY(cudaMemcpyAsync(dev, host, n * 8, kind, st));
+            else CUDA_TRY(cudaMemcpyAsync(host, dev, n * 8, kind, st));
+            return 0;
+        }
+        if (nfields == 1 || rows == 1 || n > stage_n || small_in) {
+            for (int m = 0; m < nfields; ++m) {
+                real* d = dev + m * fpitch;
+                double* hp = host + (size_t)m * width * rows;
+                if (in) CUDA_TRY(cudaMemcpy2DAsync(d, pitch * 8, hp, width * 8, width * 8, rows, kind, st));
+                else CUDA_TRY(cudaMemcpy2DAsync(hp, width * 8, d, pitch * 8, width * 8, rows, kind, st));
+            }
+            return 0;
+        }
+    }
+    const dim3 grid((unsigned)((width + 255) / 256), (unsigned)std::min(nrows, 65535ll));
+    if (in) {
+        CUDA_TRY(cudaMemcpyAsync(stage, host, n * 8, kind, st));
+        copy_rows<real, true><<<grid, 256, 0, st>>>(stage, dev, pitch, fpitch, width, rows, nrows);
+    } else {
+        copy_rows<real, false><<<grid, 256, 0, st>>>(stage, dev, pitch, fpitch, width, rows, nrows);
+        CUDA_TRY(cudaMemcpyAsync(host, stage, n * 8, kind, st));
+    }
+    CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+// The buffer for blocks of these element counts: FP32 fields need the largest,
+// FP64 ones take the largest within STAGE_BYTES, and do without when memory is short.
+inline int make_stage(double** stage, size_t* stage_n, std::initializer_list<size_t> counts, bool needed) {
+    size_t n = 0;
+    for (size_t c : counts)
+        if (needed || c * 8 <= STAGE_BYTES) n = std::max(n, c);
+    if (!n) return 0;
+    const cudaError_t e = cudaMalloc(stage, n * 8);
+    if (e != cudaSuccess) {
+        *stage = nullptr;
+        cudaGetLastError();
+        if (needed) return fail(CLAW_E_CUDA, "%s", cudaGetErrorString(e));
+        return 0;
+    }
+    *stage_n = n;
+    return 0;
+}
+
+}  // namespace clawb200
