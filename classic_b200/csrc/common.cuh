@@ -360,6 +360,53 @@ __device__ __forceinline__ real phi_limiter(int meth, real r) {
     }
 }
 
+// phi of a wave with ratio a / nn (its dot product with the upwind
+// neighbour's wave over its own square), one for a zero wave (nn = 0).  A zero
+// wave's quotient is 1 / 1, whose phi is one for every limiter, and a zero
+// numerator's, which would take the division's general path, nn / nn: two
+// compares and three selects around the division and phi, where div_ieee and
+// both cases apart took four and six.  The reference-order kernels are bound by
+// issue slots, of which three in four are not FP64 arithmetic: with upwind and
+// the known Courant number below, radial 1024^2 50.5 -> 42.2 us a step, Strang
+// 67.5 -> 54.2; this alone, 3D 128^3 1.66 -> 1.60 ms.
+template <typename real>
+__device__ __forceinline__ real phi_of(int meth, real a, real nn) {
+    const bool live = nn != real(0), zero = live && a == real(0);
+    const real den = live ? nn : real(1);
+    const real p = phi_limiter<real>(meth, (live && !zero ? a : den) / den);
+    if (meth < 1) return real(1);
+    return zero ? (meth == 5 ? a : real(0)) : p;  // (NaN nn: a is NaN too)
+}
+
+// S::dir(mw), where a solver has it: the sign of wave mw's speed; 0 where only
+// the speed itself tells.  The upwind neighbour of a wave.
+template <class S, class = void>
+struct wave_dir { __host__ __device__ static constexpr int of(int) { return 0; } };
+template <class S>
+struct wave_dir<S, decltype((void)S::dir(0))> { __host__ __device__ static constexpr int of(int mw) { return S::dir(mw); } };
+template <class S, typename real>
+__device__ __forceinline__ real upwind(int mw, real s, real left, real right) {
+    const int d = wave_dir<S>::of(mw);
+    if (d != 0) return d > 0 ? left : right;
+    return s > real(0) ? left : right;
+}
+
+// The Courant number of a solver whose speeds are one constant (S::top_speed),
+// where no capacity scales them, needs no face: every face has it.
+template <class S, class = void>
+struct const_speed { static constexpr bool value = false; };
+template <class S>
+struct const_speed<S, decltype((void)&S::top_speed)> { static constexpr bool value = true; };
+
+// min(x, 0) and max(x, 0), fmin's and fmax's values (zero for a NaN)
+template <typename real>
+__device__ __forceinline__ real neg_part(real x) { return x < real(0) ? x : real(0); }
+template <typename real>
+__device__ __forceinline__ real pos_part(real x) { return x > real(0) ? x : real(0); }
+
+// Fold a face's Courant number c into m (not NaN): fmax(m, c), by a select.
+__device__ __forceinline__ double fold_cfl(double m, double c) { return c > m ? c : m; }
+
 // phi(r) of the contracted build: the same functions by compare-and-select
 // (no fmin/fmax, whose NaN rules cost extra FP64 instructions) and a Newton
 // reciprocal in van Leer's quotient.

@@ -39,6 +39,9 @@ struct Acoustics2D {
     using real = real_;
     static constexpr int meqn = 3, mwaves = 2, maux = 0;
     real cc, zz, hz;
+    // s = -cc, cc (cc = 0 or NaN has no finite hz, and no finite wave)
+    __host__ __device__ static constexpr int dir(int mw) { return mw == 0 ? -1 : 1; }
+    __device__ __forceinline__ double top_speed() const { return (double)cc; }
 
     // Structurally zero components (the kernels skip arithmetic on them; the
     // skipped terms are exact zeros, so results are value-identical):
@@ -94,8 +97,7 @@ struct Acoustics2D {
 // (LeVeque, Finite Volume Methods for Hyperbolic Problems, 15.3 and 18.8;
 // Harten & Hyman, J. Comput. Phys. 50, 1983.)
 // FAST (the contracted build): Newton reciprocals and square roots instead
-// of IEEE division and sqrt (to about an ulp), compare-and-select instead of
-// fmin/fmax.
+// of IEEE division and sqrt (to about an ulp).
 template <typename real_, bool FAST = false>
 struct EulerRoe2D {
     using real = real_;
@@ -103,14 +105,6 @@ struct EulerRoe2D {
     static constexpr int min_blocks = EULER_MINB;  // registers for the Roe state
     real gamma, gamma1;
     using AR = Arith<FAST>;
-    __device__ __forceinline__ static real min0(real x) {
-        if constexpr (FAST) return x < real(0) ? x : real(0);
-        else return fmin(x, real(0));
-    }
-    __device__ __forceinline__ static real max0(real x) {
-        if constexpr (FAST) return x > real(0) ? x : real(0);
-        else return fmax(x, real(0));
-    }
     __host__ __device__ static constexpr bool wave_zero(int, int) { return false; }
     __host__ __device__ static constexpr bool trans_zero(int, int) { return false; }
 
@@ -257,8 +251,8 @@ struct EulerRoe2D {
         sb[2] = r.v + r.a;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            bm[m] = (min0(sb[0]) * w[0][m] + min0(sb[1]) * w[1][m]) + min0(sb[2]) * w[2][m];
-            bp[m] = (max0(sb[0]) * w[0][m] + max0(sb[1]) * w[1][m]) + max0(sb[2]) * w[2][m];
+            bm[m] = (neg_part(sb[0]) * w[0][m] + neg_part(sb[1]) * w[1][m]) + neg_part(sb[2]) * w[2][m];
+            bp[m] = (pos_part(sb[0]) * w[0][m] + pos_part(sb[1]) * w[1][m]) + pos_part(sb[2]) * w[2][m];
         }
     }
 };
@@ -280,16 +274,16 @@ struct VCAdvection2D {
         const real si = auxR[ixy - 1];
         wave[0][0] = w;
         s[0] = si;
-        amdq[0] = fmin(si, real(0)) * w;
-        apdq[0] = fmax(si, real(0)) * w;
+        amdq[0] = neg_part(si) * w;
+        apdq[0] = pos_part(si) * w;
     }
 
     __device__ __forceinline__ void rpt(int ixy, int, const real*, const real*, const real*,
                                         const real* aux2, const real* aux3, const real* asdq,
                                         real bmasdq[meqn], real bpasdq[meqn]) const {
         const int it = 2 - ixy;  // transverse velocity component (0-based)
-        bmasdq[0] = fmin(aux2[it], real(0)) * asdq[0];
-        bpasdq[0] = fmax(aux3[it], real(0)) * asdq[0];
+        bmasdq[0] = neg_part(aux2[it]) * asdq[0];
+        bpasdq[0] = pos_part(aux3[it]) * asdq[0];
     }
 };
 
@@ -336,8 +330,8 @@ struct Advection1D {
         const real d = qR[0] - qL[0];
         wave[0][0] = d;
         s[0] = u;
-        amdq[0] = fmin(u, real(0)) * d;
-        apdq[0] = fmax(u, real(0)) * d;
+        amdq[0] = neg_part(u) * d;
+        apdq[0] = pos_part(u) * d;
     }
 };
 

@@ -229,28 +229,24 @@ __global__ void __launch_bounds__(THREADS, 1) step1_kernel(const __grid_constant
             for (int m = 0; m < ME; ++m) qL[m] = __shfl_up_sync(FULL, q[m], 1);
             A.solver.rp1(qL, q, aL, a, w, s, am, ap);
             if (order2) {
-                // the waves' ratios side by side: their divisions overlap
-                real nn[MW], r[MW];
+                // the waves' limiters side by side: their divisions overlap
+                real ph[MW];
 #pragma unroll
                 for (int mw = 0; mw < MW; ++mw) {
-                    real dr = real(0);
-                    nn[mw] = real(0);
+                    real dr = real(0), nn = real(0);
 #pragma unroll
                     for (int m = 0; m < ME; ++m) {
                         const real wn = __shfl_down_sync(FULL, w[mw][m], 1);
-                        nn[mw] = nn[mw] + w[mw][m] * w[mw][m];
+                        nn = nn + w[mw][m] * w[mw][m];
                         dr = dr + w[mw][m] * wn;
                     }
                     const real dl = __shfl_up_sync(FULL, dr, 1);
-                    // a zero wave is left as it is; its ratio is not used
-                    r[mw] = div_ieee(s[mw] > real(0) ? dl : dr, nn[mw] != real(0) ? nn[mw] : real(1));
+                    ph[mw] = phi_of<real>(ANY ? A.mthlim[mw] : M::lim, s[mw] > real(0) ? dl : dr, nn);
                 }
 #pragma unroll
                 for (int mw = 0; mw < MW; ++mw) {
-                    const real p = phi_limiter<real>(ANY ? A.mthlim[mw] : M::lim, r[mw]);
-                    const real ph = nn[mw] != real(0) ? p : real(1);
 #pragma unroll
-                    for (int m = 0; m < ME; ++m) w[mw][m] = ph * w[mw][m];
+                    for (int m = 0; m < ME; ++m) w[mw][m] = ph[mw] * w[mw][m];
                 }
             }
         };

@@ -254,21 +254,16 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                  A.mthlim[5] | A.mthlim[6] | A.mthlim[7]) != 0;
     auto lim_of = [&](int mw) -> int { return M::lim >= 0 ? M::lim : A.mthlim[mw]; };
     using AR = Arith<M::fast>;
-    // max of two Courant numbers (the same value as fmax for non-NaN operands)
-    auto dmax = [](double a, double b) -> double {
-        if constexpr (M::fast) return b > a ? b : a;
-        else return fmax(a, b);
+    // phi of a wave from its dot product with the upwind one and its square
+    auto phi = [](int ml, real n, real nn) -> real {
+        if constexpr (M::fast) {
+            const real p = phi_limiter_fast<real>(ml, AR::div(n, nn));
+            return nn != real(0) ? p : real(1);
+        } else {
+            return phi_of<real>(ml, n, nn);
+        }
     };
-    auto phi = [](int ml, real r) -> real {
-        if constexpr (M::fast) return phi_limiter_fast<real>(ml, r);
-        else return phi_limiter<real>(ml, r);
-    };
-    // limiter ratio; a zero wave's is not used, and dividing by 1 keeps it off
-    // the division's general path
-    auto ratio = [](real n, real nn) -> real {
-        if constexpr (M::fast) return AR::div(n, nn);
-        else return AR::div(n, nn != real(0) ? nn : real(1));
-    };
+    constexpr bool KNOWN = const_speed<S>::value && M::capa == 0;  // Courant number
     const int lane = threadIdx.x & 31;
     const int mx = A.mx, my = A.my;
 
@@ -331,14 +326,14 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         const bool glob = left ? gm : gc, neg = left ? negm : negc;
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
-            real v = sq[m * W + at];
-            if (any_global) {
-                if (glob) v = qold[m * A.fstride + (long long)sr * A.ld + src];
-            }
-            if (m == 1) v = neg ? -v : v;
-            if (m == 2 && nyneg) v = -v;
-            q[m] = v;
+            q[m] = sq[m * W + at];
         }
+        if (any_global && glob) {
+#pragma unroll
+            for (int m = 0; m < ME; ++m) q[m] = qold[m * A.fstride + (long long)sr * A.ld + src];
+        }
+        if (ME > 1) q[ME > 1 ? 1 : 0] = neg ? -q[ME > 1 ? 1 : 0] : q[ME > 1 ? 1 : 0];
+        if (ME > 2) q[ME > 2 ? 2 : 0] = nyneg ? -q[ME > 2 ? 2 : 0] : q[ME > 2 ? 2 : 0];
         if constexpr (SRC) {
             // Strang: dt/2 of source on the data the step reads
             if (K.src == 2) src_radial_cell(A, q, left ? c - 1 : c, K.src_pre);
@@ -413,13 +408,13 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         else A.solver.rpn(2, qc_t, qc_n, a_c, a_cn, wy, sy, amy, apy);
         ky_p = scale(dtdy, dtdy_d, a_c);
         ky_t = scale(dtdy, dtdy_d, a_cn);
-        if (cy_ok && rfirst + 1 >= 0) {
+        if (!KNOWN && cy_ok && rfirst + 1 >= 0) {
             const double dt0 = ky_p.d, dt1 = ky_t.d;
             double em = 0.0;
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw)
-                em = dmax(em, dmax(dt1 * (double)sy[mw], -dt0 * (double)sy[mw]));
-            cfl = dmax(cfl, em);
+                em = fold_cfl(fold_cfl(em, dt1 * (double)sy[mw]), -dt0 * (double)sy[mw]);
+            cfl = fold_cfl(cfl, em);
         }
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
@@ -452,13 +447,13 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
             else A.solver.rpn(1, qm_t, qc_t, a_m, a_c, w, s, amdq, apdq);
             const Scale kc = scale(dtdx, dtdx_d, a_c), km = scale_left(kc);
             const real dtm = km.v, dtc = kc.v;  // dtdx1d(i-1), dtdx1d(i)
-            {
+            if constexpr (!KNOWN) {
                 const double dm = km.d, dc = kc.d;
                 double em = 0.0;
 #pragma unroll
                 for (int mw = 0; mw < MW; ++mw)
-                    em = dmax(em, dmax(dc * (double)s[mw], -dm * (double)s[mw]));
-                cfl = (cx_ok && t >= -1 && t <= my) ? dmax(cfl, em) : cfl;
+                    em = fold_cfl(fold_cfl(em, dc * (double)s[mw]), -dm * (double)s[mw]);
+                cfl = (cx_ok && t >= -1 && t <= my) ? fold_cfl(cfl, em) : cfl;
             }
             real send1[ME], qadd[ME], F[ME], cq[ME];
 #pragma unroll
@@ -496,9 +491,9 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                     for (int mw = 0; mw < MW; ++mw) {
                         const int ml = lim_of(mw);
                         if (ml == 0) continue;
-                        const real dl = __shfl_up_sync(FULL, dotr[mw], 1);
-                        const real r = ratio(s[mw] > real(0) ? dl : dotr[mw], wn2[mw]);
-                        const real ph = wn2[mw] != real(0) ? phi(ml, r) : real(1);
+                        real dl = real(0);
+                        if (wave_dir<S>::of(mw) >= 0) dl = __shfl_up_sync(FULL, dotr[mw], 1);
+                        const real ph = phi(ml, upwind<S>(mw, s[mw], dl, dotr[mw]), wn2[mw]);
 #pragma unroll
                         for (int m = 0; m < ME; ++m)
                             if (!S::wave_zero(1, m)) w[mw][m] = ph * w[mw][m];
@@ -596,13 +591,13 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
         if constexpr (solver_ctx<S>::value) A.solver.rpn_ctx(2, cyn, qc_t, qc_n, wn, sn, amn, apn);
         else A.solver.rpn(2, qc_t, qc_n, a_c, a_cn, wn, sn, amn, apn);
         const Scale ky_n = scale(dtdy, dtdy_d, a_cn);
-        {
+        if constexpr (!KNOWN) {
             const double dt0 = ky_t.d, dt1 = ky_n.d;
             double em = 0.0;
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw)
-                em = dmax(em, dmax(dt1 * (double)sn[mw], -dt0 * (double)sn[mw]));
-            cfl = (cy_ok && t + 1 <= my) ? dmax(cfl, em) : cfl;
+                em = fold_cfl(fold_cfl(em, dt1 * (double)sn[mw]), -dt0 * (double)sn[mw]);
+            cfl = (cy_ok && t + 1 <= my) ? fold_cfl(cfl, em) : cfl;
         }
         const real dty_p = ky_p.v, dty_t = ky_t.v;  // dtdy1d(t-1), dtdy1d(t)
         real cqy[ME], Fy[ME], dotr_y[MW];
@@ -634,8 +629,7 @@ __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepCons
                         nn = first ? wy[mw][m] * wy[mw][m] : nn + wy[mw][m] * wy[mw][m];
                         first = false;
                     }
-                    const real r = ratio(sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw], nn);
-                    const real ph = nn != real(0) ? phi(ml, r) : real(1);
+                    const real ph = phi(ml, upwind<S>(mw, sy[mw], dotl_y[mw], dotr_y[mw]), nn);
 #pragma unroll
                     for (int m = 0; m < ME; ++m)
                         if (!S::wave_zero(2, m)) wy[mw][m] = ph * wy[mw][m];
@@ -766,7 +760,6 @@ template <class S, class M, bool SRC = false>
 __global__ void __launch_bounds__(32 * WARPS2D, step2_minb<S>::value)
 step2_kernel(const __grid_constant__ Step2Args<S> A) {
     ClawCtl* ctl = A.ctl;
-    __shared__ double red[WARPS2D];
     using R = Ring2D<S>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -809,7 +802,14 @@ step2_kernel(const __grid_constant__ Step2Args<S> A) {
         step2_rows<S, M, SRC>(A, K, strip, r0, nr, ring, bars, seq_base, cfl, failed);
     }
 
-    cta_cfl_and_control(ctl, cfl, red);
+    if constexpr (const_speed<S>::value && M::capa == 0) {
+        const double cd = A.solver.top_speed();
+        const double v = fold_cfl(K.dtdx_d * cd, K.dtdy_d * cd);
+        cta_count_and_control(ctl, failed, [&](const CtlIn&) { return v > 0.0 ? v : 0.0; });
+    } else {
+        __shared__ double red[WARPS2D];
+        cta_cfl_and_control(ctl, cfl, red);
+    }
 }
 
 }  // namespace clawb200
@@ -905,6 +905,8 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
         u0 += nr;
         double cfl = 0.0;
         step2_rows<S, M>(A, K, strip, r0, nr, ring, bars, seq_base, cfl, failed);
+        if constexpr (const_speed<S>::value && M::capa == 0)
+            cfl = fold_cfl(K.dtdx_d * A.solver.top_speed(), K.dtdy_d * A.solver.top_speed());
         for (int o = 16; o > 0; o >>= 1) cfl = fmax(cfl, __shfl_xor_sync(FULL, cfl, o));
         if (lane == 0) {
             if (failed) atomicOr(B.err, CTL_ERR_TMA_TIMEOUT);

@@ -104,11 +104,12 @@ __device__ __forceinline__ void split_xslice(const Step2Args<S>& A, const typena
     }
     const real dtm = capa ? dtdx / am[ic] : dtdx;  // dtdx1d(i-1)
     const real dtc = capa ? dtdx / ac[ic] : dtdx;  // dtdx1d(i)
-    if (cfl_ok) {
+    if (!(const_speed<S>::value && M::capa == 0) && cfl_ok) {
         const double dm = capa ? dtdx_d / (double)am[ic] : dtdx_d;
         const double dc = capa ? dtdx_d / (double)ac[ic] : dtdx_d;
 #pragma unroll
-        for (int mw = 0; mw < MW; ++mw) cfl = fmax(fmax(cfl, dc * (double)s[mw]), -dm * (double)s[mw]);
+        for (int mw = 0; mw < MW; ++mw)
+            cfl = fold_cfl(fold_cfl(cfl, dc * (double)s[mw]), -dm * (double)s[mw]);
     }
     real send1[ME], qadd[ME], F[ME];
 #pragma unroll
@@ -144,10 +145,10 @@ __device__ __forceinline__ void split_xslice(const Step2Args<S>& A, const typena
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw) {
                 const int ml = M::lim >= 0 ? M::lim : A.mthlim[mw];
-                const real dl = __shfl_up_sync(FULL, dotr[mw], 1);
+                real dl = real(0);
+                if (wave_dir<S>::of(mw) >= 0) dl = __shfl_up_sync(FULL, dotr[mw], 1);
                 if (ml == 0) continue;
-                const real r = div_ieee(s[mw] > real(0) ? dl : dotr[mw], wn2[mw] != real(0) ? wn2[mw] : real(1));
-                const real ph = wn2[mw] != real(0) ? phi_limiter<real>(ml, r) : real(1);
+                const real ph = phi_of<real>(ml, upwind<S>(mw, s[mw], dl, dotr[mw]), wn2[mw]);
 #pragma unroll
                 for (int m = 0; m < ME; ++m)
                     if (!S::wave_zero(1, m)) w[mw][m] = ph * w[mw][m];
@@ -196,6 +197,7 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
     constexpr int MAX = MA > 0 ? MA : 1;
     constexpr int W = L::W;
     constexpr unsigned FULL = 0xffffffffu;
+    constexpr bool KNOWN = const_speed<S>::value && M::capa == 0;  // Courant number
     ClawCtl* ctl = A.ctl;
     const real* __restrict__ qold = K.qold;
     real* __restrict__ qnew = K.qnew;
@@ -267,12 +269,14 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
         const int sr = bc_map(r, my, A.bc[2], A.bc[3], nyneg);
 #pragma unroll
         for (int m = 0; m < ME; ++m) {
-            real v = sq[m * W + icc];
-            if (any_global && gc) v = qold[m * A.fstride + (long long)sr * A.ld + sc];
-            if (m == 1 && negc) v = -v;
-            if (m == 2 && nyneg) v = -v;
-            qv[m] = v;
+            qv[m] = sq[m * W + icc];
         }
+        if (any_global && gc) {
+#pragma unroll
+            for (int m = 0; m < ME; ++m) qv[m] = qold[m * A.fstride + (long long)sr * A.ld + sc];
+        }
+        if (ME > 1) qv[1] = negc ? -qv[1] : qv[1];
+        if (ME > 2) qv[ME > 2 ? 2 : 0] = nyneg ? -qv[ME > 2 ? 2 : 0] : qv[ME > 2 ? 2 : 0];
         if constexpr (SRC) {
             if (K.src == 2) src_radial_cell(A, qv, c, K.src_pre);  // Strang: before the step
         }
@@ -312,12 +316,12 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
     };
     auto ycfl = [&](int t, const real* sv, const real* alo, const real* ahi) {
         // y-interface t-1|t counts for t = 0..my
-        if (cy_ok && t >= 0 && t <= my) {
+        if (!KNOWN && cy_ok && t >= 0 && t <= my) {
             const double d0 = capa ? K.dtdy_d / (double)alo[ic] : K.dtdy_d;
             const double d1 = capa ? K.dtdy_d / (double)ahi[ic] : K.dtdy_d;
 #pragma unroll
             for (int mw = 0; mw < MW; ++mw)
-                cfl[1] = fmax(fmax(cfl[1], d1 * (double)sv[mw]), -d0 * (double)sv[mw]);
+                cfl[1] = fold_cfl(fold_cfl(cfl[1], d1 * (double)sv[mw]), -d0 * (double)sv[mw]);
         }
     };
     // Strang stage C on a row whose y-sweep is done (all lanes call)
@@ -389,8 +393,7 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
                         nn = first ? wy[mw][m] * wy[mw][m] : nn + wy[mw][m] * wy[mw][m];
                         first = false;
                     }
-                    const real r = div_ieee(sy[mw] > real(0) ? dotl_y[mw] : dotr_y[mw], nn != real(0) ? nn : real(1));
-                    const real ph = nn != real(0) ? phi_limiter<real>(ml, r) : real(1);
+                    const real ph = phi_of<real>(ml, upwind<S>(mw, sy[mw], dotl_y[mw], dotr_y[mw]), nn);
 #pragma unroll
                     for (int m = 0; m < ME; ++m)
                         if (!S::wave_zero(2, m)) wy[mw][m] = ph * wy[mw][m];
@@ -535,7 +538,6 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
     using L = SplitLayout<S, STRANG>;
     using real = typename S::real;
     ClawCtl* ctl = A.ctl;
-    __shared__ double red[3 * WARPS2D];
     extern __shared__ __align__(128) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* ring = smem + warp * L::WARP_BYTES;
@@ -590,7 +592,16 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
         u0 += nr;
         split2_rows<S, M, STRANG, SRC>(A, K, strip, r0, nr, ring, bars, seq_base, cfl, failed);
     }
-    cta_split_cfl_and_control(ctl, cfl, STRANG ? 3 : 2, red);
+    if constexpr (const_speed<S>::value && M::capa == 0) {
+        const double cd = A.solver.top_speed();
+        auto known = [&](double v) { return v > 0.0 ? v : 0.0; };
+        cta_count_and_control(ctl, failed, [&](const CtlIn& in) {
+            return split_cfl(in, STRANG ? 3 : 2, known(K.dtdx_a_d * cd), known(K.dtdy_d * cd), known(K.dtdx_c_d * cd));
+        });
+    } else {
+        __shared__ double red[3 * WARPS2D];
+        cta_split_cfl_and_control(ctl, cfl, STRANG ? 3 : 2, red);
+    }
 }
 
 }  // namespace clawb200

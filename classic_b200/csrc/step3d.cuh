@@ -467,14 +467,11 @@ __device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::rea
                 const int lim = M::lim >= 0 ? M::lim : a.mthlim[k];
                 if (order == 2 && lim > 0) {
                     const real wn2 = wB[k][0] * wB[k][0] + wB[k][1] * wB[k][1];
-                    if (wn2 != real(0)) {
-                        const real dl = wA[k][0] * wB[k][0] + wA[k][1] * wB[k][1];
-                        const real dr = wB[k][0] * wC[k][0] + wB[k][1] * wC[k][1];
-                        const real r = div_ieee(sB[k] > real(0) ? dl : dr, wn2);
-                        const real phi = phi_limiter<real>(lim, r);
-                        wl[k][0] = phi * wB[k][0];
-                        wl[k][1] = phi * wB[k][1];
-                    }
+                    const real dl = wA[k][0] * wB[k][0] + wA[k][1] * wB[k][1];
+                    const real dr = wB[k][0] * wC[k][0] + wB[k][1] * wC[k][1];
+                    const real phi = phi_of<real>(lim, sB[k] > real(0) ? dl : dr, wn2);
+                    wl[k][0] = phi * wB[k][0];
+                    wl[k][1] = phi * wB[k][1];
                 }
             }
             if (order == 2) {

@@ -126,12 +126,9 @@ __device__ __forceinline__ void ds3_flux(const Split3Args<real>& a, const real (
         const int lim = a.mthlim[k];
         if (lim > 0) {
             const real wn2 = w[k][0] * w[k][0] + w[k][1] * w[k][1];
-            if (wn2 != real(0)) {
-                const real r = div_ieee(s[k] > real(0) ? dl[k] : dr[k], wn2);
-                const real phi = phi_limiter<real>(lim, r);
-                w0 = phi * w[k][0];
-                w1 = phi * w[k][1];
-            }
+            const real phi = phi_of<real>(lim, s[k] > real(0) ? dl[k] : dr[k], wn2);
+            w0 = phi * w[k][0];
+            w1 = phi * w[k][1];
         }
         const real as_ = fabs(s[k]);
         const real coef = (real(0.5) * as_) * (real(1) - as_ * dtdxave);
@@ -184,7 +181,7 @@ __global__ void __launch_bounds__(32 * DS3_WARPS) split3_x_kernel(const Split3Ar
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk) {
                 const double c = tn_d * (double)s[kk];
-                cfl = fmax(fmax(cfl, c), -c);
+                cfl = fold_cfl(fold_cfl(cfl, c), -c);
             }
         }
         real F[2] = {real(0), real(0)};
@@ -309,7 +306,7 @@ __global__ void __launch_bounds__(32 * DS3_WARPS, 2) split3_yz_kernel(const Spli
 #pragma unroll
                 for (int kk = 0; kk < 2; ++kk) {
                     const double c = tn_d * (double)sn[kk];
-                    cfl = fmax(fmax(cfl, c), -c);
+                    cfl = fold_cfl(fold_cfl(cfl, c), -c);
                 }
             }
             const real dr0 = w[0][0] * wn[0][0] + w[0][1] * wn[0][1];
