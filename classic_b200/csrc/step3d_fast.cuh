@@ -49,8 +49,8 @@
 // reference-order build's.
 //
 // Measured against three sweep launches that formed every split (1815 FP64
-// instructions and 245 B of DRAM traffic per cell): 256^3 FP64 7.45 -> 1.32
-// ms per step, 161x130x147 FP32 1.02 -> 0.167.  What bounds it: FP64 at
+// instructions and 245 B of DRAM traffic per cell): 256^3 FP64 7.45 -> 1.30
+// ms per step, 161x130x147 FP32 1.02 -> 0.158.  What bounds it: FP64 at
 // 192^3 runs the FP64 pipe at 30 % and issue at 46 % with 12 warps per SM
 // (fixed-latency chains and the three barriers); FP32 is issue bound (71 %).
 // DRAM traffic is 77 B per cell (80 algorithmic).
@@ -64,7 +64,8 @@ namespace clawb200 {
 // a thread and nothing spills; the shared planes leave so little L1 that any
 // spill goes to L2 (256^3, ms per step: 12 rows 1.32, 13 rows at 144
 // registers 2.41, 16 rows at 128 2.1, 8 rows x 2 CTAs 1.9).  FP32: two CTAs of
-// 9 rows hide each other's barriers (161x130x147, us per step: 9 x 2 167,
+// 9 rows hide each other's barriers (161x130x147, us per step, before the
+// plane table: 9 x 2 167,
 // 8 x 2 172, 10 x 2 181, 16 x 1 177, 18 x 1 188, 7 x 3 193).
 #ifndef CLAW_STEP3F_ROWS
 #define CLAW_STEP3F_ROWS 12
@@ -111,6 +112,12 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     constexpr int kUnroll = CLAW_STEP3F_UNROLL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[ROWS];
+    // planes t-1 .. t+4 at [pos & 7]: where q and aux lie in global memory, and
+    // whether w changes its sign (1) or takes the piston's (2) there.  One thread
+    // fills an entry a plane ahead; each thread for itself, three times a plane, it
+    // cost the FP32 kernel, bound by issue, 5 % (192^3 314 -> 298 us a step; FP64
+    // 517 -> 509)
+    __shared__ struct { const real *q, *aux; int w; } zt[8];
     const Sweep3Args<real>& a = A.g;
     ClawCtl* ctl = a.ctl;
     grid_dependency_sync();
@@ -174,42 +181,40 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     // q plus its own sums, the edge fluxes at t-3/2, plane t-1's Yy
     real* SB = ex + 20 * PL;
 
-    auto zsrc = [&](int pos, bool& neg) {
-        return bc3_src(min(pos, mz + 2), mz, a.bc[4], a.bc[5], neg);
+    auto fill = [&](int pos) {
+        bool neg;
+        const int pm = bc3_src(min(pos, mz + 2), mz, a.bc[4], a.bc[5], neg);
+        zt[pos & 7].q = qold + (long long)(pm - 1) * a.qs[2];
+        zt[pos & 7].aux = aux + (long long)(min(pos, mz + 2) + 1) * a.as[2];
+        zt[pos & 7].w = (neg ? 1 : 0) | (pos > mz && a.bc[5] == BC_PISTON ? 2 : 0);
     };
     // copies of plane pos: p, Z, c into ring slot `so`, w into its parity's
     auto issue_pzc = [&](int pos, int so) {
-        bool neg;
-        const int pm = zsrc(pos, neg);
-        const long long qz = (long long)(pm - 1) * a.qs[2];
-        const long long az = (long long)(min(pos, mz + 2) + 1) * a.as[2];
+        const real *q = zt[pos & 7].q, *x = zt[pos & 7].aux;
         real* d = ring + so + own;
-        cp_async_el(d, qold + qxy + qz);
-        cp_async_el(d + PL, aux + axy + az);
-        cp_async_el(d + 2 * PL, aux + axy + az + a.afstride);
-        cp_async_el(uvw + ((pos & 1) * 3 + 2) * PL + own, qold + qxy + qz + 3 * a.fstride);
+        cp_async_el(d, q + qxy);
+        cp_async_el(d + PL, x + axy);
+        cp_async_el(d + 2 * PL, x + axy + a.afstride);
+        cp_async_el(uvw + ((pos & 1) * 3 + 2) * PL + own, q + qxy + 3 * a.fstride);
         if (edge) {
             real* h = ring + so + hal;
-            cp_async_el(h, qold + qxh + qz);
-            cp_async_el(h + PL, aux + axh + az);
-            cp_async_el(h + 2 * PL, aux + axh + az + a.afstride);
+            cp_async_el(h, q + qxh);
+            cp_async_el(h + PL, x + axh);
+            cp_async_el(h + 2 * PL, x + axh + a.afstride);
         }
     };
     auto issue_uv = [&](int pos) {
-        bool neg;
-        const int pm = zsrc(pos, neg);
-        const long long qz = (long long)(pm - 1) * a.qs[2];
+        const real* q = zt[pos & 7].q;
         real* d = uvw + (pos & 1) * 3 * PL;
-        cp_async_el(d + own, qold + qxy + qz + a.fstride);
-        cp_async_el(d + PL + own, qold + qxy + qz + 2 * a.fstride);
-        if (edge) cp_async_el(d + PL + hal, qold + qxh + qz + 2 * a.fstride);
+        cp_async_el(d + own, q + qxy + a.fstride);
+        cp_async_el(d + PL + own, q + qxy + 2 * a.fstride);
+        if (edge) cp_async_el(d + PL + hal, q + qxh + 2 * a.fstride);
     };
     // w at plane pos from its stored value (the walls' and the piston's sign)
     auto wbc = [&](int pos, real w) {
-        bool neg;
-        (void)zsrc(pos, neg);
-        if (neg) w = -w;
-        if (pos > mz && a.bc[5] == BC_PISTON) w = (real)(2.0 * piston_speed(a, i, j, tbc)) - w;
+        const int f = zt[pos & 7].w;
+        if (f & 1) w = -w;
+        if (f & 2) w = (real)(2.0 * piston_speed(a, i, j, tbc)) - w;
         return w;
     };
     auto lim_a = [&](real s, real n) { return limited_strength<real, LIM>(s, n, lim1); };
@@ -233,11 +238,10 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     const int t0 = k0 - 1;
     real w0, w1, wm;  // w at planes t, t+1 (t-1)
     real a1z, a2z, a2zm, rz, rz1, g0;
+    if (threadIdx.x < 6) fill(t0 - 1 + (int)threadIdx.x);
+    __syncthreads();
     {
-        bool neg;
-        auto w_at = [&](int pos) {
-            return wbc(pos, qold[qxy + (long long)(zsrc(pos, neg) - 1) * a.qs[2] + 3 * a.fstride]);
-        };
+        auto w_at = [&](int pos) { return wbc(pos, zt[pos & 7].q[qxy + 3 * a.fstride]); };
         wm = w_at(t0 - 1);
         w0 = w_at(t0);
         w1 = w_at(t0 + 1);
@@ -274,6 +278,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     for (int t = t0; t <= k1; ++t) {
         if (t + 3 <= k1 + 1) issue_pzc(t + 3, s3);
         if (t + 1 <= k1) issue_uv(t + 1);
+        if (threadIdx.x == 0) fill(t + 4);
         const int par = t & 1;
         real* SPt = SP + par * 3 * PL;
         real* SPm = SP + (par ^ 1) * 3 * PL;
@@ -284,7 +289,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         real u = UV[own], v = UV[PL + own];
         if (negx) u = -u;
         if (negy) v = -v;
-        if (inxy) cmax = fmax(cmax, fabs(c));
+        if (inxy && fabs(c) > cmax) cmax = fabs(c);  // a NaN leaves it
         const real zl = P[PL + lm], cl = P[2 * PL + lm];
         real rx, a1x, a2x;
         {
