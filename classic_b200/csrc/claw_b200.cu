@@ -178,6 +178,9 @@ std::unique_ptr<Runner> make_runner(const claw_config& cfg) {
         EulerRoe2D<real> s{(real)gamma, (real)(gamma - 1.0)};
         return runner2d(cfg, s);
     }
+    if (id == CLAW_SOLVER_VC_ADVECTION_2D && cfg.order == 2 && cfg.transverse_waves == 2 && cfg.capa_index > 0 &&
+        !cfg.use_fwaves)
+        return std::unique_ptr<Runner>(new Runner2D<VCAdvection2D<real>, MethodCapa2D>(VCAdvection2D<real>{}));
     if (id == CLAW_SOLVER_VC_ADVECTION_2D)
         return std::unique_ptr<Runner>(new Runner2D<VCAdvection2D<real>, MethodGeneric2D>(VCAdvection2D<real>{}));
     if (id == CLAW_SOLVER_VC_ACOUSTICS_1D)

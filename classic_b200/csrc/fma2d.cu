@@ -41,6 +41,9 @@ std::unique_ptr<Runner> make_fast_runner2d(const claw_config& cfg) {
         const double gamma = cfg.solver_params[0];
         return fast_runner(cfg, EulerRoe2D<double, true>{gamma, gamma - 1.0});
     }
+    if (id == CLAW_SOLVER_VC_ADVECTION_2D && cfg.order == 2 && cfg.transverse_waves == 2 && cfg.capa_index > 0 &&
+        !cfg.use_fwaves)
+        return std::unique_ptr<Runner>(new Runner2D<VCAdvection2D<double>, MethodCapa2DFast>(VCAdvection2D<double>{}));
     if (id == CLAW_SOLVER_VC_ADVECTION_2D)
         return std::unique_ptr<Runner>(
             new Runner2D<VCAdvection2D<double>, MethodGeneric2DFast>(VCAdvection2D<double>{}));

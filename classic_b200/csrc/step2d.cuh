@@ -64,7 +64,9 @@ struct Method2D {
 };
 using MethodGeneric2D = Method2D<-1, -1, -1, -1, -1>;
 using MethodMC2D = Method2D<2, 2, 4, 0, 0>;  // order 2, transverse 2, MC, no capa
+using MethodCapa2D = Method2D<2, 2, -1, 1, 0>;  // the same of a mapped grid, any limiter
 using MethodGeneric2DFast = Method2D<-1, -1, -1, -1, -1, 1>;
+using MethodCapa2DFast = Method2D<2, 2, -1, 1, 0, 1>;
 using MethodMC2DFast = Method2D<2, 2, 4, 0, 0, 1>;
 
 template <class S>

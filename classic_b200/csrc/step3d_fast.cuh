@@ -65,8 +65,8 @@ namespace clawb200 {
 // spill goes to L2 (256^3, ms per step: 12 rows 1.32, 13 rows at 144
 // registers 2.41, 16 rows at 128 2.1, 8 rows x 2 CTAs 1.9).  FP32: two CTAs of
 // 9 rows hide each other's barriers (161x130x147, us per step, before the
-// plane table: 9 x 2 167,
-// 8 x 2 172, 10 x 2 181, 16 x 1 177, 18 x 1 188, 7 x 3 193).
+// plane table: 9 x 2 167, 8 x 2 172, 10 x 2 181, 16 x 1 177, 18 x 1 188, 7 x 3
+// 193).
 #ifndef CLAW_STEP3F_ROWS
 #define CLAW_STEP3F_ROWS 12
 #endif
