@@ -317,6 +317,24 @@ __device__ __forceinline__ real div_ieee(real a, real b) {
     return a != real(0) ? q : (fabs(b) > real(0) ? a : real(__longlong_as_double(0x7ff8000000000000ll)));
 }
 
+// x / d, correctly rounded, from r = RN(1/d): q = x r, then q += r (x - d q)
+// twice.  The first correction leaves q within an ulp of x / d; then x - d q is
+// exact and the second rounds correctly (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990,
+// whose theorem asks for a correctly rounded reciprocal and no underflow).
+// Five operations where a division takes its whole latency of 148 cycles.
+// It holds for x that pass quot_rcp_range (zero, or |x| in 2^+-896) and d in
+// 2^+-100; outside, the division.
+__device__ __forceinline__ double quot_rcp(double x, double d, double r) {
+    double q = x * r;
+    q = fma(fma(-d, q, x), r, q);
+    return fma(fma(-d, q, x), r, q);
+}
+__device__ __forceinline__ bool quot_rcp_range(double x) {
+    const unsigned e = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return e - ((1023u - 896u) << 20) < (2u * 896u) << 20 || x == 0.0;
+}
+
 // Arithmetic policy of a kernel build: IEEE division and square root in the
 // reference-order build (bit-identical to the CPU restatement), Newton
 // reciprocals and roots in the contracted build.

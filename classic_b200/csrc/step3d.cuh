@@ -127,25 +127,7 @@ using MethodMC3D = Method3D<2, 2, 4>;  // transverse_waves 22, MC on both waves
 
 constexpr int NT3P = 2 * NT3;
 
-// x / d, correctly rounded, from r = RN(1/d): q = x r, then q += r (x - d q)
-// twice.  The first correction leaves q within an ulp of x / d; then x - d q is
-// exact and the second rounds correctly (Markstein, "Computation of elementary
-// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990,
-// whose theorem asks for a correctly rounded reciprocal and no underflow).
-// Five operations where a division takes its whole latency of 148 cycles; the
-// sums d = Z + Z' repeat over the splits, so a ring element's two reciprocals
-// serve sixteen.  `in` says that x and d are far enough from the ends of the
-// exponent range (|x| in 2^+-896, d in 2^+-100); outside it, the division.
-__device__ __forceinline__ double quot3(double x, double d, double r) {
-    double q = x * r;
-    q = fma(fma(-d, q, x), r, q);
-    return fma(fma(-d, q, x), r, q);
-}
-__device__ __forceinline__ bool quot3_range(double x) {
-    const unsigned e = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    return e - ((1023u - 896u) << 20) < (2u * 896u) << 20 || x == 0.0;
-}
-// the quotients outside that range, out of line: they hardly ever run
+// the quotients outside quot_rcp's range, out of line: they hardly ever run
 template <class S>
 __device__ __noinline__ typename S::Split split3_far(typename S::real xp, typename S::real zb, typename S::real cb,
                                                      typename S::real zm, typename S::real za,
@@ -365,8 +347,8 @@ __device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::rea
         const real* Cp = plane(pos, 1);
         const real* Rp = plane(pos, 2 + H);  // 1 / (Z + Z_next) along the own direction
         const real zb = Zp[-OWNS + w * OTHS], zm = Zp[w * OTHS], za = Zp[OWNS + w * OTHS];
-        const real b1 = -quot3(xp, zb + zm, Rp[-OWNS + w * OTHS]);
-        const real b2 = quot3(xp, zm + za, Rp[w * OTHS]);
+        const real b1 = -quot_rcp(xp, zb + zm, Rp[-OWNS + w * OTHS]);
+        const real b2 = quot_rcp(xp, zm + za, Rp[w * OTHS]);
         const real c1 = Cp[-OWNS + w * OTHS] * b1, c2 = Cp[OWNS + w * OTHS] * b2;
         return Split{c1 * zb, -c1, c2 * za, c2};
     };
@@ -492,7 +474,7 @@ __device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::rea
             // ---- the four rpt3 splits of interface p+1, side by side (their
             // quotients overlap): A-dq and cqxx at cell p, A+dq and cqxx at p+1
             if (m3 > 0) {
-                if (near && quot3_range(amB[0]) && quot3_range(apB[0]) && quot3_range(cq[0])) {
+                if (near && quot_rcp_range(amB[0]) && quot_rcp_range(apB[0]) && quot_rcp_range(cq[0])) {
                     ma = split_near(amB[0], L, 0);
                     mp = split_near(apB[0], R, 0);
                     if (m3 == 2) {
@@ -535,7 +517,7 @@ __device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::rea
                 const real y1 = *xplane(0, 1 - H, 0), y3 = *xplane(0, 1 - H, 1);
                 const real y0 = *xplane(1, 1 - H, 0), y2 = *xplane(1, 1 - H, 1);
                 Split tpm, tmm;
-                if (near && quot3_range(y0) && quot3_range(y1) && quot3_range(y2) && quot3_range(y3)) {
+                if (near && quot_rcp_range(y0) && quot_rcp_range(y1) && quot_rcp_range(y2) && quot_rcp_range(y3)) {
                     tpm = split_near(y1, L, 1);
                     tmm = split_near(y3, L, -1);
                     tpp = split_near(y0, R, 1);
