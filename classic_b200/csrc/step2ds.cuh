@@ -350,6 +350,10 @@ __device__ __forceinline__ void split2_rows(const Step2Args<S>& A, const SplitCo
         ycfl(rfirst + 1, sy, aux_p, aux_t);
     }
 
+    // two rows a turn where the registers allow (a constant-speed solver's rolling
+    // window then needs fewer copies: Strang 1024^2 54.3 -> 52.7 us a step)
+    constexpr int TURN = KNOWN ? 2 : 1;
+#pragma unroll TURN
     for (int t = rfirst + 2; t <= rlast && !failed; ++t) {
         if (!wait_row(t)) { failed = true; fail_row = t; }
         if (__any_sync(FULL, failed)) { failed = true; break; }
