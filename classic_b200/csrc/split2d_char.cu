@@ -63,10 +63,18 @@ struct CharSplitRunner : Runner {
     }
 };
 
-// MC on both waves compiled in; any other limiters read at run time
+// One limiter on both waves compiled in; two different ones, none and
+// Beam-Warming read at run time, a switch in every limited strength (Strang,
+// 2048^2, us a step: FP64 minmod 128 -> 53, superbee 135 -> 61, van Leer 138 ->
+// 63; FP32 62 -> 35, 64 -> 38, 66 -> 40)
 template <typename real, int BCM, bool STRANG>
 std::unique_ptr<Runner> pick_lim(int l1, int l2) {
-    if (l1 == 4 && l2 == 4) return std::unique_ptr<Runner>(new CharSplitRunner<real, 4, BCM, STRANG>());
+    if (l1 == l2) {
+        if (l1 == 1) return std::unique_ptr<Runner>(new CharSplitRunner<real, 1, BCM, STRANG>());
+        if (l1 == 2) return std::unique_ptr<Runner>(new CharSplitRunner<real, 2, BCM, STRANG>());
+        if (l1 == 3) return std::unique_ptr<Runner>(new CharSplitRunner<real, 3, BCM, STRANG>());
+        if (l1 == 4) return std::unique_ptr<Runner>(new CharSplitRunner<real, 4, BCM, STRANG>());
+    }
     return std::unique_ptr<Runner>(new CharSplitRunner<real, -1, BCM, STRANG>());
 }
 
