@@ -65,11 +65,12 @@ __device__ __forceinline__ double warp_max_nonneg(double c) {
     return __longlong_as_double((long long)(((unsigned long long)mh << 32) | ml));
 }
 
-// Methods compiled in: MC on every wave at order 2 without capacity, f-waves
-// or source (taken branches cost a lone warp 30-100 cycles each), and one that
-// reads everything at run time.
-struct Method1MC {
-    static constexpr int lim = 4;
+// Methods compiled in: one limiter on every wave at order 2 without capacity,
+// f-waves or source (taken branches cost a lone warp 30-100 cycles each; 800
+// cells, us a frame: minmod 213 -> 174, van Leer 226 -> 188), and one that reads everything at run time.
+template <int LIM>
+struct Method1 {
+    static constexpr int lim = LIM;
 };
 struct Method1Any {
     static constexpr int lim = -1;
