@@ -416,6 +416,14 @@ struct const_speed { static constexpr bool value = false; };
 template <class S>
 struct const_speed<S, decltype((void)&S::top_speed)> { static constexpr bool value = true; };
 
+// Courant number of a sweep whose faces all carry the speeds -c and c: the larger
+// of dt/dx s and -dt/dx s over both is |dt/dx| c, for a backward step (dt < 0)
+// too.  Zero for a NaN, which a fold over faces drops.
+__device__ __forceinline__ double sweep_cfl(double dtdx, double c) {
+    const double v = fabs(dtdx * c);
+    return v > 0.0 ? v : 0.0;
+}
+
 // min(x, 0) and max(x, 0), fmin's and fmax's values (zero for a NaN)
 template <typename real>
 __device__ __forceinline__ real neg_part(real x) { return x < real(0) ? x : real(0); }

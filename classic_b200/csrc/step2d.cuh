@@ -218,6 +218,12 @@ __device__ __forceinline__ StepConsts<S> step_consts(const Step2Args<S>& A, cons
     return k;
 }
 
+// Courant number of a step whose speeds are one constant (S::top_speed)
+template <class S>
+__device__ __forceinline__ double const_cfl(const S& s, const StepConsts<S>& K) {
+    return fold_cfl(sweep_cfl(K.dtdx_d, s.top_speed()), sweep_cfl(K.dtdy_d, s.top_speed()));
+}
+
 template <class S, class M, bool SRC = false>
 __device__ __forceinline__ void step2_rows(const Step2Args<S>& A, const StepConsts<S>& K,
                                            const int strip, const int r0, const int nr,
@@ -842,9 +848,8 @@ step2_kernel(const __grid_constant__ Step2Args<S> A) {
     }
 
     if constexpr (const_speed<S>::value && M::capa == 0) {
-        const double cd = A.solver.top_speed();
-        const double v = fold_cfl(K.dtdx_d * cd, K.dtdy_d * cd);
-        cta_count_and_control(ctl, failed, [&](const CtlIn&) { return v > 0.0 ? v : 0.0; });
+        const double v = const_cfl(A.solver, K);
+        cta_count_and_control(ctl, failed, [&](const CtlIn&) { return v; });
     } else {
         __shared__ double red[WARPS2D];
         cta_cfl_and_control(ctl, cfl, red);
@@ -945,7 +950,7 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
         double cfl = 0.0;
         step2_rows<S, M>(A, K, strip, r0, nr, ring, bars, seq_base, cfl, failed);
         if constexpr (const_speed<S>::value && M::capa == 0)
-            cfl = fold_cfl(K.dtdx_d * A.solver.top_speed(), K.dtdy_d * A.solver.top_speed());
+            cfl = const_cfl(A.solver, K);
         for (int o = 16; o > 0; o >>= 1) cfl = fmax(cfl, __shfl_xor_sync(FULL, cfl, o));
         if (lane == 0) {
             if (failed) atomicOr(B.err, CTL_ERR_TMA_TIMEOUT);

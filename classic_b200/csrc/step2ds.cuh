@@ -598,9 +598,9 @@ split2_kernel(const __grid_constant__ Step2Args<S> A) {
     }
     if constexpr (const_speed<S>::value && M::capa == 0) {
         const double cd = A.solver.top_speed();
-        auto known = [&](double v) { return v > 0.0 ? v : 0.0; };
         cta_count_and_control(ctl, failed, [&](const CtlIn& in) {
-            return split_cfl(in, STRANG ? 3 : 2, known(K.dtdx_a_d * cd), known(K.dtdy_d * cd), known(K.dtdx_c_d * cd));
+            return split_cfl(in, STRANG ? 3 : 2, sweep_cfl(K.dtdx_a_d, cd), sweep_cfl(K.dtdy_d, cd),
+                             sweep_cfl(K.dtdx_c_d, cd));
         });
     } else {
         __shared__ double red[3 * WARPS2D];

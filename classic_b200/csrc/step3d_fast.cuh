@@ -497,7 +497,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         s3 = so;
     }
     const double cd = (double)cmax;
-    const double cfl = fmax(fmax((dt / a.d[0]) * cd, (dt / a.d[1]) * cd), (dt / a.d[2]) * cd);
+    const double cfl = fmax(fmax(sweep_cfl(dt / a.d[0], cd), sweep_cfl(dt / a.d[1], cd)), sweep_cfl(dt / a.d[2], cd));
     cta_cfl_and_control(ctl, cfl, red);
 }
 
