@@ -546,8 +546,8 @@ step2_char_kernel(const __grid_constant__ CharArgs<real> A) {
     }
     // Courant number as flux2 forms it (dt/dx * c over x-interfaces, dt/dy * c
     // over y-interfaces; the speeds are constant)
-    const double cfl = fmax(dtdx_d * (double)c, dtdy_d * (double)c);
-    cta_count_and_control(ctl, failed, [&](const CtlIn&) { return cfl > 0.0 || cfl != cfl ? cfl : 0.0; });
+    const double cfl = fmax(fabs(dtdx_d * (double)c), fabs(dtdy_d * (double)c));
+    cta_count_and_control(ctl, failed, [&](const CtlIn&) { return cfl; });
 }
 
 }  // namespace clawb200

@@ -337,9 +337,8 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
     // the sweeps' Courant numbers as step2ds forms them over every interface
     // (dt_sweep/dx c; the speeds are constant), combined as dimsp2 combines them
     const double cd = (double)c;
-    auto known = [&](double v) { return v > 0.0 || v != v ? v : 0.0; };
     cta_count_and_control(ctl, failed, [&](const CtlIn& in) {
-        return split_cfl(in, STRANG ? 3 : 2, known(dtdx_a_d * cd), known(dtdy_d * cd), known(dtdx_c_d * cd));
+        return split_cfl(in, STRANG ? 3 : 2, fabs(dtdx_a_d * cd), fabs(dtdy_d * cd), fabs(dtdx_c_d * cd));
     });
 }
 
