@@ -281,7 +281,7 @@ int claw_batch_advance(claw_batch* b, double tstart, double tend, const double* 
         if (!info[k] && cfg.capa_index > cfg.num_aux) info[k] = 5;
         if (!info[k] && cfg.order < cfg.transverse_waves) info[k] = 6;
         c->maxn = maxn;
-        c->done = (info[k] != 0 || maxn == 0) ? 1 : 0;
+        c->done = (info[k] != 0 || maxn <= 0) ? 1 : 0;
         if (!c->done && c->told + c->dt > tend && tstart < tend) c->dt = tend - c->told;
         active += c->done ? 0 : 1;
     }

@@ -693,7 +693,7 @@ int claw_advance(claw_handle* h, double tstart, double tend, double dt_initial, 
         if (!ok) info = 6;
     }
     c->maxn = maxn;
-    c->done = (info != 0 || maxn == 0) ? 1 : 0;
+    c->done = (info != 0 || maxn <= 0) ? 1 : 0;  // the reference's loop runs to maxn: no step below 1
     if (!c->done && c->told + c->dt > tend && tstart < tend) c->dt = tend - c->told;
     int rc = push_ctl(h);
     if (rc) return rc;
