@@ -79,8 +79,7 @@ struct claw_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     long long launches = 0;
     int device = 0;
-    double* stage = nullptr;  // dense device copy of one instance's q (fieldcopy.cuh)
-    size_t stage_n = 0;
+    Stage stage;  // dense device copy of one instance's q (fieldcopy.cuh)
 
     // Frees everything the batch holds, so an error part-way through
     // claw_batch_create leaks nothing.
@@ -94,7 +93,6 @@ struct claw_batch {
                 if (gg.q[s]) cudaFree(gg.q[s]);
             if (gg.aux) cudaFree(gg.aux);
         }
-        if (stage) cudaFree(stage);
         if (ctl_d) cudaFree(ctl_d);
         if (ctl_h) cudaFreeHost(ctl_h);
         if (flags_d) cudaFree(flags_d);
@@ -182,7 +180,7 @@ int claw_batch_create(const claw_config* cfgs, int count, claw_batch** out) {
         const size_t n = (size_t)g.meqn * g.mx * g.my;
         if (n * sizeof(double) <= STAGE_BYTES) largest = std::max(largest, n);
     }
-    int rc = make_stage(&b->stage, &b->stage_n, {largest}, false);
+    int rc = make_stage(b->stage, {largest}, false);
     if (rc) return rc;
     rc = b->runner->prepare(b->g, cfgs, b->ctl_d, b->flags_d, b->flags_d + 1);
     if (rc) return rc;
@@ -200,7 +198,7 @@ static int batch_fields(claw_batch* b, int k, double* host, bool to_device) {
     const Geometry& g = b->g[k];
     const int cur = b->ctl_h[k].cur;
     return copy_fields(static_cast<double*>(g.q[cur]), g.ld, g.fstride, host, g.meqn, g.mx, g.my, b->stage,
-                       b->stage_n, to_device, b->stream);
+                       to_device, b->stream);
 }
 
 int claw_batch_set_q(claw_batch* b, int k, const double* q) {

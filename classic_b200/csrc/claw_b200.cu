@@ -369,8 +369,7 @@ struct claw_handle {
     int cur = 0;
     cudaStream_t stream = nullptr;
     ClawCtl* ctl_h = nullptr;  // pinned mirror
-    double* stage = nullptr;   // dense device copy of a field block (fieldcopy.cuh)
-    size_t stage_n = 0;
+    Stage stage;               // dense device copy of a field block (fieldcopy.cuh)
     std::unique_ptr<Runner> runner;
     cudaGraphExec_t gexec = nullptr;
     int gsteps = 0;
@@ -395,7 +394,6 @@ struct claw_handle {
         if (g.aux_base) cudaFree(g.aux_base);
         if (totals_scratch) cudaFree(totals_scratch);
         if (g.ctl) cudaFree(g.ctl);
-        if (stage) cudaFree(stage);
         if (ctl_h) cudaFreeHost(ctl_h);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
@@ -518,7 +516,7 @@ int claw_create(const claw_config* cfg, claw_handle** out) {
     std::memset(h->ctl_h, 0, sizeof(ClawCtl));
     h->ctl_h->done = 1;
     CUDA_TRY(cudaMemcpyAsync(g.ctl, h->ctl_h, sizeof(ClawCtl), cudaMemcpyHostToDevice, h->stream));
-    rc = make_stage(&h->stage, &h->stage_n, {q_count(g), aux_count(g)}, g.es == 4);
+    rc = make_stage(h->stage, {q_count(g), aux_count(g)}, g.es == 4);
     if (rc) return rc;
     h->runner = g.es == 8 ? make_runner<double>(*cfg) : make_runner<float>(*cfg);
     if (!h->runner) return fail(CLAW_E_UNSUPPORTED, "no kernel for solver %d", cfg->solver_id);
@@ -545,9 +543,9 @@ static int copy_block(claw_handle* h, void* dev, long long pitch, long long fpit
     double* hp = const_cast<double*>(host);  // written only when !in
     if (h->g.es == 8)
         return copy_fields(static_cast<double*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage,
-                           h->stage_n, in, h->stream);
-    return copy_fields(static_cast<float*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage,
-                       h->stage_n, in, h->stream);
+                           in, h->stream);
+    return copy_fields(static_cast<float*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage, in,
+                       h->stream);
 }
 
 int claw_set_q(claw_handle* h, const double* q) {

@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <initializer_list>
+#include <mutex>
 
 #include "common.cuh"
 #include "host.h"
@@ -25,6 +26,18 @@
 namespace clawb200 {
 
 constexpr size_t STAGE_BYTES = 8u << 20;
+
+// The buffer of an object, n doubles.  Copies through it are two operations on
+// the object's stream; `order` keeps them together, so that the stream's order
+// keeps the copies of several host threads apart.
+struct Stage {
+    double* buf = nullptr;
+    size_t n = 0;
+    std::mutex order;
+    ~Stage() {
+        if (buf) cudaFree(buf);
+    }
+};
 
 // one element a thread, rows over blockIdx.y; row r of field m is dense row
 // m*rows + r
@@ -42,11 +55,11 @@ copy_rows(double* dense, real* dev, long long pitch, long long fpitch, long long
     }
 }
 
-// Queue the copy of nfields fields on the stream (the caller waits for it).
-// `stage` holds stage_n doubles; FP64 blocks of more go directly.
+// Queue the copy of nfields fields on the object's stream (the caller waits for
+// it).  FP64 blocks larger than the buffer go directly.
 template <class real>
 int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int nfields, long long width,
-                long long rows, double* stage, size_t stage_n, bool in, cudaStream_t st) {
+                long long rows, Stage& stage, bool in, cudaStream_t st) {
     const long long nrows = nfields * rows;
     const size_t n = (size_t)nrows * width;
     const auto kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
@@ -57,7 +70,7 @@ int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int 
             else CUDA_TRY(cudaMemcpyAsync(host, dev, n * 8, kind, st));
             return 0;
         }
-        if (nfields == 1 || rows == 1 || n > stage_n || small_in) {
+        if (nfields == 1 || rows == 1 || n > stage.n || small_in) {
             for (int m = 0; m < nfields; ++m) {
                 real* d = dev + m * fpitch;
                 double* hp = host + (size_t)m * width * rows;
@@ -68,12 +81,13 @@ int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int 
         }
     }
     const dim3 grid((unsigned)((width + 255) / 256), (unsigned)std::min(nrows, 65535ll));
+    std::lock_guard<std::mutex> together(stage.order);
     if (in) {
-        CUDA_TRY(cudaMemcpyAsync(stage, host, n * 8, kind, st));
-        copy_rows<real, true><<<grid, 256, 0, st>>>(stage, dev, pitch, fpitch, width, rows, nrows);
+        CUDA_TRY(cudaMemcpyAsync(stage.buf, host, n * 8, kind, st));
+        copy_rows<real, true><<<grid, 256, 0, st>>>(stage.buf, dev, pitch, fpitch, width, rows, nrows);
     } else {
-        copy_rows<real, false><<<grid, 256, 0, st>>>(stage, dev, pitch, fpitch, width, rows, nrows);
-        CUDA_TRY(cudaMemcpyAsync(host, stage, n * 8, kind, st));
+        copy_rows<real, false><<<grid, 256, 0, st>>>(stage.buf, dev, pitch, fpitch, width, rows, nrows);
+        CUDA_TRY(cudaMemcpyAsync(host, stage.buf, n * 8, kind, st));
     }
     CUDA_TRY(cudaGetLastError());
     return 0;
@@ -81,19 +95,19 @@ int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int 
 
 // The buffer for blocks of these element counts: FP32 fields need the largest,
 // FP64 ones take the largest within STAGE_BYTES, and do without when memory is short.
-inline int make_stage(double** stage, size_t* stage_n, std::initializer_list<size_t> counts, bool needed) {
+inline int make_stage(Stage& stage, std::initializer_list<size_t> counts, bool needed) {
     size_t n = 0;
     for (size_t c : counts)
         if (needed || c * 8 <= STAGE_BYTES) n = std::max(n, c);
     if (!n) return 0;
-    const cudaError_t e = cudaMalloc(stage, n * 8);
+    const cudaError_t e = cudaMalloc(&stage.buf, n * 8);
     if (e != cudaSuccess) {
-        *stage = nullptr;
+        stage.buf = nullptr;
         cudaGetLastError();
         if (needed) return fail(CLAW_E_CUDA, "%s", cudaGetErrorString(e));
         return 0;
     }
-    *stage_n = n;
+    stage.n = n;
     return 0;
 }
 
