@@ -124,7 +124,8 @@ struct Runner1D : Runner {
         constexpr int most = step1_threads<S>();
         threads = std::min(most, 32 * ((g.mx + STRIP1 - 1) / STRIP1 + 1));
         const long long bytes = step1_smem_bytes<S>(g.mx);
-        const bool smq = bytes + 1024 <= optin;
+        const int limit = optin - 1024;  // (the kernel's static arrays are below 1 KB)
+        const bool smq = bytes <= limit;
         smem = smq ? (int)bytes : 0;
         const bool plain = cfg.order == 2 && cfg.capa_index == 0 && !cfg.use_fwaves && args.src_split == 0;
         const int lim = plain && all_limiters(cfg, cfg.limiter[0]) ? cfg.limiter[0] : 0;
@@ -137,7 +138,8 @@ struct Runner1D : Runner {
             if (lim == 3) pick<Method1<3>>();
             if (lim == 4) pick<Method1<4>>();
         }
-        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        // the kernel's attribute, not this handle's: the same for every grid
+        if (smq) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
         return 0;
     }
 
