@@ -103,27 +103,28 @@ struct Step3fArgs {
     int tilesx, tilesy, seglen;
 };
 
-template <typename real, int LIM, bool TRANS>
-__global__ void __launch_bounds__(32 * Step3fShape<real>::rows, Step3fShape<real>::minb)
-step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
+// Where a plane's q and aux lie in global memory, and whether w changes its sign
+// (1) or takes the piston's (2) there.
+template <typename real>
+struct Plane3f {
+    const real *q, *aux;
+    int w;
+};
+
+// zt holds planes t-1 .. t+4 at [pos & 7].  One thread fills an entry a plane
+// ahead; each thread for itself, three times a plane, it cost the FP32 kernel,
+// bound by issue, 5 % (192^3 314 -> 298 us a step; FP64 517 -> 509).
+// UNIT: the tile takes 2^e as its unit of impedance and pressure.
+template <typename real, int LIM, bool TRANS, bool UNIT>
+__device__ __forceinline__ void step3f_march(const Step3fArgs<real>& A, const StepHead& hd, unsigned char* smem_raw,
+                                             double* red, Plane3f<real>* zt, int e) {
     using Sh = Step3fShape<real>;
     constexpr int ROWS = Sh::rows, PL = Sh::pl;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int kUnroll = CLAW_STEP3F_UNROLL;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double red[ROWS];
-    // planes t-1 .. t+4 at [pos & 7]: where q and aux lie in global memory, and
-    // whether w changes its sign (1) or takes the piston's (2) there.  One thread
-    // fills an entry a plane ahead; each thread for itself, three times a plane, it
-    // cost the FP32 kernel, bound by issue, 5 % (192^3 314 -> 298 us a step; FP64
-    // 517 -> 509)
-    __shared__ struct { const real *q, *aux; int w; } zt[8];
     const Sweep3Args<real>& a = A.g;
     ClawCtl* ctl = a.ctl;
-    grid_dependency_sync();
     const double tbc = *(volatile double*)&ctl->told;
-    const StepHead hd = step_head(ctl);
-    if (hd.done) return;
     const int cur = hd.cur;
     const double dt = hd.dt;
     const real* __restrict__ qold = a.q[cur];
@@ -150,6 +151,18 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     const int j0 = 1 + by * Sh::outy;            // first row written
     const int j = j0 - 1 + r;                    // this warp's row
     const bool out = lane >= 2 && lane < 30 && i <= mx && r >= 1 && r < ROWS - 1 && j <= my;
+
+    // zu takes Z and pressure differences into the unit, pu takes pressure
+    // increments out of it, `one` is the 1 that u's part has beside Z Z'
+    // (negligible, or all there is, where the bound takes effect)
+    real zu = real(1), pu = real(1), one = real(1);
+    if constexpr (UNIT) {
+        zu = __int_as_float((127 - e) << 23);
+        pu = __int_as_float((127 + e) << 23);
+        one = fminf(zu * zu, 0x1p100f);
+    }
+    const real txp = UNIT ? tx * pu : tx, typ = UNIT ? ty * pu : ty, tzp = UNIT ? tz * pu : tz;
+    auto pdiff = [&](real x, real y) { return UNIT ? (x - y) * zu : x - y; };
 
     // source cell of a column and a row under the boundary conditions; cells
     // past the last ghost layer repeat it (nothing written depends on them)
@@ -210,6 +223,13 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         cp_async_el(d + PL + own, q + qxy + 2 * a.fstride);
         if (edge) cp_async_el(d + PL + hal, q + qxh + 2 * a.fstride);
     };
+    // own Z's of a landed plane into the tile's unit (before the barrier that publishes them)
+    auto to_unit = [&](int so) {
+        if (UNIT) {
+            ring[so + PL + own] *= zu;
+            if (edge) ring[so + PL + hal] *= zu;
+        }
+    };
     // w at plane pos from its stored value (the walls' and the piston's sign)
     auto wbc = [&](int pos, real w) {
         const int f = zt[pos & 7].w;
@@ -251,10 +271,14 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     issue_uv(t0);
     // the w copies of planes t0-1 and t0 must not land after those of t0+1 and t0+2
     cp_async_wait_all();
+    to_unit(sm);
+    to_unit(s0);
     __syncthreads();
     issue_pzc(t0 + 1, s1);
     issue_pzc(t0 + 2, s2);
     cp_async_wait_all();
+    to_unit(s1);
+    to_unit(s2);
     __syncthreads();
     {
         const real pA = ring[sm + own], zA = ring[sm + PL + own];
@@ -262,10 +286,10 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         const real pC = ring[s1 + own], zC = ring[s1 + PL + own];
         rz = rcp_newton(zA + zB);
         rz1 = rcp_newton(zB + zC);
-        a2zm = (zA * (w0 - wm) + (pB - pA)) * rz;
-        a1z = (zC * (w1 - w0) - (pC - pB)) * rz1;
-        a2z = (zB * (w1 - w0) + (pC - pB)) * rz1;
-        g0 = rcp_newton(real(1) + zB * zB);
+        a2zm = (zA * (w0 - wm) + pdiff(pB, pA)) * rz;
+        a1z = (zC * (w1 - w0) - pdiff(pC, pB)) * rz1;
+        a2z = (zB * (w1 - w0) + pdiff(pC, pB)) * rz1;
+        g0 = rcp_newton(one + zB * zB);
     }
     real t2zm = 0, cpzm = 0, cwzm = 0;          // z interface t-1/2: right-going fluctuation, correction flux
     real cmax = 0;
@@ -293,7 +317,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         const real zl = P[PL + lm], cl = P[2 * PL + lm];
         real rx, a1x, a2x;
         {
-            const real du = u - __shfl_up_sync(FULL, u, 1), dp = p - P[lm];
+            const real du = u - __shfl_up_sync(FULL, u, 1), dp = pdiff(p, P[lm]);
             rx = rcp_newton(zl + z);
             a1x = (z * du - dp) * rx;
             a2x = (zl * du + dp) * rx;
@@ -303,7 +327,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         {
             real vb = UV[PL + own - 32];
             if (negb) vb = -vb;
-            const real dv = v - vb, dp = p - P[own - 32];
+            const real dv = v - vb, dp = pdiff(p, P[own - 32]);
             ry = rcp_newton(zb + z);
             a1y = (z * dv - dp) * ry;
             a2y = (zb * dv + dp) * ry;
@@ -318,7 +342,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
             real va = UV[PL + own + 32];
             if (negh) va = -va;
             const real za = P[PL + own + 32];
-            SA1[own + 32] = (za * (va - v) - (P[own + 32] - p)) * rcp_newton(z + za);
+            SA1[own + 32] = (za * (va - v) - pdiff(P[own + 32], p)) * rcp_newton(z + za);
         }
         // z interface t+3/2
         const real z1 = ring[s1 + PL + own], c1 = ring[s1 + 2 * PL + own];
@@ -326,18 +350,18 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         const real w2 = wbc(t + 2, uvw[(par * 3 + 2) * PL + own]);
         real a1zn, a2zn, rz2;
         {
-            const real dw = w2 - w1, dp = ring[s2 + own] - ring[s1 + own];
+            const real dw = w2 - w1, dp = pdiff(ring[s2 + own], ring[s1 + own]);
             rz2 = rcp_newton(z1 + z2);
             a1zn = (z2 * dw - dp) * rz2;
             a2zn = (z1 * dw + dp) * rz2;
         }
-        const real g1 = rcp_newton(real(1) + z1 * z1);
+        const real g1 = rcp_newton(one + z1 * z1);
         __syncthreads();
         // ---------------------------- B: limited waves, x and z sums
         real bp = p, bu = u, bv = v, bw = w0;
         real Xx, Yx, Xz, Yz;
         {
-            const real h = real(1) + zl * z;
+            const real h = one + zl * z;
             const real n1 = __shfl_down_sync(FULL, a1x, 1) * (h * __shfl_up_sync(FULL, g0, 1));
             const real n2 = __shfl_up_sync(FULL, a2x, 1) * (h * g0);
             const real e1 = coef(cl, tx) * lim_a(a1x, n1), e2 = coef(c, tx) * lim_b(a2x, n2);
@@ -346,20 +370,20 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
             const real tr = __shfl_down_sync(FULL, ta, 1);
             const real sp = z * (tb + tr), su = tb - tr;
             const real dp = __shfl_down_sync(FULL, cp, 1) - cp, du = __shfl_down_sync(FULL, cu, 1) - cu;
-            bp -= tx * (sp + dp);
+            bp -= txp * (sp + dp);
             bu -= tx * (su + du);
             Xx = -tx * (real(0.5) * sp + xd * dp);
             Yx = sp + yd * dp;
         }
         {
-            const real h = real(1) + z * z1;
+            const real h = one + z * z1;
             const real e1 = coef(c, tz) * lim_a(a1z, a1zn * (h * g0));
             const real e2 = coef(c1, tz) * lim_b(a2z, a2zm * (h * g1));
             const real cp = z1 * e2 - z * e1, cw = e1 + e2;
             const real ta = c * a1z;
             const real sp = z * (t2zm + ta), sw = t2zm - ta;
             const real dp = cp - cpzm, dw = cw - cwzm;
-            bp -= tz * (sp + dp);
+            bp -= tzp * (sp + dp);
             bw -= tz * (sw + dw);
             Xz = -tz * (real(0.5) * sp + xd * dp);
             Yz = sp + yd * dp;
@@ -369,7 +393,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
         }
         real cpy = 0, cvy = 0, tby = 0;
         if (r >= 1) {  // y interface below this row
-            const real h = real(1) + zb * z;
+            const real h = one + zb * z;
             const real n1 = SA1[own + 32] * (h * SG[own - 32]);
             const real n2 = SA2[own - 32] * (h * g0);
             const real e1 = coef(cb, ty) * lim_a(a1y, n1), e2 = coef(c, ty) * lim_b(a2y, n2);
@@ -392,7 +416,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
             const real tr = ST1[own + 32];
             const real sp = z * (tby + tr), sv = tby - tr;
             const real dp = SCP[own + 32] - cpy, dv = SCV[own + 32] - cvy;
-            bp -= ty * (sp + dp);
+            bp -= typ * (sp + dp);
             bv -= ty * (sv + dv);
             Xy = -ty * (real(0.5) * sp + xd * dp);
             Yy = sp + yd * dp;
@@ -445,6 +469,7 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
             SE[4 * PL + own] = exyu;
         }
         cp_async_wait_all();
+        if (t + 3 <= k1 + 1) to_unit(s3);
         __syncthreads();
         // -------------------------------------------- D: plane t-1
         real op = SB[own], ou = SB[PL + own], ov = SB[2 * PL + own], ow = SB[3 * PL + own];
@@ -458,7 +483,8 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
             SB[4 * PL + own] = nexzp;
             SB[5 * PL + own] = nexzu;
             nfzw += f6 * ((exzw - __shfl_up_sync(FULL, exzw, 1)) + (eyzw - SE[2 * PL + own - 32]));
-            op -= ((fxp - __shfl_up_sync(FULL, fxp, 1)) + (fyp - SE[own - 32])) + (nfzp - fzp);
+            const real dfp = ((fxp - __shfl_up_sync(FULL, fxp, 1)) + (fyp - SE[own - 32])) + (nfzp - fzp);
+            op -= UNIT ? pu * dfp : dfp;
             ou -= fxu - __shfl_up_sync(FULL, fxu, 1);
             ov -= fyv - SE[PL + own - 32];
             ow -= nfzw - fzw;
@@ -499,6 +525,33 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     const double cd = (double)cmax;
     const double cfl = fmax(fmax(sweep_cfl(dt / a.d[0], cd), sweep_cfl(dt / a.d[1], cd)), sweep_cfl(dt / a.d[2], cd));
     cta_cfl_and_control(ctl, cfl, red);
+}
+
+template <typename real, int LIM, bool TRANS>
+__global__ void __launch_bounds__(32 * Step3fShape<real>::rows, Step3fShape<real>::minb)
+step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double red[Step3fShape<real>::rows];
+    __shared__ Plane3f<real> zt[8];
+    grid_dependency_sync();
+    const StepHead hd = step_head(A.g.ctl);
+    if (hd.done) return;
+    // FP32: products of impedances (1 + Z Z', r r' K) leave its range beyond Z =
+    // 2^+-62.  A tile whose first cell lies beyond 2^+-40 takes a power of two
+    // near that Z as its unit of impedance and pressure, which changes exponents
+    // only.  A march of its own: the few multiplications cost the others 2.8 %
+    // (161x130x147 1426 -> 1466 us a frame).
+    if constexpr (sizeof(real) == 4) {
+        using Sh = Step3fShape<real>;
+        const int bx = blockIdx.x % A.tilesx, by = blockIdx.x / A.tilesx % A.tilesy, seg = blockIdx.x / A.tilesx / A.tilesy;
+        const real z = A.g.aux[(2 + bx * Sh::outx) + (2 + by * Sh::outy) * A.g.as[1] + (2 + seg * A.seglen) * A.g.as[2]];
+        const int e = ((__float_as_int(z) >> 23) & 255) - 127;
+        if (abs(e) > 40 && abs(e) < 127) {
+            step3f_march<real, LIM, TRANS, true>(A, hd, smem_raw, red, zt, e);
+            return;
+        }
+    }
+    step3f_march<real, LIM, TRANS, false>(A, hd, smem_raw, red, zt, 0);
 }
 
 }  // namespace clawb200
