@@ -290,7 +290,8 @@ int claw_batch_advance(claw_batch* b, double tstart, double tend, const double* 
     const long long launches0 = b->launches;
     CUDA_TRY(cudaEventRecord(b->ev0, b->stream));
     if (active > 0) {
-        const int chunk = 16;
+        constexpr int chunk = 16;
+        static_assert(chunk % 2 == 0, "the launches' turns alternate from one replay to the next too");
         int rc = batch_graph(b, chunk);
         if (rc) return rc;
         for (;;) {

@@ -128,6 +128,7 @@ struct BatchRunnerT : BatchRunner {
     int nsm_ = 1, per_sm_ = 1;
 
     cudaError_t launch(cudaStream_t s) override {
+        b.turn ^= 1;
         return launch_step(step2_batch_kernel<S, M>, dim3(grid), dim3(32 * WARPS2D), smem, s, b);
     }
 };

@@ -81,12 +81,13 @@ __device__ __forceinline__ CtlIn ctl_in(const ClawCtl* c) {
 // Controller step: identical decisions to claw2's main loop.  Runs in exactly
 // one thread after every CTA of the step has published its Courant maximum
 // (cfl; its slot is the caller's to clear) and its error flag (err).  The next
-// launch sees the block when this grid is complete.
-__device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, double cfl, int err) {
+// launch sees the block when this grid is complete.  `stop` is what done becomes
+// when the call ends (the batch kernel's mark of the launch).
+__device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, double cfl, int err, int stop = 1) {
     c->ctas_done = 0u;
     c->cfl_last = cfl;
     if (err) {  // a device wait gave up: the step's output is incomplete
-        c->done = 1;
+        c->done = stop;
         return;
     }
     if (s.mode == CTL_SINGLE) {
@@ -95,7 +96,7 @@ __device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, doub
     }
     if (cfl != cfl) {  // NaN: stop instead of retrying forever
         c->err = err | CTL_ERR_NAN_CFL;
-        c->done = 1;
+        c->done = stop;
         return;
     }
     const double t = s.told + s.dt;
@@ -112,7 +113,7 @@ __device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, doub
         }
         c->n = s.n + 1;
         if (t >= s.tend || s.n + 1 >= s.maxn) {
-            c->done = 1;
+            c->done = stop;
         } else {
             c->told = t;
             if (t + dt > s.tend && s.tstart < s.tend) dt = s.tend - t;
@@ -125,7 +126,7 @@ __device__ __forceinline__ void ctl_finish_step(ClawCtl* c, const CtlIn& s, doub
             c->dt = fmin(s.dt_max, s.dt * s.cfl_desired / cfl);
         } else {
             c->cflmax_seen = fmax(cfl, s.cflmax_seen);
-            c->done = 1;
+            c->done = stop;
         }
     }
 }

@@ -877,6 +877,7 @@ struct Step2Batch {
     int count;
     int nwarps;                // warps of the launch
     int min_rows;              // tile height: fewest rows a sharing warp takes
+    int turn;                  // 0 and 1 in alternate launches
     int* active;               // instances still advancing (polled by the host)
     int* err;                  // device error flags of the batch
 };
@@ -889,9 +890,16 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
     __shared__ int pre[BATCH_MAX + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     grid_dependency_sync();
-    // units of the active instances, then their prefix sums
-    for (int k = threadIdx.x; k < B.count; k += blockDim.x)
-        pre[k + 1] = *(volatile int*)&B.ctls[k].done ? 0 : B.units[k];
+    // units of the active instances, then their prefix sums.  Every CTA must see
+    // the same ones, however late it starts (other work may hold its SM), so an
+    // instance that ends in this launch counts to its end: it is marked 2 + turn,
+    // and the next launch, whose turn is the other, puts 1 for it.
+    for (int k = threadIdx.x; k < B.count; k += blockDim.x) {
+        volatile int* done = &B.ctls[k].done;
+        const int d = *done;
+        pre[k + 1] = d == 0 || d == 2 + B.turn ? B.units[k] : 0;
+        if (d == 3 - B.turn) *done = 1;
+    }
     __syncthreads();
     if (warp == 0) {
         int run = 0;
@@ -963,7 +971,7 @@ step2_batch_kernel(const __grid_constant__ Step2Batch<S> B) {
                 __threadfence();
                 const CtlIn in = ctl_in(ctl);
                 const int err = *(volatile int*)&ctl->err;
-                ctl_finish_step(ctl, in, take_cfl(&ctl->cfl_bits), err);
+                ctl_finish_step(ctl, in, take_cfl(&ctl->cfl_bits), err, 2 + B.turn);
                 if (*(volatile int*)&ctl->done) atomicSub(B.active, 1);
             }
         }
