@@ -396,15 +396,15 @@ int claw_batch_autotune(claw_batch* b, const double* dt_trial, int repeats, int*
     };
     const int maxc = b->runner->max_ctas_per_sm();
     float best = 1e30f, best_tail = 1e30f;
-    int best_ctas = maxc, best_rows = 48;
+    int best_ctas = maxc, best_rows = BATCH_SHORTEST;
     for (int ctas = maxc; ctas >= 1 && ctas >= maxc / 2; --ctas) {
-        b->runner->set_shape(1, ctas);
+        b->runner->set_shape(BATCH_SHORTEST, ctas);
         float t = 0.f;
         int rc = time_step(trial, n, &t);
         if (rc) return rc;
         if (t < best) { best = t; best_ctas = ctas; }
     }
-    const int rows_cand[] = {16, 24, 32, 48, 96, 192};
+    const int rows_cand[] = {BATCH_SHORTEST, 24, 32, 48, 96, 192};
     for (int rows : rows_cand) {
         b->runner->set_shape(rows, best_ctas);
         float t = 0.f;
@@ -412,11 +412,11 @@ int claw_batch_autotune(claw_batch* b, const double* dt_trial, int repeats, int*
         if (rc) return rc;
         if (t < best_tail) { best_tail = t; best_rows = rows; }
     }
-    b->runner->set_shape(1, best_ctas);  // the default height, kept where it is the fastest
-    float t1 = 0.f;
-    const int rc1 = time_step(tail, 1, &t1);
-    if (rc1) return rc1;
-    if (best_tail < t1) b->runner->set_shape(best_rows, best_ctas);
+    b->runner->set_shape(best_rows, best_ctas);
+    if (best_rows != BATCH_SHORTEST) {  // the full step's time in the shape that is kept
+        const int rc = time_step(trial, n, &best);
+        if (rc) return rc;
+    }
     if (b->gexec) {  // the captured time loop holds the old launch shape
         cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;

@@ -14,15 +14,20 @@
 
 namespace clawb200 {
 
+// The shortest tile height: no fewest rows, every resident warp takes a share
+// of them.
+constexpr int BATCH_SHORTEST = 16;
+
 struct BatchRunner {
     virtual ~BatchRunner() {}
     virtual int prepare(const std::vector<Geometry>& g, const claw_config* cfgs, ClawCtl* ctls,
                         int* active, int* err) = 0;
     virtual cudaError_t launch(cudaStream_t s) = 0;
-    // launch shape: tile height (rows per warp at least) and CTAs per SM
+    // launch shape: tile height (rows per warp at least, from BATCH_SHORTEST up)
+    // and CTAs per SM
     virtual void set_shape(int min_rows, int ctas_per_sm) = 0;
     virtual int max_ctas_per_sm() const = 0;
-    int min_rows = 1, ctas_per_sm = 0;
+    int min_rows = BATCH_SHORTEST, ctas_per_sm = 0;
 };
 
 template <class S, class M>
@@ -107,22 +112,22 @@ struct BatchRunnerT : BatchRunner {
         b.count = n;
         b.active = active;
         b.err = err;
-        // Tile height 1: every resident warp takes a share of the rows.  While
+        // The shortest tiles: every resident warp takes a share of the rows.  While
         // the instances' rows outnumber the warps the height does not matter
         // (64 instances of 128..1024: 56.3 ms at any height); when they do not,
         // a warp's march is the step's time, so the shorter the better (16
         // contracted Euler instances of 128..384, 47 steps: 9.6 ms at 48 rows,
         // 5.5 at 16, 5.1 at 4 and below; 3 of 60..200: 4.8 -> 0.58 ms).
-        set_shape(1, per_sm);
+        set_shape(BATCH_SHORTEST, per_sm);
         return 0;
     }
 
     void set_shape(int rows, int ctas) override {
-        min_rows = std::max(1, rows);
+        min_rows = std::max(BATCH_SHORTEST, rows);
         ctas_per_sm = std::max(1, std::min(ctas, per_sm_));
         grid = nsm_ * ctas_per_sm;
         b.nwarps = grid * WARPS2D;
-        b.min_rows = min_rows;
+        b.min_rows = min_rows == BATCH_SHORTEST ? 1 : min_rows;
     }
     int max_ctas_per_sm() const override { return per_sm_; }
     int nsm_ = 1, per_sm_ = 1;
