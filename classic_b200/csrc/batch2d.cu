@@ -103,6 +103,8 @@ struct claw_batch {
     }
 };
 
+static Block q_block(const Geometry& g) { return Block{g.ld, g.fstride, g.meqn, g.mx, g.my}; }
+
 extern "C" {
 
 int claw_batch_create(const claw_config* cfgs, int count, claw_batch** out) {
@@ -175,14 +177,12 @@ int claw_batch_create(const claw_config* cfgs, int count, claw_batch** out) {
         }
         g.ctl = b->ctl_d + k;
     }
-    size_t largest = 0;
-    for (const Geometry& g : b->g) {
-        const size_t n = (size_t)g.meqn * g.mx * g.my;
-        if (n * sizeof(double) <= STAGE_BYTES) largest = std::max(largest, n);
-    }
-    int rc = make_stage(b->stage, {largest}, false);
+    int rc = b->runner->prepare(b->g, cfgs, b->ctl_d, b->flags_d, b->flags_d + 1);
     if (rc) return rc;
-    rc = b->runner->prepare(b->g, cfgs, b->ctl_d, b->flags_d, b->flags_d + 1);
+    size_t largest = 0;
+    for (const Geometry& g : b->g)
+        if (q_block(g).staged(8, false)) largest = std::max(largest, q_block(g).count());
+    rc = make_stage(b->stage, largest, false);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(b->stream));
     *out = b.release();
@@ -197,8 +197,7 @@ int claw_batch_destroy(claw_batch* b) {
 static int batch_fields(claw_batch* b, int k, double* host, bool to_device) {
     const Geometry& g = b->g[k];
     const int cur = b->ctl_h[k].cur;
-    return copy_fields(static_cast<double*>(g.q[cur]), g.ld, g.fstride, host, g.meqn, g.mx, g.my, b->stage,
-                       to_device, b->stream);
+    return copy_fields(static_cast<double*>(g.q[cur]), q_block(g), host, b->stage, to_device, b->stream);
 }
 
 int claw_batch_set_q(claw_batch* b, int k, const double* q) {

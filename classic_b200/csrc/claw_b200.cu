@@ -411,12 +411,13 @@ const char* claw_build_info(void) {
     return "clawb200 sm_100a; fp64 path built with --fmad=false (reference operation order)";
 }
 
-// doubles in the caller's arrays
-static long long aux_rows(const Geometry& g) {
-    return (long long)(g.dim >= 2 ? g.my + 4 : 1) * (g.dim >= 3 ? g.mz + 4 : 1);
+static Block q_block(const Geometry& g) {
+    return Block{g.ld, g.fstride, g.meqn, g.mx, (long long)g.my * g.mz};
 }
-static size_t q_count(const Geometry& g) { return (size_t)g.meqn * g.mx * g.my * g.mz; }
-static size_t aux_count(const Geometry& g) { return g.maux * (size_t)(g.mx + 4) * aux_rows(g); }
+static Block aux_block(const Geometry& g) {
+    return Block{g.ald, g.afstride, g.maux, g.mx + 4,
+                 (long long)(g.dim >= 2 ? g.my + 4 : 1) * (g.dim >= 3 ? g.mz + 4 : 1)};
+}
 
 static int validate(const claw_config* c, SolverShape* sh) {
     if (!c) return fail(CLAW_E_INVALID, "null config");
@@ -518,8 +519,6 @@ int claw_create(const claw_config* cfg, claw_handle** out) {
     std::memset(h->ctl_h, 0, sizeof(ClawCtl));
     h->ctl_h->done = 1;
     CUDA_TRY(cudaMemcpyAsync(g.ctl, h->ctl_h, sizeof(ClawCtl), cudaMemcpyHostToDevice, h->stream));
-    rc = make_stage(h->stage, {q_count(g), aux_count(g)}, g.es == 4);
-    if (rc) return rc;
     h->runner = g.es == 8 ? make_runner<double>(*cfg) : make_runner<float>(*cfg);
     if (!h->runner) return fail(CLAW_E_UNSUPPORTED, "no kernel for solver %d", cfg->solver_id);
     if (cfg->b4step_id == CLAW_B4STEP_REVERSING) {
@@ -529,6 +528,11 @@ int claw_create(const claw_config* cfg, claw_handle** out) {
         else h->runner.reset(new B4StepRunner<float>(std::move(h->runner)));
     }
     rc = h->runner->prepare(*cfg, g);
+    if (rc) return rc;
+    size_t most = 0;  // of the blocks that are copied through the buffer: q both ways, aux in
+    if (q_block(g).staged(g.es, false)) most = q_block(g).count();
+    if (aux_block(g).staged(g.es, true)) most = std::max(most, aux_block(g).count());
+    rc = make_stage(h->stage, most, g.es == 4);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     *out = h.release();
@@ -540,21 +544,17 @@ int claw_destroy(claw_handle* h) {
     return 0;
 }
 
-static int copy_block(claw_handle* h, void* dev, long long pitch, long long fpitch, const double* host,
-                      int nfields, long long width, long long rows, bool in) {
+static int copy_block(claw_handle* h, void* dev, const Block& b, const double* host, bool in) {
     double* hp = const_cast<double*>(host);  // written only when !in
-    if (h->g.es == 8)
-        return copy_fields(static_cast<double*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage,
-                           in, h->stream);
-    return copy_fields(static_cast<float*>(dev), pitch, fpitch, hp, nfields, width, rows, h->stage, in,
-                       h->stream);
+    if (h->g.es == 8) return copy_fields(static_cast<double*>(dev), b, hp, h->stage, in, h->stream);
+    return copy_fields(static_cast<float*>(dev), b, hp, h->stage, in, h->stream);
 }
 
 int claw_set_q(claw_handle* h, const double* q) {
     if (!h || !q) return fail(CLAW_E_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(h->device));
     const Geometry& g = h->g;
-    int rc = copy_block(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, true);
+    int rc = copy_block(h, g.q[h->cur], q_block(g), q, true);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return 0;
@@ -564,7 +564,7 @@ int claw_get_q(claw_handle* h, double* q) {
     if (!h || !q) return fail(CLAW_E_INVALID, "null argument");
     CUDA_TRY(cudaSetDevice(h->device));
     const Geometry& g = h->g;
-    int rc = copy_block(h, g.q[h->cur], g.ld, g.fstride, q, g.meqn, g.mx, (long long)g.my * g.mz, false);
+    int rc = copy_block(h, g.q[h->cur], q_block(g), q, false);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(h->stream));
     return 0;
@@ -575,8 +575,9 @@ int claw_set_aux(claw_handle* h, const double* aux) {
     const Geometry& g = h->g;
     if (g.maux == 0) return 0;
     CUDA_TRY(cudaSetDevice(h->device));
-    const long long rows = aux_rows(g);
-    int rc = copy_block(h, g.aux, g.ald, g.afstride, aux, g.maux, g.mx + 4, rows, true);
+    const Block block = aux_block(g);
+    const long long rows = block.rows;
+    int rc = copy_block(h, g.aux, block, aux, true);
     if (rc) return rc;
     if (g.aux_base)  // the before-step routine scales from this copy
         CUDA_TRY(cudaMemcpyAsync(g.aux_base, g.aux, (size_t)g.afstride * g.maux * g.es,

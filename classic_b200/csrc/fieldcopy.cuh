@@ -17,7 +17,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <initializer_list>
 #include <mutex>
 
 #include "common.cuh"
@@ -39,6 +38,21 @@ struct Stage {
     }
 };
 
+// A caller's dense block and its place on the device.
+struct Block {
+    long long pitch, fpitch;  // elements from row to row, from field to field
+    int nfields;
+    long long width, rows;
+    size_t count() const { return (size_t)nfields * rows * width; }
+    // whether the copy in (or out) takes the buffer; the FP64 rule is above
+    bool staged(size_t elem, bool in) const {
+        if (elem == 4) return true;
+        const size_t bytes = count() * 8;
+        const bool padded = pitch != width || fpitch != width * rows;
+        return padded && nfields > 1 && rows > 1 && bytes <= STAGE_BYTES && !(in && bytes <= 65536);
+    }
+};
+
 // one element a thread, rows over blockIdx.y; row r of field m is dense row
 // m*rows + r
 template <class real, bool IN>
@@ -55,50 +69,45 @@ copy_rows(double* dense, real* dev, long long pitch, long long fpitch, long long
     }
 }
 
-// Queue the copy of nfields fields on the object's stream (the caller waits for
-// it).  FP64 blocks larger than the buffer go directly.
+// Queue the copy of a block on the object's stream (the caller waits for it).
 template <class real>
-int copy_fields(real* dev, long long pitch, long long fpitch, double* host, int nfields, long long width,
-                long long rows, Stage& stage, bool in, cudaStream_t st) {
-    const long long nrows = nfields * rows;
-    const size_t n = (size_t)nrows * width;
+int copy_fields(real* dev, const Block& b, double* host, Stage& stage, bool in, cudaStream_t st) {
+    const size_t n = b.count();
     const auto kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
     if constexpr (sizeof(real) == 8) {
         const bool small_in = in && n * 8 <= 65536;
-        if (pitch == width && fpitch == width * rows && !small_in) {
+        if (b.pitch == b.width && b.fpitch == b.width * b.rows && !small_in) {
             if (in) CUDA_TRY(cudaMemcpyAsync(dev, host, n * 8, kind, st));
             else CUDA_TRY(cudaMemcpyAsync(host, dev, n * 8, kind, st));
             return 0;
         }
-        if (nfields == 1 || rows == 1 || n > stage.n || small_in) {
-            for (int m = 0; m < nfields; ++m) {
-                real* d = dev + m * fpitch;
-                double* hp = host + (size_t)m * width * rows;
-                if (in) CUDA_TRY(cudaMemcpy2DAsync(d, pitch * 8, hp, width * 8, width * 8, rows, kind, st));
-                else CUDA_TRY(cudaMemcpy2DAsync(hp, width * 8, d, pitch * 8, width * 8, rows, kind, st));
+        if (!b.staged(8, in) || n > stage.n) {  // (no buffer where memory was short)
+            for (int m = 0; m < b.nfields; ++m) {
+                real* d = dev + m * b.fpitch;
+                double* hp = host + (size_t)m * b.width * b.rows;
+                if (in) CUDA_TRY(cudaMemcpy2DAsync(d, b.pitch * 8, hp, b.width * 8, b.width * 8, b.rows, kind, st));
+                else CUDA_TRY(cudaMemcpy2DAsync(hp, b.width * 8, d, b.pitch * 8, b.width * 8, b.rows, kind, st));
             }
             return 0;
         }
     }
-    const dim3 grid((unsigned)((width + 255) / 256), (unsigned)std::min(nrows, 65535ll));
+    const long long nrows = b.nfields * b.rows;
+    const dim3 grid((unsigned)((b.width + 255) / 256), (unsigned)std::min(nrows, 65535ll));
     std::lock_guard<std::mutex> together(stage.order);
     if (in) {
         CUDA_TRY(cudaMemcpyAsync(stage.buf, host, n * 8, kind, st));
-        copy_rows<real, true><<<grid, 256, 0, st>>>(stage.buf, dev, pitch, fpitch, width, rows, nrows);
+        copy_rows<real, true><<<grid, 256, 0, st>>>(stage.buf, dev, b.pitch, b.fpitch, b.width, b.rows, nrows);
     } else {
-        copy_rows<real, false><<<grid, 256, 0, st>>>(stage.buf, dev, pitch, fpitch, width, rows, nrows);
+        copy_rows<real, false><<<grid, 256, 0, st>>>(stage.buf, dev, b.pitch, b.fpitch, b.width, b.rows, nrows);
         CUDA_TRY(cudaMemcpyAsync(host, stage.buf, n * 8, kind, st));
     }
     CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
-// The buffer for blocks of these element counts: FP32 fields need the largest,
-// FP64 ones take the largest within STAGE_BYTES, and do without when memory is short.
-inline int make_stage(Stage& stage, std::initializer_list<size_t> counts, bool needed) {
-    size_t n = 0;
-    for (size_t c : counts)
-        if (needed || c * 8 <= STAGE_BYTES) n = std::max(n, c);
+// The buffer for copies of up to n doubles (0: none takes it).  FP32 fields
+// cannot do without (`needed`), FP64 ones can when memory is short.
+inline int make_stage(Stage& stage, size_t n, bool needed) {
     if (!n) return 0;
     const cudaError_t e = cudaMalloc(&stage.buf, n * 8);
     if (e != cudaSuccess) {
