@@ -10,8 +10,10 @@
 // single field, a 1D grid and up to 64 KB in are cheaper directly (annulus
 // 40x120: 28 against 38; 40^2 42 against 43 to 58; one unpadded field of 64^2
 // 17 against 29 for a 1D copy), and where no row is padded the whole block is
-// one copy (four of 128^2 out: 90 against 54).  FP32 blocks need the buffer for the conversion
-// at any size.
+// one copy (four of 128^2 out: 90 against 54).  FP32 blocks need the buffer for
+// the conversion at any size; a single field of 24 to 64 KB goes into it as a 2D
+// block too (64x128 22 against 51, 90x91 34 against 50; the other way 30x90, 21
+// KB, 32 against 26, three fields of 45^2 61 against 41).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -25,6 +27,7 @@
 namespace clawb200 {
 
 constexpr size_t STAGE_BYTES = 8u << 20;
+constexpr size_t SMALL_IN = 64u << 10;
 
 // The buffer of an object, n doubles.  Copies through it are two operations on
 // the object's stream; `order` keeps them together, so that the stream's order
@@ -49,7 +52,7 @@ struct Block {
         if (elem == 4) return true;
         const size_t bytes = count() * 8;
         const bool padded = pitch != width || fpitch != width * rows;
-        return padded && nfields > 1 && rows > 1 && bytes <= STAGE_BYTES && !(in && bytes <= 65536);
+        return padded && nfields > 1 && rows > 1 && bytes <= STAGE_BYTES && !(in && bytes <= SMALL_IN);
     }
 };
 
@@ -75,7 +78,7 @@ int copy_fields(real* dev, const Block& b, double* host, Stage& stage, bool in, 
     const size_t n = b.count();
     const auto kind = in ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
     if constexpr (sizeof(real) == 8) {
-        const bool small_in = in && n * 8 <= 65536;
+        const bool small_in = in && n * 8 <= SMALL_IN;
         if (b.pitch == b.width && b.fpitch == b.width * b.rows && !small_in) {
             if (in) CUDA_TRY(cudaMemcpyAsync(dev, host, n * 8, kind, st));
             else CUDA_TRY(cudaMemcpyAsync(host, dev, n * 8, kind, st));
@@ -95,7 +98,10 @@ int copy_fields(real* dev, const Block& b, double* host, Stage& stage, bool in, 
     const dim3 grid((unsigned)((b.width + 255) / 256), (unsigned)std::min(nrows, 65535ll));
     std::lock_guard<std::mutex> together(stage.order);
     if (in) {
-        CUDA_TRY(cudaMemcpyAsync(stage.buf, host, n * 8, kind, st));
+        if (b.nfields == 1 && n * 8 > (24u << 10) && n * 8 <= SMALL_IN)
+            CUDA_TRY(cudaMemcpy2DAsync(stage.buf, b.width * 8, host, b.width * 8, b.width * 8, b.rows, kind, st));
+        else
+            CUDA_TRY(cudaMemcpyAsync(stage.buf, host, n * 8, kind, st));
         copy_rows<real, true><<<grid, 256, 0, st>>>(stage.buf, dev, b.pitch, b.fpitch, b.width, b.rows, nrows);
     } else {
         copy_rows<real, false><<<grid, 256, 0, st>>>(stage.buf, dev, b.pitch, b.fpitch, b.width, b.rows, nrows);
