@@ -77,17 +77,24 @@ __device__ __forceinline__ real mx2(real x, real y) {
 //   MC        sign(a) max(0, min(2A, 2N, (A + N) / 2))
 //   Beam-Warming  n
 // a == 0 gives 0, as the reference skips a zero wave.  FP64 superbee selects
-// between a and n by magnitude and sign bits (2048^2, us a step: 50.0 -> 46.3;
-// minmod that way 94.4 -> 95.3 at 3072^2); van Leer without magnitudes 56.4 ->
-// 49.0, FP32 35.9 -> 33.5.
+// between a and n by magnitude and sign bits (2048^2, us a step: 50.0 -> 46.3);
+// van Leer without magnitudes 56.4 -> 49.0, FP32 35.9 -> 33.5.  SEL: FP64 minmod
+// by select too, where that is the faster: the Strang kernel (2048^2 54.5 ->
+// 52.1, 3072^2 112.4 -> 107.1) and the fused 3D step (192^3 488 -> 482); not the
+// unsplit kernel (3072^2 92.6 -> 95.7), nor Godunov beyond the L2 (3072^2 97.4
+// -> 98.9; 2048^2 42.6 -> 41.7).
 // LIM >= 0 fixes the limiter at compile time; LIM = -1 reads it at run time
 // (a warp-uniform branch; there the forms that share |a| and N, so that the
 // branches stay short: MC / none, FP64 4096^2, 73 against 62 G cells/s).
-template <typename real, int LIM>
+template <typename real, int LIM, bool SEL = false>
 __device__ __forceinline__ real limited_strength(real a, real n, int lim_rt) {
     const int lim = LIM >= 0 ? LIM : lim_rt;
     if constexpr (sizeof(real) == 8) {
         if (lim == 4) return mc_strength(a, n);
+        if (SEL && LIM >= 0 && lim == 1) {  // where the signs agree, the smaller
+            const real m = fabs(n) < fabs(a) ? n : a;
+            return (__double2hiint(a) ^ __double2hiint(n)) >= 0 ? m : real(0);
+        }
         if (LIM >= 0 && lim == 2) {  // where the signs agree, with a's sign: the smaller of
             const bool lt = fabs(a) < fabs(n);  // twice the smaller and the other
             const real t = real(2) * (lt ? a : n), big = lt ? n : a;

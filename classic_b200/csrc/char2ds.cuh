@@ -63,7 +63,7 @@ __device__ __forceinline__ CharSplitConsts<real> char_xsweep_consts(double dtdx_
 // c0, c1 and (pM, uM) at c0-1; returns the swept p and u of c0 and c1 (exact
 // where lanes l-1 and l+1 hold real data).  flux2 without the transverse part
 // (flux2.f90:110-181) and step2ds's update (step2ds.f90:201-214).
-template <typename real, int LIM>
+template <typename real, int LIM, bool SEL>
 __device__ __forceinline__ void char_xsweep(real pM, real uM, real p0, real u0, real p1, real u1,
                                             const CharSplitConsts<real>& K, const CharAcoustics2D<real>& S,
                                             int lim, int lim2, real& xp0, real& xu0, real& xp1, real& xu1) {
@@ -75,10 +75,10 @@ __device__ __forceinline__ void char_xsweep(real pM, real uM, real p0, real u0, 
     const real a2_1 = Z * (u1 - u0) + (p1 - p0);
     const real a1_R = __shfl_down_sync(FULL, a1_0, 1);  // interface c1+1 (lane+1's I0)
     const real a2_L = __shfl_up_sync(FULL, a2_1, 1);    // interface c0-1 (lane-1's I1)
-    const real l1_0 = limited_strength<real, LIM>(a1_0, a1_1, lim);
-    const real l2_0 = limited_strength<real, LIM>(a2_0, a2_L, lim2);
-    const real l1_1 = limited_strength<real, LIM>(a1_1, a1_R, lim);
-    const real l2_1 = limited_strength<real, LIM>(a2_1, a2_0, lim2);
+    const real l1_0 = limited_strength<real, LIM, SEL>(a1_0, a1_1, lim);
+    const real l2_0 = limited_strength<real, LIM, SEL>(a2_0, a2_L, lim2);
+    const real l1_1 = limited_strength<real, LIM, SEL>(a1_1, a1_R, lim);
+    const real l2_1 = limited_strength<real, LIM, SEL>(a2_1, a2_0, lim2);
     const real d0 = l2_0 - l1_0, s0 = l1_0 + l2_0;
     const real d1 = l2_1 - l1_1, s1 = l1_1 + l2_1;
     const real dR = __shfl_down_sync(FULL, d0, 1), sR = __shfl_down_sync(FULL, s0, 1);
@@ -231,7 +231,7 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
                 fetch2(sq, sr, ng, 2, v[0], v[1]);
                 const real pM = fetchM(sq, sr, ng, 0), uM = fetchM(sq, sr, ng, 1);
                 real xp0, xu0, xp1, xu1;
-                char_xsweep<real, LIM>(pM, uM, p[0], u[0], p[1], u[1], KA, A.s, A.lim, A.lim2, xp0, xu0, xp1,
+                char_xsweep<real, LIM, STRANG>(pM, uM, p[0], u[0], p[1], u[1], KA, A.s, A.lim, A.lim2, xp0, xu0, xp1,
                                        xu1);
                 xa[0][0] = (INT || xin0) ? xp0 : p[0];
                 xa[0][1] = (INT || xin0) ? xu0 : u[0];
@@ -272,8 +272,8 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
                     const real dp = xn[k][0] - xc[k][0], dv = xn[k][2] - xc[k][2];
                     a1n[k] = Z * dv - dp;
                     a2n[k] = Z * dv + dp;
-                    const real b1 = limited_strength<real, LIM>(a1y[k], a1n[k], A.lim);      // upwind t+1
-                    const real b2 = limited_strength<real, LIM>(a2y[k], a2y_lo[k], A.lim2);  // upwind t-1
+                    const real b1 = limited_strength<real, LIM, STRANG>(a1y[k], a1n[k], A.lim);      // upwind t+1
+                    const real b2 = limited_strength<real, LIM, STRANG>(a2y[k], a2y_lo[k], A.lim2);  // upwind t-1
                     dyk[k] = b2 - b1;
                     syk[k] = b1 + b2;
                     o[k][0] = (xb[k][0] - qpyh * (a2y_lo[k] + a1y[k])) - kpy * (dyk[k] - dy_lo[k]);
@@ -285,7 +285,7 @@ step2s_char_kernel(const __grid_constant__ CharArgs<real> A) {
                     // c0-1 is lane l-1's c1 (ghost columns keep the y-swept value)
                     const real pM = __shfl_up_sync(FULL, o[1][0], 1), uM = __shfl_up_sync(FULL, o[1][1], 1);
                     real xp0, xu0, xp1, xu1;
-                    char_xsweep<real, LIM>(pM, uM, o[0][0], o[0][1], o[1][0], o[1][1], KC, A.s, A.lim, A.lim2,
+                    char_xsweep<real, LIM, STRANG>(pM, uM, o[0][0], o[0][1], o[1][0], o[1][1], KC, A.s, A.lim, A.lim2,
                                            xp0, xu0, xp1, xu1);
                     if (INT || xin0) { o[0][0] = xp0; o[0][1] = xu0; }
                     if (INT || xin1) { o[1][0] = xp1; o[1][1] = xu1; }

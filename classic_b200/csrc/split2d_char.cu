@@ -65,7 +65,7 @@ struct CharSplitRunner : Runner {
 
 // One limiter on both waves compiled in; two different ones, none and
 // Beam-Warming read at run time, a switch in every limited strength (Strang,
-// 2048^2, us a step: FP64 minmod 128 -> 56, superbee 135 -> 61, van Leer 138 ->
+// 2048^2, us a step: FP64 minmod 128 -> 52, superbee 135 -> 61, van Leer 138 ->
 // 63; FP32 62 -> 35, 64 -> 38, 66 -> 40)
 template <typename real, int BCM, bool STRANG>
 std::unique_ptr<Runner> pick_lim(int l1, int l2) {

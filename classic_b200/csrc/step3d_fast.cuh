@@ -237,8 +237,8 @@ __device__ __forceinline__ void step3f_march(const Step3fArgs<real>& A, const St
         if (f & 2) w = (real)(2.0 * piston_speed(a, i, j, tbc)) - w;
         return w;
     };
-    auto lim_a = [&](real s, real n) { return limited_strength<real, LIM>(s, n, lim1); };
-    auto lim_b = [&](real s, real n) { return limited_strength<real, LIM>(s, n, lim2); };
+    auto lim_a = [&](real s, real n) { return limited_strength<real, LIM, true>(s, n, lim1); };
+    auto lim_b = [&](real s, real n) { return limited_strength<real, LIM, true>(s, n, lim2); };
     // factor of a limited wave in the correction flux of a direction: |s| (1 - |s| dt/dn) / 2
     auto coef = [&](real c, real tn) { return half2 * fabs(c) * (real(1) - fabs(c) * tn); };
     // p, u (along A-B) and v (along A-C) of an edge flux
