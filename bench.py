@@ -457,6 +457,7 @@ def other_configs(peaks, cpu=True):
                 upd = n3 * (st["steps_taken"] + st["steps_rejected"])
                 es = 4 if prec == "fp32" else 8
                 rate = upd / (st["device_ms"] * 1e-3)
+                # (sweep3f_*: the keys of step3f_kernel's figures)
                 kern = {"fp64": "sweep3p_fp64", "fp64_fma": "sweep3f_fp64_fma",
                         "fp32": "sweep3f_fp32"}[prec]
                 e = {"cell_updates_per_s": rate, "steps": st["steps_taken"],

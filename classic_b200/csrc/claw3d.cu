@@ -13,8 +13,8 @@ std::unique_ptr<Runner> make_runner3d(const claw_config& cfg) {
     if (cfg.dimensional_split > 0)
         return std::unique_ptr<Runner>(new SplitRunner3D<VCAcoustics3D<double>, 0>());
     using S = VCAcoustics3D<double>;
-    // one limiter on both waves compiled in (128^3, us a step: minmod 1870 ->
-    // 1600, van Leer 1925 -> 1685)
+    // one limiter on both waves compiled in (128^3, us a step: minmod 1888 ->
+    // 1600, superbee 1884 -> 1612, van Leer 1929 -> 1695, MC 1911 -> 1622)
     if (cfg.order == 2 && cfg.transverse_waves == 22 && cfg.limiter[0] == cfg.limiter[1]) {
         const int lim = cfg.limiter[0];
         if (lim == 1) return std::unique_ptr<Runner>(new Runner3D<S, Method3D<2, 2, 1>>());

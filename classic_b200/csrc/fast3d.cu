@@ -40,8 +40,9 @@ struct Step3fRunner : Runner {
 template <typename real>
 static std::unique_ptr<Runner> step3f_runner(const claw_config& cfg) {
     if (cfg.transverse_waves < 10) return std::unique_ptr<Runner>(new Step3fRunner<real, -1, false>());
-    // one limiter on both waves compiled in (128^3, us a step, FP64 / FP32: minmod 233 ->
-    // 200 / 150 -> 135, van Leer 240 -> 209 / 150 -> 139)
+    // one limiter on both waves compiled in (128^3, us a step, FP64 / FP32: minmod 229 ->
+    // 196 / 147 -> 132, superbee 234 -> 201 / 146 -> 133, van Leer 235 -> 205 / 147 -> 136,
+    // MC 216 -> 202 / 147 -> 134)
     if (cfg.limiter[0] == cfg.limiter[1]) {
         const int lim = cfg.limiter[0];
         if (lim == 1) return std::unique_ptr<Runner>(new Step3fRunner<real, 1, true>());

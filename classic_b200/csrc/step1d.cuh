@@ -66,8 +66,16 @@ __device__ __forceinline__ double warp_max_nonneg(double c) {
 }
 
 // Methods compiled in: one limiter on every wave at order 2 without capacity,
-// f-waves or source (taken branches cost a lone warp 30-100 cycles each; 800
-// cells, us a frame: minmod 213 -> 174, van Leer 226 -> 188), and one that reads everything at run time.
+// f-waves or source (taken branches cost a lone warp 30-100 cycles each), and
+// one that reads everything at run time.  us a step, run time -> compiled in:
+//               minmod         superbee       van Leer       MC
+// acoustics 100   1.32 -> 0.92   1.35 -> 0.93   1.41 -> 1.09   1.35 -> 0.92
+//           800   2.32 -> 1.84   2.41 -> 1.92   2.48 -> 2.07   2.40 -> 1.91
+//          2500   6.17 -> 4.70   6.43 -> 4.88   6.54 -> 5.28   6.37 -> 4.86
+// varying   800   2.74 -> 2.19   2.90 -> 2.32   2.92 -> 2.32   2.90 -> 2.32
+// advection 800   1.42 -> 1.18   1.46 -> 1.19   1.53 -> 1.26   1.45 -> 1.19
+// Euler     800   6.53 -> 5.47   6.71 -> 5.65   6.98 -> 5.89   6.80 -> 5.64
+// and 12 to 30 % for each of them at 100 and 2500 cells.
 template <int LIM>
 struct Method1 {
     static constexpr int lim = LIM;

@@ -295,7 +295,9 @@ __device__ __forceinline__ double sweep3p_march(const Sweep3Args<typename S::rea
     };
     // 1 / (Z + Z_next) along A and B of ring position pos, from its landed Z.
     // The next tile element is the next cell, or the same clamped cell past
-    // the grid's last ghost; the tile's last row and column are never read.
+    // the grid's last ghost.  The tile's last row and column have no next and
+    // stay unset: only splits of halo slices read them, whose terms reach no
+    // slice that is written.
     auto make_rcp = [&](int pos) {
         real* dst = saux + (pos & (RING3 - 1)) * NPL * NS3;
         for (int e = tid; e < NS3; e += NT3P) {
@@ -650,7 +652,7 @@ __global__ void __launch_bounds__(NT3P, CLAW_SWEEP3_MINB) sweep3p_kernel(const S
     using real = typename S::real;
     double* red = reinterpret_cast<double*>(reinterpret_cast<real*>(smem_raw) +
                                             RING3 * NPL3 * NS3 + (NTERM3 + XCH3 + QST3 + VST3) * NT3);
-    __shared__ int far;  // some Z + Z' of the tile is out of quot3's range
+    __shared__ int far;  // some Z + Z' of the tile is out of quot_rcp's range for divisors
     ClawCtl* ctl = a.ctl;
     grid_dependency_sync();
     if (ctl->done) return;

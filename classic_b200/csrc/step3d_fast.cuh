@@ -25,8 +25,8 @@
 //     yA = c_D Y_A, yB = c_C Y_B, yC = c_B Y_C, yD = c_A Y_D and, with a the
 //     A-C, b the B-D, g the A-B and e the C-D face's r, m1 = a e K_C,
 //     m2 = b g K_B, m3 = b e K_D, m4 = a g K_A.
-// About 330 FP64 instructions per cell and step where the splits written out
-// one by one took 1815.  The limiter works on wave strengths: the ratio of
+// 434 FP64 instructions per cell written, halo included (316 per cell computed),
+// where the splits written out one by one took 1815.  The limiter works on wave strengths: the ratio of
 // two waves' products is a'/a (1 + Z Z')/(1 + Z^2) with per-cell 1/(1 + Z^2).
 //
 // The march.  A warp holds 32 cells of a row (lane = x), a CTA ROWS rows; the
@@ -51,9 +51,9 @@
 // Measured against three sweep launches that formed every split (1815 FP64
 // instructions and 245 B of DRAM traffic per cell): 256^3 FP64 7.45 -> 1.30
 // ms per step, 161x130x147 FP32 1.02 -> 0.158.  What bounds it: FP64 at
-// 192^3 runs the FP64 pipe at 30 % and issue at 46 % with 12 warps per SM
+// 192^3 runs the FP64 pipe at 30 % and issue at 50 % with 12 warps per SM
 // (fixed-latency chains and the three barriers); FP32 is issue bound (71 %).
-// DRAM traffic is 77 B per cell (80 algorithmic).
+// DRAM traffic is 76 B per cell (80 algorithmic).
 #pragma once
 #include "char2d.cuh"
 #include "step3d.cuh"
@@ -61,7 +61,7 @@
 namespace clawb200 {
 
 // Rows (warps) of a CTA and resident CTAs.  FP64: 12 rows leave 168 registers
-// a thread and nothing spills; the shared planes leave so little L1 that any
+// a thread and 8 bytes spill; the shared planes leave so little L1 that any
 // spill goes to L2 (256^3, ms per step: 12 rows 1.32, 13 rows at 144
 // registers 2.41, 16 rows at 128 2.1, 8 rows x 2 CTAs 1.9).  FP32: two CTAs of
 // 9 rows hide each other's barriers (161x130x147, us per step, before the

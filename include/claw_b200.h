@@ -155,7 +155,9 @@ int claw_create(const claw_config* cfg, claw_handle** out);
 int claw_destroy(claw_handle* h);
 
 /* Copy the interior of q from / to the host (pageable or pinned).  Replaces
- * qinit's fill of q (src/2d/claw2ez.f:244) and the read of q by out2. */
+ * qinit's fill of q (src/2d/claw2ez.f:244) and the read of q by out2.  These
+ * three copies of one handle may run from several host threads at once, but not
+ * beside a call that steps it. */
 int claw_set_q(claw_handle* h, const double* q);
 int claw_get_q(claw_handle* h, double* q);
 /* aux with its two ghost layers, as setaux fills it (src/2d/claw2ez.f:224). */
@@ -257,7 +259,8 @@ typedef struct claw_batch claw_batch;
 /* count instances (1..1024), cfgs[k] for instance k; FP64, 2D. */
 int claw_batch_create(const claw_config* cfgs, int count, claw_batch** out);
 int claw_batch_destroy(claw_batch* b);
-/* q of instance k, [num_eqn][my][mx] as for claw_set_q / claw_get_q */
+/* q of instance k, [num_eqn][my][mx] as for claw_set_q / claw_get_q; different
+ * instances from several host threads, too */
 int claw_batch_set_q(claw_batch* b, int k, const double* q);
 int claw_batch_get_q(claw_batch* b, int k, double* q);
 /* Advance every instance from tstart to tend.  dt_initial[k] seeds instance

@@ -44,7 +44,10 @@ int nn_conv3x3_dgrad(const void* dz, const void* w, const float* z, void* dx, in
  * accumulator gave up, and that launch left its output unwritten); clear != 0
  * resets them.  Synchronises with the device. */
 int nn_device_error(int clear);
-/* wt[ci][tap][co] = w[co][8-tap][ci]: the data gradient dx = conv3x3(dz, wt). */
+/* The two steps that nn_conv3x3_dgrad takes into its convolution, by themselves:
+ * the library does not call them; they serve callers that want the unfused form
+ * and the checks of the fused one (as nn_adam does for nn_adam_multi).
+ * wt[ci][tap][co] = w[co][8-tap][ci]: the data gradient dx = conv3x3(dz, wt). */
 int nn_flip_weights(const void* w, void* wt, int cout, int cin, void* stream);
 /* dz = dy * GELU'(z), n elements. */
 int nn_gelu_backward(const void* dy, const float* z, void* dz, long long n, void* stream);
