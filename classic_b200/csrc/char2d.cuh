@@ -45,7 +45,7 @@ __device__ __forceinline__ float sign_times(float x, float s) {
 // operations), but no fmin/fmax: their NaN rules cost extra instructions in
 // FP64, and the select picks one of two registers.
 __device__ __forceinline__ double mc_strength(double a, double n) {
-    const double mn = fabs(a) < fabs(n) ? a : n;  // |mn| = min(|a|, |n|)
+    const double mn = fabs(n) < fabs(a) ? n : a;  // |mn| = min(|a|, |n|); a where n is NaN
     const double q = 0.25 * (fabs(a) + fabs(n));
     const double r = q < fabs(mn) ? q : mn;       // |r| = the smaller of the two
     const int ah = __double2hiint(a), nh = __double2hiint(n);
