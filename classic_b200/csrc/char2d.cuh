@@ -112,9 +112,9 @@ __device__ __forceinline__ real limited_strength(real a, real n, int lim_rt) {
     const real A = fabs(a), N = sign_times(n, a);
     real m;
     if (lim == 1) {
-        m = mn2(A, N);
+        m = mn2(N, A);  // (A where N is NaN)
     } else if (lim == 2) {
-        m = mx2(mn2(A, real(2) * N), mn2(real(2) * A, N));
+        m = mx2(mn2(real(2) * N, A), mn2(N, real(2) * A));
     } else if (lim == 3) {
         const real pos = N > real(0) ? N : real(0);
         m = real(2) * A * pos * rcp_newton(A + (N > real(0) ? N : real(1)));
