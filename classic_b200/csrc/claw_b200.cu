@@ -529,6 +529,7 @@ int claw_create(const claw_config* cfg, claw_handle** out) {
     }
     rc = h->runner->prepare(*cfg, g);
     if (rc) return rc;
+    CUDA_TRY(h->runner->aux_set(h->stream));
     size_t most = 0;  // of the blocks that are copied through the buffer: q both ways, aux in
     if (q_block(g).staged(g.es, false)) most = q_block(g).count();
     if (aux_block(g).staged(g.es, true)) most = std::max(most, aux_block(g).count());
@@ -579,6 +580,7 @@ int claw_set_aux(claw_handle* h, const double* aux) {
     const long long rows = block.rows;
     int rc = copy_block(h, g.aux, block, aux, true);
     if (rc) return rc;
+    CUDA_TRY(h->runner->aux_set(h->stream));
     if (g.aux_base)  // the before-step routine scales from this copy
         CUDA_TRY(cudaMemcpyAsync(g.aux_base, g.aux, (size_t)g.afstride * g.maux * g.es,
                                  cudaMemcpyDeviceToDevice, h->stream));

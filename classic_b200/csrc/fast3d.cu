@@ -12,6 +12,12 @@ struct Step3fRunner : Runner {
     using Sh = Step3fShape<real>;
     Step3fArgs<real> args;
     int grid = 1;
+    int* zrange = nullptr;  // FP32: the exponents of Z
+    long long nz = 0;
+
+    ~Step3fRunner() override {
+        if (zrange) cudaFree(zrange);
+    }
 
     int prepare(const claw_config& cfg, const Geometry& g) override {
         auto k = &step3f_kernel<real, LIM, TRANS>;
@@ -30,7 +36,21 @@ struct Step3fRunner : Runner {
         const long long n = tiles * ((g.mz + args.seglen - 1) / args.seglen);
         if (n > 0x7fffffffLL) return fail(CLAW_E_UNSUPPORTED, "3D grid too large");
         grid = (int)n;
+        if (sizeof(real) == 4) {
+            CUDA_TRY(cudaMalloc(&zrange, 2 * sizeof(int)));
+            args.zrange = zrange;
+            nz = g.afstride;
+        }
         return 0;
+    }
+    cudaError_t aux_set(cudaStream_t s) override {
+        if constexpr (sizeof(real) == 4) {
+            const cudaError_t e = cudaMemsetAsync(zrange, 0, 2 * sizeof(int), s);
+            if (e != cudaSuccess) return e;
+            impedance_range<<<(int)std::min((nz + 1023) / 1024, 592ll), 256, 0, s>>>(args.g.aux, nz, zrange);
+            return cudaGetLastError();
+        }
+        return cudaSuccess;
     }
     cudaError_t launch(cudaStream_t s) override {
         return launch_step(&step3f_kernel<real, LIM, TRANS>, dim3(grid), dim3(32 * Sh::rows), Sh::smem, s, args);

@@ -28,6 +28,7 @@ struct Runner {
     virtual ~Runner() {}
     virtual int prepare(const claw_config& cfg, const Geometry& g) = 0;
     virtual cudaError_t launch(cudaStream_t s) = 0;  // one time step
+    virtual cudaError_t aux_set(cudaStream_t) { return cudaSuccess; }  // g.aux has new values
     virtual int launches_per_step() const { return 1; }
 };
 

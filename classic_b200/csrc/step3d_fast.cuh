@@ -101,7 +101,26 @@ template <typename real>
 struct Step3fArgs {
     Sweep3Args<real> g;  // q, aux, strides, sizes, boundary conditions, method
     int tilesx, tilesy, seglen;
+    const int* zrange;  // FP32: from impedance_range
 };
+
+// The exponents of n impedances: out[0] = 200 + the largest, out[1] = 200 - the
+// smallest (zeroed before; 0 where there is no normal number).
+__global__ void __launch_bounds__(256) impedance_range(const float* z, long long n, int* out) {
+    int hi = 0, lo = 0;
+    for (long long k = blockIdx.x * 256ll + threadIdx.x; k < n; k += gridDim.x * 256ll) {
+        const int e = ((__float_as_int(z[k]) >> 23) & 255) - 127;
+        if (e == -127 || e == 128) continue;
+        hi = max(hi, 200 + e);
+        lo = max(lo, 200 - e);
+    }
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    lo = __reduce_max_sync(0xffffffffu, lo);
+    if ((threadIdx.x & 31) == 0 && hi > 0) {
+        atomicMax(out, hi);
+        atomicMax(out + 1, lo);
+    }
+}
 
 // Where a plane's q and aux lie in global memory, and whether w changes its sign
 // (1) or takes the piston's (2) there.
@@ -114,7 +133,7 @@ struct Plane3f {
 // zt holds planes t-1 .. t+4 at [pos & 7].  One thread fills an entry a plane
 // ahead; each thread for itself, three times a plane, it cost the FP32 kernel,
 // bound by issue, 5 % (192^3 314 -> 298 us a step; FP64 517 -> 509).
-// UNIT: the tile takes 2^e as its unit of impedance and pressure.
+// UNIT: the grid takes 2^e as its unit of impedance and pressure.
 template <typename real, int LIM, bool TRANS, bool UNIT>
 __device__ __forceinline__ void step3f_march(const Step3fArgs<real>& A, const StepHead& hd, unsigned char* smem_raw,
                                              double* red, Plane3f<real>* zt, int e) {
@@ -223,7 +242,7 @@ __device__ __forceinline__ void step3f_march(const Step3fArgs<real>& A, const St
         cp_async_el(d + PL + own, q + qxy + 2 * a.fstride);
         if (edge) cp_async_el(d + PL + hal, q + qxh + 2 * a.fstride);
     };
-    // own Z's of a landed plane into the tile's unit (before the barrier that publishes them)
+    // own Z's of a landed plane into the unit (before the barrier that publishes them)
     auto to_unit = [&](int so) {
         if (UNIT) {
             ring[so + PL + own] *= zu;
@@ -537,16 +556,14 @@ step3f_kernel(const __grid_constant__ Step3fArgs<real> A) {
     const StepHead hd = step_head(A.g.ctl);
     if (hd.done) return;
     // FP32: products of impedances (1 + Z Z', r r' K) leave its range beyond Z =
-    // 2^+-62.  A tile whose first cell lies beyond 2^+-40 takes a power of two
-    // near that Z as its unit of impedance and pressure, which changes exponents
-    // only.  A march of its own: the few multiplications cost the others 2.8 %
+    // 2^+-62.  A grid with some Z beyond 2^+-40 takes the power of two amid its
+    // Z's as unit of impedance and pressure, which changes exponents only.  A
+    // march of its own: the few multiplications cost the others 2.8 %
     // (161x130x147 1426 -> 1466 us a frame).
     if constexpr (sizeof(real) == 4) {
-        using Sh = Step3fShape<real>;
-        const int bx = blockIdx.x % A.tilesx, by = blockIdx.x / A.tilesx % A.tilesy, seg = blockIdx.x / A.tilesx / A.tilesy;
-        const real z = A.g.aux[(2 + bx * Sh::outx) + (2 + by * Sh::outy) * A.g.as[1] + (2 + seg * A.seglen) * A.g.as[2]];
-        const int e = ((__float_as_int(z) >> 23) & 255) - 127;
-        if (abs(e) > 40 && abs(e) < 127) {
+        const int hi = A.zrange[0] - 200, lo = 200 - A.zrange[1];
+        const int e = max(-126, min(126, (hi + lo) / 2));
+        if (hi > -200 && (hi > 40 || lo < -40) && e != 0) {
             step3f_march<real, LIM, TRANS, true>(A, hd, smem_raw, red, zt, e);
             return;
         }

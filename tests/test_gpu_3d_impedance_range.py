@@ -10,6 +10,8 @@ import pytest
 
 from classic_b200 import problems
 from classic_b200.solver import Solver
+from helpers import rel_diff
+from pyoracle import OracleGrid
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +43,24 @@ def test_scaled_medium(near, far, limiters, trans, bc):
     (a, sa), (b, sb) = _run(near, limiters, trans, bc), _run(far, limiters, trans, bc)
     assert np.isfinite(a).all() and sa == sb
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("low,high", [(-45, 20), (45, -20), (-90, -60), (90, 20)])
+def test_contrast(low, high):
+    """Layers of very different Z, the first beyond the range in which the tile
+    keeps the plain unit, against the oracle.  Two steps of under 200 rounded
+    terms each of the size of the field: 2 * 200 * 2^-24 = 2.4e-5 (bar: 5e-5)."""
+    rd, solver, params, q0, aux = problems.random_acoustics_3d(30, 12, 14, seed=3, limiter="mc")
+    q, a = np.float32(q0).astype(np.float64), np.float32(aux).astype(np.float64)
+    a[0, :9] *= 2.0**low
+    a[0, 9:] *= 2.0**high
+    g, o = Solver(rd.clawdata, solver, params, "fp32"), OracleGrid(rd.clawdata, solver, params)
+    for s in (g, o):
+        s.set_q(q)
+        s.set_aux(a)
+    for dt in (0.004, 0.006):
+        g.step(dt)
+        o.step(dt)
+    out = g.get_q()
+    g.close()
+    assert np.isfinite(out).all() and np.all(rel_diff(out, o.get_q()) <= 5e-5)
